@@ -145,7 +145,7 @@ def opt_weights(case, seed):
     D, H, F = cfg.hidden_size, cfg.n_head, cfg.n_inner
     unit = torch.nn.functional.normalize
     kinds = unit(r.f32(TOKEN_KINDS, D), dim=1)
-    words = r.f32(VOCAB, D, std=0.5).view(-1, TOKEN_KINDS, D).add_(0.4 * D ** 0.5 * kinds)
+    words = r.f32(VOCAB, D, std=0.5).view(-1, TOKEN_KINDS, D).add_(D ** 0.5 * kinds)
     W = {"transformer.embeddings.word_embeddings.weight": words.view(VOCAB, D).half(),
          "transformer.embeddings.position_embeddings.weight": r.normal(cfg.max_position_embeddings, D, std=0.5),
          "transformer.ln_f.weight": r.normal(D, std=0.1, mean=1.0), "transformer.ln_f.bias": r.normal(D)}
