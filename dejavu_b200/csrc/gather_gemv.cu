@@ -31,16 +31,10 @@ template <int B, int ACT>
 static void launch_rowdot(const RowdotPlan &p, __half *Y, const __half *W, const __half *X,
                           const void *idx, const __half *bias, int M, int N, long long ldw,
                           int idx64, cudaStream_t st) {
-#define DJV_RD(WPR_, ROWS_)                                                               \
-  djv::launch_kernel(rowdot_kernel<__half, __half, B, ACT, WPR_, ROWS_, 4>, p.grid, RD_THREADS, 0, st, Y, W, X, idx, bias, M, N, \
-                     ldw, idx64, (idx == nullptr || early_prefetch()) ? 1 : 0, 0.f)
-  constexpr int R = (B <= 2) ? 2 : 1;
-  switch (p.wpr) {
-    case 1: DJV_RD(1, R); break;
-    case 2: DJV_RD(2, R); break;
-    case 4: DJV_RD(4, R); break;
-    default: DJV_RD(8, R); break;
-  }
+#define DJV_RD(WPR_, R_, U_)                                                                                            \
+  djv::launch_kernel(rowdot_kernel<__half, __half, B, ACT, WPR_, R_, U_>, p.grid, RD_THREADS, 0, st, Y, W, X, idx, bias, \
+                     M, N, ldw, idx64, (idx == nullptr || early_prefetch()) ? 1 : 0, 0.f, p.per_block, p.rest)
+  DJV_ROWDOT(p, B, DJV_RD);
 #undef DJV_RD
 }
 
@@ -67,7 +61,7 @@ static int dispatch_act(const RowdotPlan &p, int act, __half *Y, const __half *W
 // (each slice re-reads the gathered rows).
 static int rowdot_slice(int B, int act, __half *Y, const __half *W, const __half *X, const void *idx,
                         const __half *bias, int M, int N, long long ldw, int idx64, cudaStream_t st) {
-  const RowdotPlan p = plan_rowdot(M, N / 8, B, B <= 2 ? 2 : 1);
+  const RowdotPlan p = plan_rowdot(M, N / 8, 1, B);
   switch (B) {
     case 1: return dispatch_act<1>(p, act, Y, W, X, idx, bias, M, N, ldw, idx64, st);
     case 2: return dispatch_act<2>(p, act, Y, W, X, idx, bias, M, N, ldw, idx64, st);

@@ -34,17 +34,12 @@ rowdot_any_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restri
 template <typename T, typename TO, int B, int ACT>
 static void launch_rowdot_dense(TO *Y, const T *W, const T *X, int M, int N, long long ldw, float param,
                                 cudaStream_t st) {
-  constexpr int R = (B <= 2 || is_glu(ACT)) ? 2 : 1;
-  const RowdotPlan p = plan_rowdot(M, N / Chunk<T>::N, B, R);
-#define DJV_RD(WPR_)                                                                                            \
-  djv::launch_kernel(rowdot_kernel<T, TO, B, ACT, WPR_, R, 4>, p.grid, RD_THREADS, 0, st, Y, W, X,              \
-                     static_cast<const void *>(nullptr), static_cast<const T *>(nullptr), M, N, ldw, 0, 1, param)
-  switch (p.wpr) {
-    case 1: DJV_RD(1); break;
-    case 2: DJV_RD(2); break;
-    case 4: DJV_RD(4); break;
-    default: DJV_RD(8); break;
-  }
+  const RowdotPlan p = plan_rowdot(M, N / Chunk<T>::N, is_glu(ACT) ? 2 : 1, B);
+#define DJV_RD(WPR_, R_, U_)                                                                                            \
+  djv::launch_kernel(rowdot_kernel<T, TO, B, ACT, WPR_, R_, U_>, p.grid, RD_THREADS, 0, st, Y, W, X,                     \
+                     static_cast<const void *>(nullptr), static_cast<const T *>(nullptr), M, N, ldw, 0, 1, param, \
+                     p.per_block, p.rest)
+  DJV_ROWDOT(p, B, DJV_RD);
 #undef DJV_RD
   count_launch();
 }

@@ -29,23 +29,33 @@ __device__ __forceinline__ float apply_act_param(float v, float p) {
 }
 
 // -------------------------------------------------------------------------------------------
-// rowdot. A block has 8 warps split into 8/WPR groups of WPR warps; a group owns ROWS rows at a
-// time and its 32*WPR lanes stride over the 16-byte chunks of those rows, U chunks in flight per
-// lane per row. x is read through L1 (it is tiny and reused by every warp); weights bypass L1.
-// Small M uses large WPR so that the whole device has loads in flight for a handful of rows.
+// rowdot. A block owns a contiguous range of rows, the rows / blocks of them give or take one (pair, for gated units), and
+// has 8 / WPR groups of WPR warps. A pass gives every group ROWS rows, whose 16-byte chunks its 32*WPR lanes stride over
+// with U chunks in flight per lane per row. x is read through L1 (it is tiny and reused by every group); weights bypass L1.
+//
+// The grid is all blocks that are resident at once. Handing out rows in rounds instead (a grid of up to 6 blocks per
+// multiprocessor of which 4 fit) left a part of the blocks without work in the last round: bf16, 1 row of x, us before /
+// now: 12352 x 4096 23.6 / 16.9 (0.92 of the copy rate), 6144 x 4096 12.3 / 9.7, 22016 x 4096 gated 34.0 / 29.4,
+// 50272 x 4096 67.7 / 60.2, 11264 x 2048 gated 10.8 / 9.0; fp16 gathered, 4096 x 12288 19.1 / 18.5. Short lists are bound by
+// the chain launch, x and first weights, sums, store: 4096 x 4096 7.3 / 6.9, 2048 x 2048 2.8 either way.
 // -------------------------------------------------------------------------------------------
 constexpr int RD_THREADS = 256;
 constexpr int RD_WARPS = RD_THREADS / WARP;
+constexpr int RD_SPAN = 128;  // rows whose sums a block keeps before it finishes them
+
+// Blocks per multiprocessor that the registers of a pass leave room for: ROWS * U 16-byte loads, ROWS * B sums.
+__host__ __device__ constexpr int rd_blocks(int B) { return B == 1 ? 4 : B == 2 ? 3 : B <= 4 ? 2 : 1; }
 
 template <typename T, typename TO, int B, int ACT, int WPR, int ROWS, int U>
-__global__ void __launch_bounds__(RD_THREADS)
+__global__ void __launch_bounds__(RD_THREADS, rd_blocks(B))
 rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__ X,
               const void *__restrict__ idx, const T *__restrict__ bias, int M, int N,
-              long long ldw, int idx64, int early, float act_param) {
-  static_assert(!is_glu(ACT) || ROWS % 2 == 0, "a group owns whole (gate, up) pairs of rows");
+              long long ldw, int idx64, int early, float act_param, int per_block, int rest) {
+  constexpr int UNIT = is_glu(ACT) ? 2 : 1;  // rows 2i, 2i + 1 of the matrix are the gate and up rows of output i
   constexpr int GROUPS = RD_WARPS / WPR;
   constexpr int GLANES = WARP * WPR;
-  __shared__ float red[WPR > 1 ? RD_WARPS * ROWS * B : 1];
+  constexpr int SPAN = U == 4 ? 2 : RD_SPAN;  // (with 4 chunks per row a block has two rows at most)
+  __shared__ float red[B][SPAN][WPR];
 
   const int tid = threadIdx.x;
   const int warp = tid / WARP, lane = tid % WARP;
@@ -53,152 +63,147 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   const int glane = wig * WARP + lane;
   const int nchunks = N / Chunk<T>::N;
   const uint4 *Xv = reinterpret_cast<const uint4 *>(X);
+  const int units = M / UNIT;
+  const int bx = blockIdx.x;
+  const int first = (bx * per_block + min(bx, rest)) * UNIT;  // the first `rest` blocks have one more
+  const int last = first + (per_block + (bx < rest ? 1 : 0)) * UNIT;
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (early) {
-    // Weights are not produced by any kernel, and the index list is complete (identity, or the caller's
-    // promise): the first 8 KB of the first rows of this group are requested while the kernel before this
-    // one is still running.
-    const int m0 = blockIdx.x * GROUPS * ROWS + group * ROWS;
-    constexpr int LINES = 64;
+    // Weights are not produced by any kernel, and the index list is complete (identity, or the caller's promise): the
+    // first 8 KB of the block's rows are requested while the kernel before this one is still running. A prefetch can
+    // neither fault nor return a stale value, whatever the promise is worth.
+    constexpr int LINES = 64, MAX_ROWS = 16;
     const int row_lines = (int)min((long long)LINES, ((long long)N * (int)sizeof(T) + 127) / 128);
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if (m0 + j < M) {
-        const long long r = load_index(idx, m0 + j, idx64);
-        const char *w0 = reinterpret_cast<const char *>(W + r * ldw);
-        for (int l = glane; l < row_lines; l += GLANES) prefetch_l2(w0 + (size_t)l * 128);
-      }
+    for (int m = first + warp; m < min(last, first + MAX_ROWS); m += RD_WARPS) {
+      const char *w0 = reinterpret_cast<const char *>(W + load_index(idx, m, idx64) * ldw);
+      for (int l = lane; l < row_lines; l += WARP) prefetch_l2(w0 + (size_t)l * 128);
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  const int rows_per_pass = gridDim.x * GROUPS * ROWS;
-  // trip count is uniform over the block so that __syncthreads below is legal
-  for (int base = blockIdx.x * GROUPS * ROWS; base < M; base += rows_per_pass) {
-    const int m0 = base + group * ROWS;
-    const uint4 *wp[ROWS];
-    float bv[ROWS];
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      const int m = m0 + j;
-      const bool ok = m < M;
-      const long long r = ok ? load_index(idx, m, idx64) : 0;
-      wp[j] = reinterpret_cast<const uint4 *>(W + r * ldw);
-      bv[j] = (bias != nullptr && ok) ? to_f(bias[r]) : 0.f;
-      if (!ok) wp[j] = nullptr;
-    }
-    float acc[ROWS][B];
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j)
-#pragma unroll
-      for (int b = 0; b < B; ++b) acc[j][b] = 0.f;
+  // the bias of the row that this thread finishes in the first span, on its way while the products are made
+  const int outs0 = min(last - first, SPAN) / UNIT;
+  float bias0 = 0.f;
+  if (UNIT == 1 && bias != nullptr && tid < outs0) bias0 = to_f(bias[load_index(idx, first + tid, idx64)]);
 
-    for (int c0 = glane; c0 < nchunks; c0 += GLANES * U) {
-      uint4 wv[ROWS][U];
+  for (int s0 = first; s0 < last; s0 += SPAN) {  // (the same trips for all threads of the block)
+    const int s1 = min(last, s0 + SPAN);
+    for (int m0 = s0 + group * ROWS; m0 < s1; m0 += GROUPS * ROWS) {
+      const uint4 *wp[ROWS];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = c0 + u * GLANES;
-#pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-          if (c < nchunks && wp[j] != nullptr)
-            wv[j][u] = ld_stream16(wp[j] + c);
-          else
-            wv[j][u] = make_uint4(0, 0, 0, 0);
-        }
+      for (int j = 0; j < ROWS; ++j) {
+        const long long r = m0 + j < s1 ? load_index(idx, m0 + j, idx64) : -1;
+        wp[j] = r < 0 ? nullptr : reinterpret_cast<const uint4 *>(W + r * ldw);
       }
+      float acc[ROWS][B];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c = c0 + u * GLANES;
-        if (c < nchunks) {
+      for (int j = 0; j < ROWS; ++j)
 #pragma unroll
-          for (int b = 0; b < B; ++b) {
-            const uint4 xv = ld_cached16(Xv + (size_t)b * nchunks + c);
+        for (int b = 0; b < B; ++b) acc[j][b] = 0.f;
+      for (int c0 = glane; c0 < nchunks; c0 += GLANES * U) {
+        uint4 wv[ROWS][U];
 #pragma unroll
-            for (int j = 0; j < ROWS; ++j) acc[j][b] = dot_chunk<T>(wv[j][u], xv, acc[j][b]);
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + u * GLANES;
+#pragma unroll
+          for (int j = 0; j < ROWS; ++j)
+            wv[j][u] = (c < nchunks && wp[j] != nullptr) ? ld_stream16(wp[j] + c) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + u * GLANES;
+          if (c < nchunks) {
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+              const uint4 xv = ld_cached16(Xv + (size_t)b * nchunks + c);
+#pragma unroll
+              for (int j = 0; j < ROWS; ++j) acc[j][b] = dot_chunk<T>(wv[j][u], xv, acc[j][b]);
+            }
           }
         }
       }
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          const float v = warp_sum(acc[j][b]);
+          if (lane == 0 && m0 + j < s1) red[b][m0 + j - s0][wig] = v;
+        }
     }
+    __syncthreads();
+    const int outs = (s1 - s0) / UNIT;
+    for (int o = tid; o < outs * B; o += RD_THREADS) {
+      const int b = o / outs, i = o % outs;
+      float v[UNIT];
 #pragma unroll
-    for (int j = 0; j < ROWS; ++j)
+      for (int j = 0; j < UNIT; ++j) {
+        const int row = i * UNIT + j;
+        v[j] = 0.f;
 #pragma unroll
-      for (int b = 0; b < B; ++b) acc[j][b] = warp_sum(acc[j][b]);
-
-    if (WPR > 1) {
-      if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < ROWS; ++j)
-#pragma unroll
-          for (int b = 0; b < B; ++b) red[(warp * ROWS + j) * B + b] = acc[j][b];
+        for (int w2 = 0; w2 < WPR; ++w2) v[j] += red[b][row][w2];
+        if (UNIT == 1 && bias != nullptr)
+          v[j] += s0 == first && o == tid ? bias0 : to_f(bias[load_index(idx, s0 + row, idx64)]);
       }
-      __syncthreads();
-      if (wig == 0 && lane == 0) {
-#pragma unroll
-        for (int j = 0; j < ROWS; ++j)
-#pragma unroll
-          for (int b = 0; b < B; ++b) {
-            float s = 0.f;
-#pragma unroll
-            for (int w2 = 0; w2 < WPR; ++w2) s += red[((group * WPR + w2) * ROWS + j) * B + b];
-            acc[j][b] = s;
-          }
-      }
+      const size_t at = (size_t)b * units + s0 / UNIT + i;
+      if constexpr (is_glu(ACT)) Y[at] = from_f<TO>(apply_glu<ACT>(v[0], v[1], act_param));
+      else Y[at] = from_f<TO>(apply_act_param<ACT>(v[0], act_param));
     }
-    if (wig == 0 && lane == 0) {
-      if (is_glu(ACT)) {
-        // rows 2i, 2i + 1 of the matrix are the gate and up rows of output i
-#pragma unroll
-        for (int j = 0; j + 1 < ROWS; j += 2) {
-          const int m = m0 + j;
-          if (m + 1 < M) {
-#pragma unroll
-            for (int b = 0; b < B; ++b)
-              Y[(size_t)b * (M / 2) + m / 2] =
-                  from_f<TO>(apply_glu<ACT>(acc[j][b] + bv[j], acc[j + 1][b] + bv[j + 1], act_param));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-          const int m = m0 + j;
-          if (m < M) {
-#pragma unroll
-            for (int b = 0; b < B; ++b)
-              Y[(size_t)b * M + m] = from_f<TO>(apply_act_param<ACT>(acc[j][b] + bv[j], act_param));
-          }
-        }
-      }
-    }
-    if (WPR > 1) __syncthreads();  // red[] is reused by the next pass
+    if (s1 < last) __syncthreads();  // red[] is reused by the next span
   }
 }
 
 struct RowdotPlan {
-  int wpr, rows, grid;
+  int wpr, grid, per_block, rest;
+  bool few;  // at most two rows per block: 2 rows x 4 chunks per lane instead of 4 x 2
 };
 
-inline RowdotPlan plan_rowdot(int M, int nchunks, int B, int rows) {
-  const int sms = sm_count();
-  static const int k_wpr = env_int("DJV_RD_WPR", 0);  // development knobs
-  static const int k_cap = env_int("DJV_RD_BLOCKS_PER_SM", 6);
-  // As many warps per row as still lets every block be resident at once (4 blocks of 256 threads per SM):
-  // a second, partial wave of blocks costs more than fewer lanes per row (measured: K=4096, d=9216 runs at
-  // 0.77 of the HBM peak with 2 warps per row, 0.71 with 4, 0.67 with 1).
-  const long long resident = (long long)sms * 4;
-  int wpr = 1;
-  while (wpr < 8 && (long long)ceil_div(M, (RD_WARPS / (wpr * 2)) * rows) <= resident && nchunks >= 64 * wpr * 2)
-    wpr *= 2;
-  if (k_wpr > 0) {
-    wpr = k_wpr;
-    while (wpr > 1 && nchunks < 32 * wpr) wpr /= 2;
+// A block with p rows makes ceil(p / (groups * 4)) passes of ceil(nchunks / (64 * wpr)) trips of the chunk loop, and a pass
+// costs about one trip on top (row pointers, sums of the warps, a block barrier at the end). The least of the four is
+// within 3 % of the best of them at every shape above; of equals the one with fewer lanes per row has more rows under way.
+inline RowdotPlan plan_rowdot(int M, int nchunks, int unit, int B) {
+  static const int k_wpr = env_int("DJV_RD_WPR", 0);  // development knob
+  const int slots = sm_count() * rd_blocks(B), units = M / unit;
+  const int p = ceil_div(units, slots) * unit;
+  RowdotPlan r{};
+  r.few = B == 1 && p <= 2;
+  if (r.few)
+    for (r.wpr = 8; r.wpr > 1 && nchunks < WARP * r.wpr;) r.wpr /= 2;
+  long long best = -1;
+  for (int wpr = 1; wpr <= 8 && !r.few; wpr *= 2) {
+    const int passes = ceil_div(p, RD_WARPS / wpr * 4);
+    const long long cost = (long long)passes * (ceil_div(nchunks, WARP * wpr * 2) + 1);
+    if (best < 0 || cost < best) {
+      best = cost;
+      r.wpr = wpr;
+    }
   }
-  const int groups = RD_WARPS / wpr;
-  int grid = ceil_div(M, groups * rows);
-  const int cap = sms * k_cap;
-  if (grid > cap) grid = cap;
-  if (grid < 1) grid = 1;
-  return {wpr, rows, grid};
+  if (k_wpr > 0) r.wpr = k_wpr;
+  r.grid = max(1, min(slots, ceil_div(M, r.few ? 2 : unit)));
+  r.per_block = units / r.grid;
+  r.rest = units % r.grid;
+  return r;
 }
+
+// launch(WPR, ROWS, U) with compile-time arguments
+#define DJV_ROWDOT_WPR(plan, ROWS_, U_, LAUNCH)       \
+  do {                                                \
+    switch ((plan).wpr) {                             \
+      case 1: LAUNCH(1, ROWS_, U_); break;            \
+      case 2: LAUNCH(2, ROWS_, U_); break;            \
+      case 4: LAUNCH(4, ROWS_, U_); break;            \
+      default: LAUNCH(8, ROWS_, U_); break;           \
+    }                                                 \
+  } while (0)
+#define DJV_ROWDOT(plan, B_, LAUNCH)                  \
+  do {                                                \
+    if constexpr ((B_) == 1) {                        \
+      if ((plan).few) {                               \
+        DJV_ROWDOT_WPR(plan, 2, 4, LAUNCH);           \
+        break;                                        \
+      }                                               \
+    }                                                 \
+    DJV_ROWDOT_WPR(plan, 4, 2, LAUNCH);               \
+  } while (0)
 
 }  // namespace djv
