@@ -82,10 +82,10 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // the bias of the row that this thread finishes in the first span, on its way while the products are made
+  // the bias of the output that this thread finishes first, on its way while the products are made
   const int outs0 = min(last - first, SPAN) / UNIT;
   float bias0 = 0.f;
-  if (UNIT == 1 && bias != nullptr && tid < outs0) bias0 = to_f(bias[load_index(idx, first + tid, idx64)]);
+  if (UNIT == 1 && bias != nullptr && tid < outs0 * B) bias0 = to_f(bias[load_index(idx, first + tid % outs0, idx64)]);
 
   for (int s0 = first; s0 < last; s0 += SPAN) {  // (the same trips for all threads of the block)
     const int s1 = min(last, s0 + SPAN);
