@@ -10,6 +10,7 @@
 // Algorithmic bytes: QKV 3*a*hd*d*2 (+bias, x); attention 2*a*len*hd*2; out_proj d*a*hd*2 (+bias, ctx, y).
 #include <cooperative_groups.h>
 
+#include "attention_batch.cuh"
 #include "attn_state.cuh"
 #include "common.cuh"
 #include "push.cuh"
@@ -30,22 +31,9 @@ __global__ void attn_state_reset_kernel(int *st, int nheads, int prompt_len) {
 // Step 1 of djv_attn_step as a kernel of its own (see attn_prep_block).
 __global__ void __launch_bounds__(1024)
 attn_prep_kernel(int *__restrict__ st, const int *__restrict__ head_idx, int nnz,
-                 const __half *__restrict__ x, __half *__restrict__ x_ring, int d, int nheads, int S, int nseq,
-                 long long seq_ring) {
+                 const __half *__restrict__ x, __half *__restrict__ x_ring, int d, int nheads, int S) {
   pdl_prologue();
   attn_prep_block(st, head_idx, nnz, x, x_ring, d, nheads, S);
-  if (nseq > 1) {
-    // the other sequences of the batch share this state; each has its own window: x_ring[b][slot] = x[b]
-    __syncthreads();
-    if (st[ST_STATUS] != 0) return;
-    const int slot = st[ST_SLOT];
-    const int per = d / 8;
-    for (int c = threadIdx.x; c < (nseq - 1) * per; c += blockDim.x) {
-      const int b = 1 + c / per, k = c % per;
-      reinterpret_cast<uint4 *>(x_ring + (size_t)b * seq_ring + (size_t)slot * d)[k] =
-          reinterpret_cast<const uint4 *>(x + (size_t)b * d)[k];
-    }
-  }
 }
 
 __global__ void attn_finish_kernel(int *st) {
@@ -89,17 +77,7 @@ struct QkvArgs {
   const __half *x_cur;
   __half *x_ring_w;
   int early;  // MODE 1: the state is complete before this kernel can start; prefetch weights before the wait
-  // MODE 1 with nseq sequences that share the state (same head selection, same window): elements between two
-  // sequences' windows (x), query rows (q_out) and caches. Block (., y) takes sequences y*QKV_SEQ_GROUP ..: their
-  // token rows go through the same pass over the weight rows, 16 at a time.
-  int nseq;
-  long long seq_x, seq_q, seq_k, seq_v;
 };
-constexpr int QKV_SEQ_GROUP = 8;  // sequences per block
-// a token row of MODE 1: (sequence << 4) | window slot
-__device__ __forceinline__ int row_seq(int code) { return code >> 4; }
-__device__ __forceinline__ int row_slot(int code) { return code & (DJV_KV_WINDOW - 1); }
-static_assert(DJV_KV_WINDOW == 16, "token-row codes keep the window slot in 4 bits");
 
 // ROWS weight rows against NB token rows: every activation chunk is loaded (through L1) once and used for
 // all ROWS weight rows, so L1 traffic per weight byte is NB / ROWS. Without that sharing a head with three
@@ -165,10 +143,8 @@ __device__ __forceinline__ void qkv_mma_rows(const QkvArgs &a, int qkv, int h, i
   for (int j = 0; j < NT; ++j) {
     xr[j] = nullptr;
     if (j * 8 + g < nrows) {
-      const int code = rows_s[j * 8 + g];
-      const int r = (MODE == 1) ? row_slot(code) : code;
-      const __half *xs = (MODE == 1) ? a.x + (size_t)row_seq(code) * a.seq_x : a.x;
-      xr[j] = (MODE == 1 && a.x_cur != nullptr && r == cur_slot) ? a.x_cur : xs + (size_t)r * a.d;
+      const int r = rows_s[j * 8 + g];
+      xr[j] = (MODE == 1 && a.x_cur != nullptr && r == cur_slot) ? a.x_cur : a.x + (size_t)r * a.d;
     }
   }
 
@@ -221,19 +197,17 @@ __device__ __forceinline__ void qkv_mma_rows(const QkvArgs &a, int qkv, int h, i
     const int jj = jrow0 + tl * 16 + row;
     if (a.bias) sum += __half2float(a.bias[((size_t)qkv * a.nheads + h) * a.hd + jj]);
     const __half out = __float2half_rn(sum);
-    const int code = rows_s[tok];
-    const int trow = (MODE == 1) ? row_slot(code) : code;
-    const size_t sq = (MODE == 1) ? (size_t)row_seq(code) : 0;
+    const int trow = rows_s[tok];
     if (MODE == 0) {
       a.y[(((size_t)trow * 3 + qkv) * a.nheads + h) * a.hd + jj] = out;
     } else if (qkv == 1) {
       const int pos = base + trow;
-      a.k_cache[sq * a.seq_k + (((size_t)h * (a.hd / 8) + jj / 8) * a.S + pos) * 8 + jj % 8] = out;
+      a.k_cache[(((size_t)h * (a.hd / 8) + jj / 8) * a.S + pos) * 8 + jj % 8] = out;
     } else if (qkv == 2) {
       const int pos = base + trow;
-      a.v_cache[sq * a.seq_v + ((size_t)h * a.S + pos) * a.hd + jj] = out;
+      a.v_cache[((size_t)h * a.S + pos) * a.hd + jj] = out;
     } else {
-      a.q_out[sq * a.seq_q + (size_t)h * a.hd + jj] = out;
+      a.q_out[(size_t)h * a.hd + jj] = out;
     }
   }
 }
@@ -266,7 +240,7 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int U = (ROWS == 1) ? 8 : (ROWS == 2 ? 4 : 2);  // ROWS * U = 8 weight loads in flight per lane
   __shared__ float red[QKV_WARPS][ROWS][8];
-  __shared__ int rows_s[QKV_SEQ_GROUP * DJV_KV_WINDOW];
+  __shared__ int rows_s[DJV_KV_WINDOW];
   __shared__ int nrows_s;
 
   const int jblocks = a.hd / RPB;
@@ -300,13 +274,9 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
         if (r >= 0) rows_s[n++] = r;
       }
     } else {
-      // the sequences of this block, sequence-major (all of them have the same pending window slots)
-      const int seq0 = blockIdx.y * QKV_SEQ_GROUP;
-      const int seq1 = min(a.nseq > 0 ? a.nseq : 1, seq0 + QKV_SEQ_GROUP);
       const unsigned m = (qkv == 0) ? (1u << slot) : (unsigned)st_rowmask(a.state, a.nheads)[i];
-      for (int sq = seq0; sq < seq1; ++sq)
-        for (int s = 0; s <= slot; ++s)
-          if (m >> s & 1u) rows_s[n++] = (sq << 4) | s;
+      for (int s = 0; s <= slot; ++s)
+        if (m >> s & 1u) rows_s[n++] = s;
     }
     nrows_s = n;
   }
@@ -316,13 +286,8 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
   if constexpr (RPB >= 8) {
     // full or half tensor-core tiles; measured faster than the CUDA-core path below even for one token row
     __shared__ float red_mma[QKV_WARPS * 2 * 16 * 8];
-    // 16 token rows per pass over the block's weight rows (one pass unless several sequences have rows pending)
-    for (int r0 = 0; r0 < nrows; r0 += 16) {
-      const int nr = min(16, nrows - r0);
-      if (r0 > 0) __syncthreads();  // the reduction buffer of the pass before has been read
-      if (nr <= 8) qkv_mma_rows<MODE, RPB, 1>(a, qkv, h, jb * RPB, nr, rows_s + r0, base, slot, red_mma);
-      else qkv_mma_rows<MODE, RPB, 2>(a, qkv, h, jb * RPB, nr, rows_s + r0, base, slot, red_mma);
-    }
+    if (nrows <= 8) qkv_mma_rows<MODE, RPB, 1>(a, qkv, h, jb * RPB, nrows, rows_s, base, slot, red_mma);
+    else qkv_mma_rows<MODE, RPB, 2>(a, qkv, h, jb * RPB, nrows, rows_s, base, slot, red_mma);
     // (the CUDA-core path below is compiled for the one-row-per-block variant only)
   } else {
 
@@ -348,11 +313,9 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
     const uint4 *xp[NBMAX];
 #pragma unroll
     for (int r = 0; r < NBMAX; ++r) {
-      const int code = rows_s[r0 + (r < nb ? r : 0)];
-      const int tr = (MODE == 1) ? row_slot(code) : code;
-      const uint4 *xs = (MODE == 1) ? Xv + (size_t)row_seq(code) * (a.seq_x / 8) : Xv;
+      const int tr = rows_s[r0 + (r < nb ? r : 0)];
       xp[r] = (MODE == 1 && a.x_cur != nullptr && tr == slot) ? reinterpret_cast<const uint4 *>(a.x_cur)
-                                                              : xs + (size_t)tr * nchunks;
+                                                              : Xv + (size_t)tr * nchunks;
     }
     if (nb == 1) {
       const uint4 *x1[1] = {xp[0]};
@@ -407,19 +370,17 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
         const int j = j0 + jr;
         for (int r = 0; r < nb; ++r) {
           const __half out = __float2half_rn(acc[jr][r] + bv[jr]);
-          const int code = rows_s[r0 + r];
-          const int row = (MODE == 1) ? row_slot(code) : code;
-          const size_t sq = (MODE == 1) ? (size_t)row_seq(code) : 0;
+          const int row = rows_s[r0 + r];
           if (MODE == 0) {
             a.y[(((size_t)row * 3 + qkv) * a.nheads + h) * a.hd + j] = out;
           } else if (qkv == 0) {
-            a.q_out[sq * a.seq_q + (size_t)h * a.hd + j] = out;
+            a.q_out[(size_t)h * a.hd + j] = out;
           } else if (qkv == 1) {
             const int pos = base + row;
-            a.k_cache[sq * a.seq_k + (((size_t)h * (a.hd / 8) + j / 8) * a.S + pos) * 8 + j % 8] = out;
+            a.k_cache[(((size_t)h * (a.hd / 8) + j / 8) * a.S + pos) * 8 + j % 8] = out;
           } else {
             const int pos = base + row;
-            a.v_cache[sq * a.seq_v + ((size_t)h * a.S + pos) * a.hd + j] = out;
+            a.v_cache[((size_t)h * a.S + pos) * a.hd + j] = out;
           }
         }
       }
@@ -610,6 +571,7 @@ __global__ void __launch_bounds__(AT_THREADS) decode_attn_kernel(AttnArgs a) {
 // ------------------------------------------------------------------------------------------
 constexpr int OP_THREADS = 256;
 constexpr int OP_ROWS = 4;
+constexpr int OP_MAX_B = 4;  // rows of the context on the CUDA cores; more take out_proj_mma_kernel
 
 template <int HD, int B>
 __global__ void __launch_bounds__(OP_THREADS)
@@ -746,7 +708,7 @@ using namespace djv;
 // the largest that still gives every multiprocessor about two blocks. Very small calls put a whole block on
 // one row.
 template <int MODE>
-static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream_t st, int nseq = 1) {
+static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream_t st) {
   const long long sms = sm_count();
   // development knob, read at every launch: DJV_QKV_RPB (32, 16, 8 or 1: force the rows-per-block variant)
   const int force = env_int("DJV_QKV_RPB", 0);
@@ -755,8 +717,7 @@ static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream
   if (a.hd % rpb != 0) rpb = 8;
 #define DJV_QKV(WPR_, ROWS_)                                                                       \
   djv::launch_kernel(qkv_sparse_kernel<MODE, WPR_, ROWS_>,                                         \
-                     dim3(capacity_heads * 3 * (a.hd / ((QKV_WARPS / WPR_) * ROWS_)), (nseq + QKV_SEQ_GROUP - 1) / QKV_SEQ_GROUP), \
-                     QKV_THREADS, 0, st, a)
+                     dim3(capacity_heads * 3 * (a.hd / ((QKV_WARPS / WPR_) * ROWS_))), QKV_THREADS, 0, st, a)
   if (rpb == 32) DJV_QKV(1, 4);
   else if (rpb == 16) DJV_QKV(2, 4);
   else if (rpb == 8) DJV_QKV(2, 2);
@@ -807,7 +768,6 @@ static int launch_out_proj(int B, __half *Y, const __half *W, const __half *X, c
     case 2: DJV_OP(2); break;
     case 3: DJV_OP(3); break;
     case 4: DJV_OP(4); break;
-    case 8: DJV_OP(8); break;
     default: set_error("out_proj_sparse: internal batch slice %d", B); return DJV_ERR_INVALID;
   }
 #undef DJV_OP
@@ -824,19 +784,24 @@ extern "C" int djv_out_proj_sparse(void *y, const void *w, const void *x, const 
   DJV_REQUIRE(nnz >= 0 && nnz <= nheads, "out_proj_sparse: nnz=%d outside [0,%d]", nnz, nheads);
   DJV_REQUIRE(aligned16(w) && aligned16(x), "out_proj_sparse: w and x must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // slices of 8 rows of x while 8 are left, then of up to 4 (each slice reads the selected columns once)
-  for (int b0 = 0, bs = 0; b0 < B; b0 += bs) {
-    bs = (B - b0 >= 8) ? 8 : ((B - b0 < 4) ? (B - b0) : 4);
-    __half *Y = static_cast<__half *>(y) + (size_t)b0 * d;
-    const __half *X = static_cast<const __half *>(x) + (size_t)b0 * nheads * hd;
-    const __half *W = static_cast<const __half *>(w);
-    const __half *bi = static_cast<const __half *>(bias);
-    if (hd == 128) rc = launch_out_proj<128>(bs, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
-    else if (hd == 64) rc = launch_out_proj<64>(bs, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
-    else rc = launch_out_proj<32>(bs, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
-    if (rc) return rc;
+  __half *Y = static_cast<__half *>(y);
+  const __half *X = static_cast<const __half *>(x), *W = static_cast<const __half *>(w), *bi = static_cast<const __half *>(bias);
+  if (B > OP_MAX_B) {
+#define DJV_OM(HD_, NT_)                                                                                                   \
+  djv::launch_kernel(out_proj_mma_kernel<HD_, NT_>, dim3(ceil_div(d, OM_ROWS)), dim3(OM_THREADS), 0, st, Y, W, X, head_idx, \
+                     n_active_dev, bi, B, d, nheads, nnz)
+    if (hd == 128) B <= 8 ? DJV_OM(128, 1) : DJV_OM(128, 2);
+    else if (hd == 64) B <= 8 ? DJV_OM(64, 1) : DJV_OM(64, 2);
+    else B <= 8 ? DJV_OM(32, 1) : DJV_OM(32, 2);
+#undef DJV_OM
     count_launch();
+    return check_launch("out_proj_sparse");
   }
+  if (hd == 128) rc = launch_out_proj<128>(B, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
+  else if (hd == 64) rc = launch_out_proj<64>(B, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
+  else rc = launch_out_proj<32>(B, Y, W, X, head_idx, n_active_dev, bi, d, nheads, nnz, st);
+  if (rc) return rc;
+  count_launch();
   return check_launch("out_proj_sparse");
 }
 
@@ -956,11 +921,22 @@ static int attn_step_project(void *q_out, const void *wqkv, const void *bqkv, co
               "attn_step: pointers must be 16-byte aligned");
   DJV_REQUIRE(B == 1 || !step_is_open, "attn_step: a batch opens its step itself");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long seq_ring = (long long)DJV_KV_WINDOW * d;
+  const int typical = head_idx ? (nnz > 0 ? nnz : 1) : nheads;
   if (!step_is_open) {
+    // (with several sequences the projection puts the token rows into their windows)
     djv::launch_kernel(attn_prep_kernel, 1, 1024, 0, st, state, head_idx, head_idx ? nnz : 0,
-                       static_cast<const __half *>(x), static_cast<__half *>(x_ring), d, nheads, S, B, seq_ring);
+                       B == 1 ? static_cast<const __half *>(x) : nullptr, static_cast<__half *>(x_ring), d, nheads, S);
     count_launch();
+  }
+  if (B > 1) {
+    const QkvBatchArgs a{static_cast<const __half *>(wqkv), static_cast<const __half *>(bqkv), static_cast<const __half *>(x),
+                         static_cast<__half *>(x_ring), state, static_cast<__half *>(q_out), static_cast<__half *>(k_cache),
+                         static_cast<__half *>(v_cache), B, d, nheads, S};
+    rc = hd == 128 ? launch_qkv_batch<128>(a, typical, st) : hd == 64 ? launch_qkv_batch<64>(a, typical, st)
+                                                                      : launch_qkv_batch<32>(a, typical, st);
+    if (rc) return rc;
+    count_launch();
+    return check_launch("attn_step_project");
   }
   QkvArgs a{};
   a.w = static_cast<const __half *>(wqkv);
@@ -972,18 +948,12 @@ static int attn_step_project(void *q_out, const void *wqkv, const void *bqkv, co
   a.k_cache = static_cast<__half *>(k_cache);
   a.v_cache = static_cast<__half *>(v_cache);
   a.S = S;
-  a.nseq = B;
-  a.seq_x = seq_ring;
-  a.seq_q = (long long)nheads * hd;
-  a.seq_k = (long long)nheads * hd * S;
-  a.seq_v = (long long)nheads * hd * S;
   if (step_is_open) {
     a.x_cur = static_cast<const __half *>(x);
     a.x_ring_w = static_cast<__half *>(x_ring);
     a.early = early_prefetch() ? 1 : 0;
   }
-  const int typical = head_idx ? (nnz > 0 ? nnz : 1) : nheads;
-  launch_qkv<1>(a, nheads, (long long)typical * 3 * hd, st, B);
+  launch_qkv<1>(a, nheads, (long long)typical * 3 * hd, st);
   count_launch();
   return check_launch("attn_step_project");
 }

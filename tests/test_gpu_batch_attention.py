@@ -1,0 +1,65 @@
+"""The projections of a decode step of several sequences with one lazy-K/V state, against the same products in double."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# one rounding to fp16 behind fp32 sums (see test_gpu_decode_shapes)
+ROUNDING = 2 ** -11 + 2e-6
+
+
+def near(got, want):
+    err = (got.double() - want).abs().max().item()
+    assert err <= ROUNDING * max(1.0, want.abs().max().item()), err
+
+
+# token rows per pass (1 .. 64) and passes, columns that end inside a stage, fewer columns than a cluster has blocks
+@pytest.mark.parametrize("B,nheads,hd,d", [(2, 5, 32, 8), (3, 4, 64, 328), (5, 32, 128, 4096), (9, 3, 128, 1000), (16, 12, 64, 768),
+                                           (17, 2, 32, 72), (33, 2, 128, 136)])
+def test_lazy_projection_of_a_batch(cuda, B, nheads, hd, d):
+    from dejavu_b200 import _lib, ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + d)
+    prompt, steps = 5, 35
+    S = prompt + steps
+    w = (torch.randn(3, nheads, hd, d, device=cuda, generator=g) * d ** -0.5).half()
+    bias = torch.randn(3, nheads, hd, device=cuda, generator=g).half()
+    f16 = {"dtype": torch.float16, "device": cuda}
+    ring, q = torch.zeros(B, 16, d, **f16), torch.zeros(B, nheads, hd, **f16)
+    k, v = torch.zeros(B, nheads, hd // 8, S, 8, **f16), torch.zeros(B, nheads, S, hd, **f16)
+    want_k, want_v = (torch.zeros(B, nheads, S, hd, dtype=torch.float64, device=cuda) for _ in range(2))
+    state = torch.zeros(_lib.ATTN_STATE_HDR + 3 * nheads, dtype=torch.int32, device=cuda)
+    _lib.call("djv_attn_state_reset", state.data_ptr(), nheads, prompt, ops._stream())
+    waiting = [[] for _ in range(nheads)]  # (position, token rows) that a head has not seen
+    for t in range(steps):
+        x = torch.randn(B, d, device=cuda, generator=g).half()
+        few = torch.randperm(nheads, device=cuda, generator=g)[:max(1, nheads // 3)].int()
+        _lib.call("djv_attn_step_project_batch", q.data_ptr(), w.data_ptr(), bias.data_ptr(), x.data_ptr(), ring.data_ptr(),
+                  k.data_ptr(), v.data_ptr(), state.data_ptr(), few.data_ptr(), few.numel(), d, nheads, hd, S, B, ops._stream())
+        full = torch.einsum("bd,chjd->cbhj", x.double(), w.double()) + bias.double()[:, None]
+        heads = range(nheads) if t % 16 == 15 else few.tolist()
+        for h in range(nheads):
+            waiting[h].append((prompt + t, full[1:, :, h]))
+        for h in heads:
+            for pos, kv in waiting[h]:
+                want_k[:, h, pos], want_v[:, h, pos] = kv[0], kv[1]
+            waiting[h] = []
+        used = torch.tensor(sorted(heads), device=cuda)
+        near(q[:, used], full[0][:, used])
+        near(k.transpose(2, 3).reshape(B, nheads, S, hd), want_k)
+        near(v, want_v)
+        assert torch.equal(ring[:, t % 16], x)
+    assert state[3].item() == 0
+
+
+@pytest.mark.parametrize("B", [4, 5, 8, 9, 15, 16])
+@pytest.mark.parametrize("nheads,hd,d,nnz", [(4, 32, 128, 4), (7, 64, 384, 5), (32, 128, 4096, 12), (40, 128, 256, 33), (6, 32, 128, 0)])
+def test_output_projection_of_a_batch(cuda, B, nheads, hd, d, nnz):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + d)
+    w = (torch.randn(d, nheads, hd, device=cuda, generator=g) * max(1, nnz * hd) ** -0.5).half()
+    bias, x = torch.randn(d, device=cuda, generator=g).half(), torch.randn(B, nheads, hd, device=cuda, generator=g).half()
+    heads = torch.randperm(nheads, device=cuda, generator=g)[:nnz]
+    want = torch.einsum("bhj,nhj->bn", x[:, heads].double(), w[:, heads].double()) + bias.double()
+    near(ops.out_proj_sparse(x, w, heads.int(), bias), want)
