@@ -14,7 +14,7 @@
 #include "attn_state.cuh"
 #include "common.cuh"
 #include "push.cuh"
-#include "rowdot_mma.cuh"
+#include "mma.cuh"
 
 namespace djv {
 

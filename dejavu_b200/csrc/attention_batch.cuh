@@ -207,7 +207,7 @@ inline int qkv_batch_split(int heads, int d, int hd) {
 }
 
 template <int HD>
-inline int launch_qkv_batch(const QkvBatchArgs &a, int heads, cudaStream_t st) {
+static int launch_qkv_batch(const QkvBatchArgs &a, int heads, cudaStream_t st) {
   constexpr size_t smem = QkvBatchSmem<HD>::BYTES;
   static_assert(smem <= 113 * 1024, "shared memory of two blocks");
   static const cudaError_t prepared =

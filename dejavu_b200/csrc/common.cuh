@@ -82,6 +82,8 @@ inline cudaError_t launch_kernel_cluster(void (*kernel)(P...), dim3 grid, dim3 b
 // ---- device side --------------------------------------------------------------------------
 constexpr int WARP = 32;
 
+__host__ __device__ constexpr int ceil_div_dev(int a, int b) { return (a + b - 1) / b; }
+
 __device__ __forceinline__ void pdl_prologue() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

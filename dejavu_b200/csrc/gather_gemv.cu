@@ -76,46 +76,29 @@ static int rowdot_slice(int B, int act, __half *Y, const __half *W, const __half
   return DJV_ERR_INVALID;
 }
 
-template <int NT>
-static int launch_rowdot_mma(int act, __half *Y, const __half *W, const __half *X, const void *idx,
-                             const __half *bias, int M, int N, long long ldw, int idx64, int B, cudaStream_t st) {
-  static const int bps = [] {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rowdot_mma_kernel<__half, __half, NT, DJV_ACT_RELU>,
-                                                      MM_THREADS, 0) != cudaSuccess) {
-      cudaGetLastError();
-      n = 1;
-    }
-    return n < 1 ? 1 : n;
-  }();
-  const int tiles = ceil_div(M, MM_ROWS);
-  const int S = rowdot_mma_split(M, N, NT, bps);
-  const dim3 grid(tiles, S), cluster(1, S, 1);
-#define DJV_MM(ACT_)                                                                                          \
-  djv::launch_kernel_cluster(rowdot_mma_kernel<__half, __half, NT, ACT_>, grid, dim3(MM_THREADS), 0, st, cluster, \
-                             Y, W, X, idx, bias, M, N, ldw, idx64, B, 0.f)
-  switch (act) {
-    case DJV_ACT_ID: DJV_MM(DJV_ACT_ID); break;
-    case DJV_ACT_RELU: DJV_MM(DJV_ACT_RELU); break;
-    case DJV_ACT_GELU: DJV_MM(DJV_ACT_GELU); break;
-    case DJV_ACT_GELU_APPROX: DJV_MM(DJV_ACT_GELU_APPROX); break;
-    case DJV_ACT_SQUARED_RELU: DJV_MM(DJV_ACT_SQUARED_RELU); break;
-    default: set_error("gather_gemv: unknown activation %d", act); return DJV_ERR_INVALID;
-  }
-#undef DJV_MM
-  return DJV_OK;
-}
-
-// 9 <= B <= 32
-static int rowdot_mma(int B, int act, __half *Y, const __half *W, const __half *X, const void *idx,
-                      const __half *bias, int M, int N, long long ldw, int idx64, cudaStream_t st) {
+template <int ACT>
+static int rowdot_mma_act(int B, __half *Y, const __half *W, const __half *X, const void *idx, const __half *bias, int M, int N,
+                          long long ldw, int idx64, cudaStream_t st) {
   switch ((B + 7) / 8) {
-    case 1: return launch_rowdot_mma<1>(act, Y, W, X, idx, bias, M, N, ldw, idx64, B, st);
-    case 2: return launch_rowdot_mma<2>(act, Y, W, X, idx, bias, M, N, ldw, idx64, B, st);
-    case 3: return launch_rowdot_mma<3>(act, Y, W, X, idx, bias, M, N, ldw, idx64, B, st);
-    case 4: return launch_rowdot_mma<4>(act, Y, W, X, idx, bias, M, N, ldw, idx64, B, st);
+    case 1: return launch_rowdot_mma<__half, __half, 1, ACT>(Y, W, X, idx, bias, M, N, ldw, idx64, B, 0.f, st);
+    case 2: return launch_rowdot_mma<__half, __half, 2, ACT>(Y, W, X, idx, bias, M, N, ldw, idx64, B, 0.f, st);
+    case 3: return launch_rowdot_mma<__half, __half, 3, ACT>(Y, W, X, idx, bias, M, N, ldw, idx64, B, 0.f, st);
+    case 4: return launch_rowdot_mma<__half, __half, 4, ACT>(Y, W, X, idx, bias, M, N, ldw, idx64, B, 0.f, st);
   }
   set_error("gather_gemv: batch %d outside the tensor-core kernel's range", B);
+  return DJV_ERR_INVALID;
+}
+
+static int rowdot_mma(int B, int act, __half *Y, const __half *W, const __half *X, const void *idx,
+                      const __half *bias, int M, int N, long long ldw, int idx64, cudaStream_t st) {
+  switch (act) {
+    case DJV_ACT_ID: return rowdot_mma_act<DJV_ACT_ID>(B, Y, W, X, idx, bias, M, N, ldw, idx64, st);
+    case DJV_ACT_RELU: return rowdot_mma_act<DJV_ACT_RELU>(B, Y, W, X, idx, bias, M, N, ldw, idx64, st);
+    case DJV_ACT_GELU: return rowdot_mma_act<DJV_ACT_GELU>(B, Y, W, X, idx, bias, M, N, ldw, idx64, st);
+    case DJV_ACT_GELU_APPROX: return rowdot_mma_act<DJV_ACT_GELU_APPROX>(B, Y, W, X, idx, bias, M, N, ldw, idx64, st);
+    case DJV_ACT_SQUARED_RELU: return rowdot_mma_act<DJV_ACT_SQUARED_RELU>(B, Y, W, X, idx, bias, M, N, ldw, idx64, st);
+  }
+  set_error("gather_gemv: unknown activation %d", act);
   return DJV_ERR_INVALID;
 }
 
@@ -182,12 +165,11 @@ extern "C" int djv_gather_gemv(void *y, const void *w, const void *x, const void
   static const int k_mma_min_b = env_int("DJV_MMA_MIN_B", 3);         // development knobs
   static const int k_mma_always_b = env_int("DJV_MMA_ALWAYS_B", 5);
   static const int k_mma_min_tiles = env_int("DJV_MMA_MIN_TILES", 256);
-  if (B >= k_mma_always_b || (B >= k_mma_min_b && ceil_div(M, MM_ROWS) >= k_mma_min_tiles)) {
+  if (B >= k_mma_always_b || (B >= k_mma_min_b && ceil_div(M, 16) >= k_mma_min_tiles)) {
     rc = rowdot_mma(B, act, static_cast<__half *>(y), static_cast<const __half *>(w),
                     static_cast<const __half *>(x), idx, static_cast<const __half *>(bias), M, N, ldw,
                     idx_is_64, st);
     if (rc) return rc;
-    count_launch();
     return check_launch("gather_gemv");
   }
   for (int b0 = 0; b0 < B; b0 += 8) {

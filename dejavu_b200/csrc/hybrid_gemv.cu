@@ -44,41 +44,20 @@ static void launch_rowdot_dense(TO *Y, const T *W, const T *X, int M, int N, lon
   count_launch();
 }
 
-template <typename T, typename TO, int NT, int ACT>
-static void launch_mma_dense(TO *Y, const T *W, const T *X, int B, int M, int N, long long ldw, float param,
-                             cudaStream_t st) {
-  static const int bps = [] {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rowdot_mma_kernel<T, TO, NT, ACT>, MM_THREADS, 0) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      n = 1;
-    }
-    return n < 1 ? 1 : n;
-  }();
-  const int S = rowdot_mma_split(M, N, NT, bps);
-  djv::launch_kernel_cluster(rowdot_mma_kernel<T, TO, NT, ACT>, dim3(ceil_div(M, MM_ROWS), S), dim3(MM_THREADS), 0, st,
-                             dim3(1, S, 1), Y, W, X, static_cast<const void *>(nullptr),
-                             static_cast<const T *>(nullptr), M, N, ldw, 0, B, param);
-  count_launch();
-}
-
-// tensor cores for 5 rows of x and more, 16-bit element types only
+// 16-bit element types only: tensor cores for 5 rows of x and more, and for 3 and 4 where the weights are large. bf16, us on the
+// CUDA cores / tensor cores for 4 rows: 2048 x 2048 3.8 / 5.0, 4096 x 4096 9.8 / 8.2, 11264 x 2048 12.9 / 10.8, 22016 x 4096
+// 39.9 / 29.2; for 2 rows 4096 x 4096 9.2 / 8.4, 11264 x 2048 9.8 / 10.8, 22016 x 4096 30.3 / 29.1, 50272 x 4096 62.4 / 64.
+static bool takes_mma(int B, int M, int N) { return B >= 5 || (B >= 3 && (long long)M * N >= 1ll << 24); }
 template <typename TO, int ACT>
-static bool try_mma(TO *Y, const bf16 *W, const bf16 *X, int B, int M, int N, long long ldw, float param,
-                    cudaStream_t st) {
-  if (B < 5) return false;
+static int dense_mma(TO *Y, const bf16 *W, const bf16 *X, int B, int M, int N, long long ldw, float param, cudaStream_t st) {
+#define DJV_DM(NT_) launch_rowdot_mma<bf16, TO, NT_, ACT>(Y, W, X, nullptr, nullptr, M, N, ldw, 0, B, param, st)
   switch ((B + 7) / 8) {
-    case 1: launch_mma_dense<bf16, TO, 1, ACT>(Y, W, X, B, M, N, ldw, param, st); break;
-    case 2: launch_mma_dense<bf16, TO, 2, ACT>(Y, W, X, B, M, N, ldw, param, st); break;
-    case 3: launch_mma_dense<bf16, TO, 3, ACT>(Y, W, X, B, M, N, ldw, param, st); break;
-    default: launch_mma_dense<bf16, TO, 4, ACT>(Y, W, X, B, M, N, ldw, param, st); break;
+    case 1: return DJV_DM(1);
+    case 2: return DJV_DM(2);
+    case 3: return DJV_DM(3);
+    default: return DJV_DM(4);
   }
-  return true;
-}
-template <typename TO, int ACT>
-static bool try_mma(TO *, const float *, const float *, int, int, int, long long, float, cudaStream_t) {
-  return false;
+#undef DJV_DM
 }
 
 template <typename T, typename TO, int ACT>
@@ -90,7 +69,8 @@ static int dense(TO *Y, const T *W, const T *X, int B, int M, int N, long long l
     count_launch();
     return DJV_OK;
   }
-  if (try_mma<TO, ACT>(Y, W, X, B, M, N, ldw, param, st)) return DJV_OK;
+  if constexpr (sizeof(T) == 2)
+    if (takes_mma(B, M, N)) return dense_mma<TO, ACT>(Y, W, X, B, M, N, ldw, param, st);
   for (int b0 = 0; b0 < B; b0 += 4) {
     TO *y = Y + (size_t)b0 * M_out;
     const T *x = X + (size_t)b0 * N;

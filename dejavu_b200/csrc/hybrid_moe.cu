@@ -8,7 +8,7 @@
 
 #include "../../include/dejavu_b200_routed.h"
 #include "hybrid_moe.cuh"
-#include "mma.cuh"
+#include "weight_ring.cuh"
 
 namespace djv {
 
@@ -312,103 +312,20 @@ __global__ void __launch_bounds__(MO_THREADS) moe_decode_down_kernel(MoeDecodeAr
 }
 
 // ---- decode, several rows: every weight row is read once -----------------------------------------------------------
-// mma.sync tiles of 16 weight rows x 8 * NT sequences, the reduction split over the block's warps; weights and activations
-// are permuted along it the same way (see rowdot_mma.cuh). A sequence that did not choose the expert takes no part: its
-// products are not stored (up), or its activations are zeros (down, which adds up all experts in one accumulator).
-constexpr int MM_ROWS_TILE = 16, MM_B = 32;
+// Streamed by weight_ring.cuh. The up stage goes through the gate and up rows of all experts that any sequence chose, one
+// after another and the shared one last, dealt out evenly whatever expert they belong to; a sequence that did not choose the
+// expert of a row does not store that row's product. The down stage adds all experts up in one accumulator: its columns are
+// those of all experts in a row, and a sequence that did not choose an expert meets it with zeros.
+// 8 sequences, 8 experts of 3648 x 4096 and the shared one, us: up 114 -> 87 (75 at copy rate), down 83 -> 51 (38) (tiles of 16 rows and all
+// columns per block before, no loads under way while a block found its experts or added up).
+constexpr int MM_B = 32;
 
-template <int NT>
-__device__ __forceinline__ void mma_chunk(float (&acc)[NT][4], const uint4 &lo, const uint4 &hi, const uint4 (&x)[NT]) {
-#pragma unroll
-  for (int j = 0; j < NT; ++j) {
-    mma_m16n8k16_t<bf16>(acc[j], lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
-    mma_m16n8k16_t<bf16>(acc[j], lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
-  }
-}
-
-template <int NT>  // grid (tiles of 16 gate and up rows, experts and the shared one)
-__global__ void __launch_bounds__(MO_THREADS) moe_up_mma_kernel(MoeDecodeArgs a) {
-  __shared__ float red[MO_WARPS][NT][MM_ROWS_TILE][8], weight[MM_B];
-  __shared__ int slot[MM_B];
-  pdl_prologue();
-  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, e = blockIdx.y;
-  const bool shared = e == a.E;
-  const int rows = 2 * (shared ? a.F_shared : a.F), m0 = blockIdx.x * MM_ROWS_TILE;
-  if (m0 >= rows) return;
-  bool mine = false;
-  for (int b = warp; b < a.B; b += MO_WARPS) {  // the expert's place among the sequence's choices
-    int ahead = shared ? a.top : 0;
-    float z = 0.f;
-    if (!shared) {
-      z = a.z[(size_t)b * a.E + e];
-      for (int o = lane; o < a.E; o += WARP) {
-        const float v = a.z[(size_t)b * a.E + o];
-        ahead += v > z || (v == z && o < e);
-      }
-      ahead = (int)__reduce_add_sync(0xffffffffu, (unsigned)ahead);
-    }
-    const bool in = shared || ahead < a.top;
-    mine |= in;
-    if (lane == 0) {
-      slot[b] = in ? ahead : -1;
-      weight[b] = shared ? 1.f : sigmoid_f(z);
-    }
-  }
-  if (!__syncthreads_or(mine)) return;
-  const int g = lane / 4, t = lane % 4;
-  const bf16 *W = shared ? static_cast<const bf16 *>(a.shared_gu) : static_cast<const bf16 *>(a.w_gu) + (size_t)e * 2 * a.F * a.D;
-  const bool ok_lo = m0 + g < rows, ok_hi = m0 + g + 8 < rows;
-  const bf16 *w_lo = W + (size_t)(m0 + g) * a.D, *w_hi = w_lo + (size_t)8 * a.D, *X = static_cast<const bf16 *>(a.x);
-  float acc[NT][4] = {};
-  constexpr int U = 2;
-  const int kblocks = (a.D + 31) / 32;
-  for (int kb = warp; kb < kblocks; kb += MO_WARPS * U) {
-    uint4 lo[U], hi[U], x[U][NT];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = (kb + u * MO_WARPS) * 32 + t * 8;
-      const bool ok = k < a.D;
-      lo[u] = ok && ok_lo ? ld_stream16(w_lo + k) : make_uint4(0, 0, 0, 0);
-      hi[u] = ok && ok_hi ? ld_stream16(w_hi + k) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < NT; ++j)
-        x[u][j] = ok && j * 8 + g < a.B ? ld_cached16(X + (size_t)(j * 8 + g) * a.D + k) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) mma_chunk<NT>(acc, lo[u], hi[u], x[u]);
-  }
-#pragma unroll
-  for (int j = 0; j < NT; ++j)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) red[warp][j][g + (x / 2) * 8][2 * t + x % 2] = acc[j][x];
+// every block finds for itself: list [n] of experts in use, place [E][MM_B] of an expert among a sequence's choices or -1
+__device__ __forceinline__ int moe_in_use(const MoeDecodeArgs &a, int *list, signed char *place, int *n_list) {
+  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP;
+  for (int i = tid; i < a.E * MM_B / 4; i += WR_THREADS) reinterpret_cast<int *>(place)[i] = -1;
   __syncthreads();
-  const int slots = a.top + (a.shared_gu ? 1 : 0);
-  for (int o = tid; o < NT * MM_ROWS_TILE / 2 * 8; o += MO_THREADS) {  // (sequence group, gated unit, sequence)
-    const int c = o % 8, r = o / 8 % (MM_ROWS_TILE / 2) * 2, j = o / (MM_ROWS_TILE / 2 * 8), b = j * 8 + c;
-    if (b >= a.B || slot[b] < 0 || m0 + r >= rows) continue;
-    float gate = 0.f, up = 0.f;
-#pragma unroll
-    for (int w = 0; w < MO_WARPS; ++w) {
-      gate += red[w][j][r][c];
-      up += red[w][j][r + 1][c];
-    }
-    static_cast<bf16 *>(a.act)[((size_t)b * slots + slot[b]) * a.ld_act + (m0 + r) / 2] =
-        from_f<bf16>(silu_glu(weight[b] * gate, weight[b] * up));
-  }
-}
-
-template <int NT>  // grid (tiles of 16 rows, S), a cluster over the S parts of the reduction
-__global__ void __launch_bounds__(MO_THREADS) moe_down_mma_kernel(MoeDecodeArgs a, int slots) {
-  extern __shared__ int sm[];
-  __shared__ float red[MO_WARPS][NT][MM_ROWS_TILE][8], part[NT][MM_ROWS_TILE][8];
-  __shared__ int n_list;
-  pdl_prologue();
-  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, S = gridDim.y, sb = blockIdx.y;
-  int *list = sm;                                            // [E]: experts that any sequence chose
-  signed char *place = reinterpret_cast<signed char *>(list + a.E);  // [E][MM_B]: the expert's place among a sequence's choices
-  for (int i = tid; i < a.E * MM_B / 4; i += MO_THREADS) reinterpret_cast<int *>(place)[i] = -1;
-  __syncthreads();
-  for (int b = warp; b < a.B; b += MO_WARPS) {
+  for (int b = warp; b < a.B; b += WR_WARPS) {
     int e;
     float v;
     warp_topk(a.z + (size_t)b * a.E, a.E, a.top, e, v);
@@ -425,84 +342,177 @@ __global__ void __launch_bounds__(MO_THREADS) moe_down_mma_kernel(MoeDecodeArgs 
       if (used) list[n + __popc(mask & ((1u << lane) - 1))] = e0 + lane;
       n += __popc(mask);
     }
-    if (lane == 0) n_list = n;
+    if (lane == 0) *n_list = n;
   }
   __syncthreads();
-  const int g = lane / 4, t = lane % 4, m0 = blockIdx.x * MM_ROWS_TILE;
-  const bool ok_lo = m0 + g < a.D, ok_hi = m0 + g + 8 < a.D;
-  // blocks of 32 reduction elements of all experts in a row, then the shared one's
-  const int kf = (a.F + 31) / 32, routed = n_list * kf, total = routed + (slots > a.top ? (a.F_shared + 31) / 32 : 0);
-  const bf16 *act = static_cast<const bf16 *>(a.act);
-  float acc[NT][4] = {};
-  constexpr int U = NT == 1 ? 4 : 2;
-  const int stride = MO_WARPS * S;
-  for (int i0 = sb * MO_WARPS + warp; i0 < total; i0 += stride * U) {
-    uint4 lo[U], hi[U], x[U][NT];
+  return *n_list;
+}
+
+struct MoeUpSource {
+  const MoeDecodeArgs &a;
+  const int *list;
+  const signed char *place;
+  int n_list, slots, first, last, rows, S, rank;  // units (pairs of rows) of the cluster; weight rows of its tiles
+  const bf16 *row[WR_WP];
+  int k;
+
+  // the expert of a unit (E: the shared one), and the unit's number in it
+  __device__ __forceinline__ int expert(int &unit) const {
+    const int at = min(unit / a.F, n_list);
+    unit -= at * a.F;
+    return at < n_list ? list[at] : a.E;
+  }
+  __device__ __forceinline__ void seek(int t, int c) {
+    if (c == 0)
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int i = i0 + u * stride;
-      lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < NT; ++j) x[u][j] = make_uint4(0, 0, 0, 0);
-      if (i >= total) continue;
-      const bool shared = i >= routed;
-      const int at = shared ? 0 : i / kf, k = (i - (shared ? routed : at * kf)) * 32 + t * 8;
-      const int F = shared ? a.F_shared : a.F, e = shared ? 0 : list[at];
-      if (k >= F) continue;
-      const bf16 *w = (shared ? static_cast<const bf16 *>(a.shared_down) : static_cast<const bf16 *>(a.w_down) + (size_t)e * a.D * F) +
-                      (size_t)(m0 + g) * F + k;
-      if (ok_lo) lo[u] = ld_stream16(w);
-      if (ok_hi) hi[u] = ld_stream16(w + (size_t)8 * F);
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int b = j * 8 + g, s = b >= a.B ? -1 : (shared ? a.top : place[e * MM_B + b]);
-        if (s >= 0) x[u][j] = *reinterpret_cast<const uint4 *>(act + ((size_t)b * slots + s) * a.ld_act + k);
+      for (int i = 0; i < WR_WP; ++i) {
+        const int r = (int)threadIdx.x / WR_PPR + WR_RP * i;
+        int unit = first + (t * rows + r) / 2;
+        const bool ok = r < rows && unit < last;
+        row[i] = nullptr;
+        if (ok) {
+          const int e = expert(unit);
+          row[i] = (e == a.E ? static_cast<const bf16 *>(a.shared_gu) : static_cast<const bf16 *>(a.w_gu) + (size_t)e * 2 * a.F * a.D) +
+                   (size_t)(2 * unit + r % 2) * a.D;
+        }
       }
+    k = (c * S + rank) * WR_K + (int)threadIdx.x % WR_PPR * 8;
+  }
+  __device__ __forceinline__ const void *w(int i, bool &ok) const {
+    ok = k < a.D;
+    return row[i] != nullptr ? row[i] + (ok ? k : 0) : nullptr;
+  }
+  __device__ __forceinline__ const void *x(int i, bool &ok) const {
+    const int b = (int)threadIdx.x / WR_PPR + WR_RP * i;
+    ok = k < a.D;
+    return b < a.B ? static_cast<const bf16 *>(a.x) + (size_t)b * a.D + (ok ? k : 0) : nullptr;
+  }
+  __device__ __forceinline__ void begin(int) {}
+  __device__ __forceinline__ void store(int t, int pair, int b, float2 v) const {
+    int unit = first + t * rows / 2 + pair;
+    if (2 * pair >= rows || unit >= last) return;
+    const int e = expert(unit), s = e == a.E ? a.top : place[e * MM_B + b];
+    if (s < 0) return;
+    const float wt = e == a.E ? 1.f : sigmoid_f(a.z[(size_t)b * a.E + e]);
+    static_cast<bf16 *>(a.act)[((size_t)b * slots + s) * a.ld_act + unit] = from_f<bf16>(silu_glu(wt * v.x, wt * v.y));
+  }
+};
+
+struct MoeDownSource {
+  const MoeDecodeArgs &a;
+  const int *list;
+  const signed char *place;
+  int n_list, slots, first, last, rows, S, rank;  // rows of the cluster, of its tiles
+  // the chunk's number in its expert, the expert's chunks, row length and place in the list (n_list: the shared one), and of
+  // the thread's pieces the rows of weights and of activations (xs: whether the sequence chose the expert)
+  int j, kf, F, at, k;
+  const bf16 *row[WR_WP], *act[(MM_B + WR_RP - 1) / WR_RP];
+  bool xs[(MM_B + WR_RP - 1) / WR_RP];
+
+  __device__ __forceinline__ void enter(int t) {
+    const bool shared = at == n_list;
+    const int e = shared ? a.E : list[at];
+    F = shared ? a.F_shared : a.F;
+    kf = ceil_div_dev(F, WR_K);
+    const bf16 *base = shared ? static_cast<const bf16 *>(a.shared_down) : static_cast<const bf16 *>(a.w_down) + (size_t)e * a.D * a.F;
+#pragma unroll
+    for (int i = 0; i < WR_WP; ++i) {
+      const int r = (int)threadIdx.x / WR_PPR + WR_RP * i, m = first + t * rows + r;
+      row[i] = r < rows && m < last ? base + (size_t)m * F : nullptr;
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) mma_chunk<NT>(acc, lo[u], hi[u], x[u]);
-  }
-#pragma unroll
-  for (int j = 0; j < NT; ++j)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) red[warp][j][g + (x / 2) * 8][2 * t + x % 2] = acc[j][x];
-  __syncthreads();
-  for (int o = tid; o < NT * MM_ROWS_TILE * 8; o += MO_THREADS) {
-    const int c = o % 8, r = o / 8 % MM_ROWS_TILE, j = o / (MM_ROWS_TILE * 8);
-    float s = 0.f;
-#pragma unroll
-    for (int w = 0; w < MO_WARPS; ++w) s += red[w][j][r][c];
-    part[j][r][c] = s;
-  }
-  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-  if (S > 1) cluster.sync();
-  else __syncthreads();
-  if (sb == 0)
-    for (int o = tid; o < NT * MM_ROWS_TILE * 8; o += MO_THREADS) {
-      const int r = o % MM_ROWS_TILE, c = o / MM_ROWS_TILE % 8, j = o / (MM_ROWS_TILE * 8), b = j * 8 + c, m = m0 + r;
-      if (b >= a.B || m >= a.D) continue;
-      float s = a.init ? a.init[(size_t)b * a.D + m] : 0.f;
-      for (int q = 0; q < S; ++q) s += S > 1 ? cluster.map_shared_rank(&part[0][0][0], q)[(j * MM_ROWS_TILE + r) * 8 + c] : part[j][r][c];
-      a.y[(size_t)b * a.D + m] = s;
+    for (int i = 0; i < (MM_B + WR_RP - 1) / WR_RP; ++i) {
+      const int b = (int)threadIdx.x / WR_PPR + WR_RP * i;
+      const int s = b >= a.B ? -1 : shared ? a.top : place[e * MM_B + b];
+      xs[i] = s >= 0;
+      act[i] = b < a.B ? static_cast<const bf16 *>(a.act) + ((size_t)b * slots + max(s, 0)) * a.ld_act : nullptr;
     }
-  if (S > 1) cluster.sync();  // no block leaves while block 0 may still read its sums
+  }
+  __device__ __forceinline__ void seek(int t, int c) {
+    if (c == 0) {
+      j = rank;
+      at = 0;
+      enter(t);
+    } else {
+      j += S;
+    }
+    while (j >= kf && at < n_list) {  // (the list ends with the shared expert, or with the last chunk)
+      j -= kf;
+      ++at;
+      enter(t);
+    }
+    k = j * WR_K + (int)threadIdx.x % WR_PPR * 8;
+  }
+  __device__ __forceinline__ const void *w(int i, bool &ok) const {
+    ok = k < F;
+    return row[i] != nullptr ? row[i] + (ok ? k : 0) : nullptr;
+  }
+  __device__ __forceinline__ const void *x(int i, bool &ok) const {
+    ok = k < F && xs[i];
+    return act[i] != nullptr ? act[i] + (ok ? k : 0) : nullptr;
+  }
+  __device__ __forceinline__ void begin(int) {}
+  __device__ __forceinline__ void store(int t, int pair, int b, float2 v) const {
+    const int at = first + t * rows + 2 * pair;
+    if (2 * pair >= rows) return;
+    const size_t o = (size_t)b * a.D + at;
+    if (at < last) a.y[o] = v.x + (a.init ? a.init[o] : 0.f);
+    if (at + 1 < last) a.y[o + 1] = v.y + (a.init ? a.init[o + 1] : 0.f);
+  }
+};
+
+template <int NT, bool UP>
+__global__ void __launch_bounds__(WR_THREADS, WR_BPS) moe_ring_kernel(MoeDecodeArgs a, int slots) {
+  extern __shared__ __align__(128) unsigned char wr_smem[];
+  __shared__ int n_s;
+  int *list = reinterpret_cast<int *>(wr_smem + WeightRing<NT>::BYTES);
+  signed char *place = reinterpret_cast<signed char *>(list + a.E);
+  pdl_prologue();
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), cl = blockIdx.x / S, clusters = gridDim.x / S;
+  const int n = moe_in_use(a, list, place, &n_s);
+  const bool shared = a.shared_gu != nullptr;
+  const int units = UP ? n * a.F + (shared ? a.F_shared : 0) : a.D, per = units / clusters, rest = units % clusters;
+  const int first = cl * per + min(cl, rest), last = first + per + (cl < rest ? 1 : 0), rows_all = (last - first) * (UP ? 2 : 1);
+  const int tiles = ceil_div_dev(rows_all, WR_ROWS), rows = tiles ? ceil_div_dev(ceil_div_dev(rows_all, tiles), 2) * 2 : 0;
+  const int all = UP ? ceil_div_dev(a.D, WR_K) : n * ceil_div_dev(a.F, WR_K) + (shared ? ceil_div_dev(a.F_shared, WR_K) : 0);
+  const int chunks = rank < all ? (all - rank + S - 1) / S : 0;
+  if constexpr (UP) {
+    MoeUpSource src{a, list, place, n, slots, first, last, rows, S, rank};
+    weight_ring<bf16, NT>(src, tiles, chunks, a.B, wr_smem);
+  } else {
+    MoeDownSource src{a, list, place, n, slots, first, last, rows, S, rank};
+    weight_ring<bf16, NT>(src, tiles, chunks, a.B, wr_smem);
+  }
+}
+
+template <int NT, bool UP>
+static int launch_ring(const MoeDecodeArgs &a, int slots, cudaStream_t st) {
+  static int resident[4];
+  static const cudaError_t prepared = [] {
+    const cudaError_t e = ring_residency<NT>(moe_ring_kernel<NT, UP>, resident);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(moe_ring_kernel<NT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   WeightRing<NT>::BYTES + 40 * 1024);
+  }();
+  if (prepared != cudaSuccess) {
+    set_error("moe_decode: %s", cudaGetErrorString(prepared));
+    return DJV_ERR_CUDA;
+  }
+  // (which experts are in use is known on the device only: as many as there can be)
+  const int n = a.E < a.B * a.top ? a.E : a.B * a.top, kf = ceil_div(a.F, WR_K), kf_shared = ceil_div(a.F_shared, WR_K);
+  const RingPlan p = UP ? ring_plan(n * a.F + a.F_shared, 2, ceil_div(a.D, WR_K), resident)
+                        : ring_plan(a.D, 1, n * kf + kf_shared, resident);
+  djv::launch_kernel_cluster(moe_ring_kernel<NT, UP>, dim3(p.clusters * p.S), dim3(WR_THREADS),
+                             WeightRing<NT>::BYTES + (size_t)a.E * (4 + MM_B), st, dim3(p.S), a, slots);
+  count_launch();
+  return DJV_OK;
 }
 
 template <int NT>
-static void launch_mma(const MoeDecodeArgs &a, int slots, int fmax, bool up, bool down, cudaStream_t st) {
-  if (up) {
-    djv::launch_kernel(moe_up_mma_kernel<NT>, dim3(ceil_div(2 * fmax, MM_ROWS_TILE), a.E + (a.shared_gu ? 1 : 0)), dim3(MO_THREADS),
-                       0, st, a);
-    count_launch();
-  }
-  if (down) {
-    const int tiles = ceil_div(a.D, MM_ROWS_TILE);
-    int S = 1;
-    while (S < 8 && tiles * S < 4 * sm_count()) S *= 2;
-    djv::launch_kernel_cluster(moe_down_mma_kernel<NT>, dim3(tiles, S), dim3(MO_THREADS), (size_t)a.E * (4 + MM_B), st,
-                               dim3(1, S, 1), a, slots);
-    count_launch();
-  }
+static int launch_mma(const MoeDecodeArgs &a, int slots, bool up, bool down, cudaStream_t st) {
+  const int rc = up ? launch_ring<NT, true>(a, slots, st) : DJV_OK;
+  return rc || !down ? rc : launch_ring<NT, false>(a, slots, st);
 }
 
 template <typename T>
@@ -515,13 +525,14 @@ static int launch_decode(const MoeDecodeArgs &a, bool up, bool down, cudaStream_
   if constexpr (sizeof(T) == 2) {
     // several rows share weights (both stages take this form or neither: they agree on where a choice's activations are)
     if (a.B >= 2 && a.B <= MM_B && vec_up && vec_down && (size_t)a.E * (4 + MM_B) <= 40 * 1024) {
+      int rc;
       switch ((a.B + 7) / 8) {
-        case 1: launch_mma<1>(a, slots, fmax, up, down, st); break;
-        case 2: launch_mma<2>(a, slots, fmax, up, down, st); break;
-        case 3: launch_mma<3>(a, slots, fmax, up, down, st); break;
-        default: launch_mma<4>(a, slots, fmax, up, down, st); break;
+        case 1: rc = launch_mma<1>(a, slots, up, down, st); break;
+        case 2: rc = launch_mma<2>(a, slots, up, down, st); break;
+        case 3: rc = launch_mma<3>(a, slots, up, down, st); break;
+        default: rc = launch_mma<4>(a, slots, up, down, st); break;
       }
-      return check_launch("moe_decode");
+      return rc ? rc : check_launch("moe_decode");
     }
   }
   if (up) {

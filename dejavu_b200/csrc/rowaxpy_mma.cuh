@@ -22,7 +22,7 @@
 // slower: 43 us against 40 at 8 activation rows and 6144 gathered rows of 12288 columns, 55 against 47 at 32 rows.)
 #pragma once
 #include "common.cuh"
-#include "rowdot_mma.cuh"
+#include "mma.cuh"
 
 namespace djv {
 

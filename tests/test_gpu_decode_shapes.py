@@ -45,3 +45,52 @@ def test_gathered_rows_split_over_resident_blocks(cuda, B, N, Z, M):
     want = (x.double() @ w[idx].double().t() + bias[idx].double()).relu()
     near(ops.gather_gemv(x, w, idx.int(), bias, "relu"), want)
     near(ops.gather_gemv(x, w, idx, bias, "relu"), want)
+
+
+# the ring: parts of a tile, several tiles, a column tail, one chunk and fewer than a cluster has blocks, 1 to 4 groups of x
+@pytest.mark.parametrize("B", [3, 5, 8, 9, 17, 32])
+@pytest.mark.parametrize("N,M", [(8, 2), (128, 34), (136, 592), (1000, 1186), (4104, 4096), (2056, 12352), (264, 75778)])
+def test_weights_streamed_for_several_rows(cuda, B, N, M):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + N + M)
+    x = torch.randn(B, N, device=cuda, generator=g).bfloat16()
+    w = (torch.randn(M, N, device=cuda, generator=g) * N ** -0.5).bfloat16()
+    y = x.double() @ w.double().t()
+    near(ops.linear_gemv(x, w, torch.float32), y)
+    near(ops.linear_gemv(x, w), y)
+    gate, up = y[:, 0::2], y[:, 1::2]
+    near(ops.linear_gemv(x, w, None, "silu_glu"), gate * torch.sigmoid(gate) * up)
+    bias = torch.randn(M, device=cuda, generator=g).half()
+    idx = torch.randperm(M, device=cuda, generator=g)[:M - 1]
+    want = (x.half().double() @ w.half()[idx].double().t() + bias[idx].double()).relu()
+    near(ops.gather_gemv(x.half(), w.half(), idx, bias, "relu"), want)
+
+
+@pytest.mark.parametrize("B,E,top,D,F,Fs", [(2, 1, 1, 8, 8, 0), (3, 5, 2, 136, 24, 40), (8, 8, 2, 512, 200, 328), (9, 40, 3, 264, 136, 8),
+                                            (17, 4, 4, 1032, 72, 0), (32, 300, 1, 64, 16, 16)])
+def test_routed_weights_streamed_for_several_rows(cuda, B, E, top, D, F, Fs):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + E + D)
+
+    def rnd(*shape):
+        return torch.randn(*shape, device=cuda, generator=g).mul_(shape[-1] ** -0.5).bfloat16()
+
+    x, z = torch.randn(B, D, device=cuda, generator=g).bfloat16(), torch.randn(B, E, device=cuda, generator=g)
+    gu, down = rnd(E, 2 * F, D), rnd(E, D, F)
+    shared = (rnd(2 * Fs, D), rnd(D, Fs)) if Fs else (None, None)
+    got = ops.moe_decode(x, z, gu, down, top, *shared)
+
+    def unit(v, up, dn):  # the activation is kept in bf16, as it was before
+        p = v @ up.double().t()
+        a = p[:, 0::2] * torch.sigmoid(p[:, 0::2]) * p[:, 1::2]
+        return a.bfloat16().double() @ dn.double().t()
+
+    want = unit(x.double(), *shared) if Fs else torch.zeros(B, D, dtype=torch.float64, device=cuda)
+    w, idx = torch.sigmoid(z.double()).topk(top, 1)
+    for b in range(B):
+        for k in range(top):
+            want[b] += unit(w[b, k] * x[b:b + 1].double(), gu[idx[b, k]], down[idx[b, k]])[0]
+    # an activation on the edge of two bf16 values may round the other way: 2^-8 of itself, among F * (top + 1) that add up
+    assert (got.double() - want).norm() <= 2e-3 * want.norm()
