@@ -49,6 +49,7 @@ SIGNATURES = {
     "djv_out_proj_sparse": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "djv_k_cache_copy_sparse": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _ll, _ll, _vp]),
     "djv_v_cache_copy_sparse": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _ll, _ll, _vp]),
+    "djv_kv_store": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "djv_attn_state_reset": (_i, [_vp, _i, _i, _vp]),
     "djv_attn_step_scratch_bytes": (_sz, [_i, _i, _i]),
     "djv_attn_step": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),

@@ -229,7 +229,9 @@ class GPTLMHeadModel(nn.Module, GenerationMixin):
     def tie_weights(self):
         self.lm_head.weight = self.transformer.embeddings.word_embeddings.weight
 
-    def forward(self, input_ids, position_ids=None, inference_params=None):
+    selects_logit_rows = True  # forward(logit_rows=...) computes logits at those tokens only
+
+    def forward(self, input_ids, position_ids=None, inference_params=None, logit_rows=None):
         # A decode step of several sequences runs kernels of several waves of blocks: programmatic dependent launch
         # then costs more than it hides (see djv_set_programmatic_launch), so the step's kernels are launched plain.
         plain = (input_ids.is_cuda and input_ids.size(0) > 1 and input_ids.size(1) == 1
@@ -237,16 +239,25 @@ class GPTLMHeadModel(nn.Module, GenerationMixin):
         if plain:
             _lib.load().djv_set_programmatic_launch(0)
         try:
-            return self._forward(input_ids, position_ids, inference_params)
+            return self._forward(input_ids, position_ids, inference_params, logit_rows)
         finally:
             if plain:
                 _lib.load().djv_set_programmatic_launch(1)
 
-    def _forward(self, input_ids, position_ids=None, inference_params=None):
+    def _forward(self, input_ids, position_ids=None, inference_params=None, logit_rows=None):
         hidden_states = self.transformer(input_ids, position_ids=position_ids, inference_params=inference_params)
+        n = hidden_states.size(1)
+        if logit_rows is not None:  # places among the tokens whose logits are wanted
+            rows = list(logit_rows)
+            if len(rows) == 1 and -n <= rows[0] < n:
+                hidden_states = hidden_states.narrow(1, rows[0] % n, 1)
+            elif rows != list(range(n)):
+                hidden_states = hidden_states[:, rows]
         B, L, d = hidden_states.shape
-        if L == 1 and hidden_states.is_cuda and B <= 32:
-            lm_logits = ops.dense_gemv(hidden_states.view(B, d), self.lm_head.weight).view(B, 1, -1)
+        weight = self.lm_head.weight
+        if L == 1 and hidden_states.is_cuda and B <= 32 and (
+                n == 1 or (d % 8 == 0 and self.lm_head.bias is None and modules._inference_fp16(hidden_states, weight))):
+            lm_logits = ops.dense_gemv(hidden_states.reshape(B, d), weight).view(B, 1, -1)
         else:
             lm_logits = self.lm_head(hidden_states)
         world = _world(self.process_group)

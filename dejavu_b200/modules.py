@@ -161,6 +161,11 @@ def _rank(pg) -> int:
     return 0 if pg is None else pg.rank()
 
 
+def _inference_fp16(*tensors) -> bool:
+    """Whether a prompt pass may take kernels that autograd does not know: fp16 on the GPU, no gradients recorded."""
+    return not torch.is_grad_enabled() and all(t.is_cuda and t.dtype == torch.float16 for t in tensors)
+
+
 def all_reduce(x: torch.Tensor, process_group) -> torch.Tensor:
     """SUM over the tensor-parallel group (flash_attn.utils.distributed.all_reduce at
     Dejavu/src/models/modules/mha_dejavu.py:1498, fused_dense_sparse_dejavu.py:940)."""
@@ -520,8 +525,12 @@ class ParallelMHASparseAttMlp(nn.Module):
             off = inference_params.sequence_len_offset
             assert off == 0 and L <= S
             # K cache (B, n, hd/8, S, 8), V cache (B, n, S, hd)   (mha_dejavu.py:385-447)
-            k_cache[:, :, :, :L, :] = k.permute(0, 2, 3, 1).reshape(B, n, hd // 8, 8, L).permute(0, 1, 2, 4, 3)
-            v_cache[:, :, :L, :] = v.permute(0, 2, 1, 3)
+            if (_inference_fp16(qkv, k_cache, v_cache) and hd in (32, 64, 128) and k_cache.size(0) == B
+                    and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (qkv, k_cache, v_cache))):
+                ops.kv_store(k_cache, v_cache, qkv)
+            else:
+                k_cache[:, :, :, :L, :] = k.permute(0, 2, 3, 1).reshape(B, n, hd // 8, 8, L).permute(0, 1, 2, 4, 3)
+                v_cache[:, :, :L, :] = v.permute(0, 2, 1, 3)
             self.reset_decode_state(L, x.device, S, B)
         ctx = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2),
                                              is_causal=True, scale=self.softmax_scale)

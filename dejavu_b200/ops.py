@@ -452,6 +452,17 @@ def add_layernorm(x, residual, weight, bias, eps: float, xbias=None):
     return y, r
 
 
+def kv_store(k_cache, v_cache, qkv):
+    """Keys and values of a prompt, qkv (B, L, 3, nheads, hd), into positions 0 .. L-1 of the caches
+    (B, nheads, hd/8, S, 8) and (B, nheads, S, hd) (mha_dejavu.py:385-447)."""
+    B, L, _, nheads, hd = qkv.shape
+    S = v_cache.shape[2]
+    assert v_cache.shape == (B, nheads, S, hd) and k_cache.shape == (B, nheads, hd // 8, S, 8) and 1 <= L <= S
+    assert all(t.dtype == torch.float16 and t.is_contiguous() for t in (k_cache, v_cache, qkv))
+    _require_cuda(k_cache, v_cache, qkv)
+    call("djv_kv_store", k_cache.data_ptr(), v_cache.data_ptr(), qkv.data_ptr(), B, L, nheads, hd, S, _stream())
+
+
 def decode_attention(q, k_cache, v_cache, head_idx, length: int, softmax_scale: float):
     """ctx[b,h] = softmax(scale * q[b,h] . K[b,h,:length]) V[b,h,:length] for h in head_idx (or all heads
     when head_idx is None); rows of other heads are uninitialised. q (B, nheads, hd);

@@ -257,6 +257,10 @@ int djv_v_cache_copy_sparse(const void *v, void *v_cache, const int32_t *head_id
 #define DJV_ATTN_STATE_HDR 8
 #define DJV_ATTN_STATE_WORDS(nheads) (DJV_ATTN_STATE_HDR + 3 * (nheads))
 
+/* Keys and values of a prompt into positions 0 .. L-1 of the caches: qkv (B,L,3,nheads,hd) contiguous, k_cache
+ * (B,nheads,hd/8,S,8), v_cache (B,nheads,S,hd), fp16, 16-byte aligned, hd 32, 64 or 128 (mha_dejavu.py:385-447). */
+int djv_kv_store(void *k_cache, void *v_cache, const void *qkv, int B, int L, int nheads, int hd, int S, void *stream);
+
 /* state := {slot 0, base = prompt_len, nothing pending}. */
 int djv_attn_state_reset(int32_t *state, int nheads, int prompt_len, void *stream);
 
