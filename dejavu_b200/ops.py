@@ -25,7 +25,7 @@ _scratch_cache: dict = {}
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # (without a Stream object for each call)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -38,9 +38,9 @@ def _require_cuda(*tensors):
             raise RuntimeError("dejavu_b200 operators run on CUDA tensors only (there is no CPU path)")
 
 
-def _scratch(nbytes: int, device: torch.device) -> torch.Tensor:
+def _scratch(nbytes: int, device: torch.device, stream: Optional[int] = None) -> torch.Tensor:
     """Zero-initialised per-(device, stream) workspace; the kernels leave their counters zeroed."""
-    key = (device.index, _stream())
+    key = (device.index, _stream() if stream is None else stream)
     buf = _scratch_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         size = max(nbytes, 1 << 20)
@@ -172,6 +172,23 @@ def dense_transposed_gemv(x: torch.Tensor, weight_t: torch.Tensor, bias: Optiona
     return output
 
 
+def _mlp_sparse_call(x, W1, W2t, idx, bias1, bias2):
+    """Both products of mlp_sparse behind one call into the library, one workspace for the hidden values and the result."""
+    batch, N = x.shape
+    M = idx.shape[0]
+    lib = _lib.load()
+    need = lib.djv_gather_transposed_gemv_scratch_bytes(batch, N, M)
+    if batch <= 4:
+        need = max(need, lib.djv_mlp_sparse_fused_scratch_bytes(batch, N, M))
+    stream = _stream()
+    scratch = _scratch(need, x.device, stream)
+    hidden, output = x.new_empty(batch, M), x.new_empty(batch, N)
+    call("djv_mlp_sparse", output.data_ptr(), hidden.data_ptr(), W1.data_ptr(), W2t.data_ptr(), x.data_ptr(), idx.data_ptr(),
+         _ptr(bias1), _ptr(bias2), batch, N, M, W1.stride(0), W2t.stride(0), 1 if idx.dtype == torch.int64 else 0,
+         scratch.data_ptr(), scratch.numel(), stream)
+    return output
+
+
 def mlp_sparse(x, W1, W2t, idx, bias1=None, bias2=None, push_comm=None, fused=False):
     """x (batch, d); W1 (4d, d); W2t (4d, d) = W2 transposed, contiguous; bias1 (4d); bias2 (d).
     gather_gemv followed by gather_transposed_gemv, as in the reference; with fused=True one kernel and one pass
@@ -185,6 +202,14 @@ def mlp_sparse(x, W1, W2t, idx, bias1=None, bias2=None, push_comm=None, fused=Fa
         assert x.dtype == W1.dtype == W2t.dtype == torch.float16 and W1.stride(1) == 1 and W2t.stride(1) == 1
         assert W1.shape[1] == N and W2t.shape[1] == N
     if not fused:
+        tensors = [t for t in (x, W1, W2t, bias1, bias2) if t is not None]
+        if (push_comm is None and 1 <= batch <= _lib.MAX_BATCH and W1.shape[1] == N == W2t.shape[1] and W1.stride(1) == 1
+                and W2t.stride(1) == 1 and all(t.is_cuda and t.dtype == torch.float16 for t in tensors)
+                and idx.is_cuda and idx.dtype in (torch.int32, torch.int64) and idx.is_contiguous() and x.is_contiguous()
+                and (bias1 is None or (bias1.shape == W1.shape[:1] and bias1.is_contiguous()))
+                and (bias2 is None or (bias2.shape == (N,) and bias2.is_contiguous()))):
+            return _mlp_sparse_call(x, W1, W2t, idx, bias1, bias2)
+        # other forms, and what is refused: one product at a time
         x = gather_gemv(x, W1, idx, bias1, activation="relu")
         return gather_transposed_gemv(x, W2t, idx, bias2, push_comm=push_comm)
     _require_cuda(x, W1, W2t, idx, bias1, bias2)
