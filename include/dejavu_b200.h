@@ -293,7 +293,7 @@ int djv_attn_step_project(void *q_out, const void *wqkv, const void *bqkv, const
  * list for all rows of a batch) and therefore one window position and one set of pending rows. Per-sequence data is
  * contiguous over the batch: q_out / q / ctx (B,nheads,hd), x (B,d), x_ring (B,16,d), k_cache (B,nheads,hd/8,S,8),
  * v_cache (B,nheads,S,hd); scratch >= djv_decode_attn_scratch_bytes(nheads, B, hd, S). One launch each whatever B
- * is: the blocks of all sequences that work on the same weight rows run side by side and share them through L2. */
+ * is: a head's weights are read once for the pending token rows of all sequences. */
 int djv_attn_step_project_batch(void *q_out, const void *wqkv, const void *bqkv, const void *x, void *x_ring,
                                 void *k_cache, void *v_cache, int32_t *state, const int32_t *head_idx, int nnz,
                                 int d, int nheads, int hd, int S, int B, void *stream);
