@@ -210,8 +210,11 @@ template <int HD>
 static int launch_qkv_batch(const QkvBatchArgs &a, int heads, cudaStream_t st) {
   constexpr size_t smem = QkvBatchSmem<HD>::BYTES;
   static_assert(smem <= 113 * 1024, "shared memory of two blocks");
-  static const cudaError_t prepared =
-      cudaFuncSetAttribute(qkv_batch_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static DevicePrep prep;
+  const int (*unused)[4];
+  const cudaError_t prepared = prep.get([](int (&)[4]) {
+    return cudaFuncSetAttribute(qkv_batch_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  }, unused);
   if (prepared != cudaSuccess) {
     set_error("attn_step: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;

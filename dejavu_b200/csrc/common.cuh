@@ -6,6 +6,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <mutex>
+
 #include "../../include/dejavu_b200.h"
 
 namespace djv {
@@ -78,6 +80,33 @@ inline cudaError_t launch_kernel_cluster(void (*kernel)(P...), dim3 grid, dim3 b
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+
+// What a kernel's first launch on a device sets and asks (attributes are per device): `prepare` runs once for each, and fills
+// in how many clusters of 1, 2, 4, 8 blocks are resident where that matters. One static object per kernel.
+class DevicePrep {
+ public:
+  template <typename F>
+  cudaError_t get(F prepare, const int (*&resident)[4]) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= MAX) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> hold(mutex_);
+    if (!done_[dev]) {
+      e = prepare(resident_[dev]);
+      if (e != cudaSuccess) return e;
+      done_[dev] = true;
+    }
+    resident = &resident_[dev];
+    return cudaSuccess;
+  }
+
+ private:
+  static constexpr int MAX = 64;
+  std::mutex mutex_;
+  bool done_[MAX] = {};
+  int resident_[MAX][4] = {};
+};
 
 // ---- device side --------------------------------------------------------------------------
 constexpr int WARP = 32;

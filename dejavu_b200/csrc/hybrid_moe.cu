@@ -316,8 +316,9 @@ __global__ void __launch_bounds__(MO_THREADS) moe_decode_down_kernel(MoeDecodeAr
 // after another and the shared one last, dealt out evenly whatever expert they belong to; a sequence that did not choose the
 // expert of a row does not store that row's product. The down stage adds all experts up in one accumulator: its columns are
 // those of all experts in a row, and a sequence that did not choose an expert meets it with zeros.
-// 8 sequences, 8 experts of 3648 x 4096 and the shared one, us: up 114 -> 87 (75 at copy rate), down 83 -> 51 (38) (tiles of 16 rows and all
-// columns per block before, no loads under way while a block found its experts or added up).
+// 8 sequences, 8 experts of 3648 x 4096 and the shared one, us: up 114 -> 87 (75 at copy rate), down 83 -> 51 (38). Before,
+// a block took 16 rows and all columns, with no loads under way while it found its experts or added up. (Finding a chunk's
+// expert by a division for every chunk cost the down stage 24 us.)
 constexpr int MM_B = 32;
 
 // every block finds for itself: list [n] of experts in use, place [E][MM_B] of an expert among a sequence's choices or -1
@@ -488,21 +489,22 @@ __global__ void __launch_bounds__(WR_THREADS, WR_BPS) moe_ring_kernel(MoeDecodeA
 
 template <int NT, bool UP>
 static int launch_ring(const MoeDecodeArgs &a, int slots, cudaStream_t st) {
-  static int resident[4];
-  static const cudaError_t prepared = [] {
-    const cudaError_t e = ring_residency<NT>(moe_ring_kernel<NT, UP>, resident);
+  static DevicePrep prep;
+  const int (*resident)[4];
+  const cudaError_t prepared = prep.get([](int (&r)[4]) {
+    const cudaError_t e = ring_residency<NT>(moe_ring_kernel<NT, UP>, r);
     return e != cudaSuccess ? e
                             : cudaFuncSetAttribute(moe_ring_kernel<NT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    WeightRing<NT>::BYTES + 40 * 1024);
-  }();
+  }, resident);
   if (prepared != cudaSuccess) {
     set_error("moe_decode: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
   }
   // (which experts are in use is known on the device only: as many as there can be)
   const int n = a.E < a.B * a.top ? a.E : a.B * a.top, kf = ceil_div(a.F, WR_K), kf_shared = ceil_div(a.F_shared, WR_K);
-  const RingPlan p = UP ? ring_plan(n * a.F + a.F_shared, 2, ceil_div(a.D, WR_K), resident)
-                        : ring_plan(a.D, 1, n * kf + kf_shared, resident);
+  const RingPlan p = UP ? ring_plan(n * a.F + a.F_shared, 2, ceil_div(a.D, WR_K), *resident)
+                        : ring_plan(a.D, 1, n * kf + kf_shared, *resident);
   djv::launch_kernel_cluster(moe_ring_kernel<NT, UP>, dim3(p.clusters * p.S), dim3(WR_THREADS),
                              WeightRing<NT>::BYTES + (size_t)a.E * (4 + MM_B), st, dim3(p.S), a, slots);
   count_launch();

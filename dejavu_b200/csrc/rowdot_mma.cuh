@@ -96,13 +96,14 @@ template <typename T, typename TO, int NT, int ACT>
 static int launch_rowdot_mma(TO *Y, const T *W, const T *X, const void *idx, const T *bias, int M, int N, long long ldw,
                              int idx64, int B, float act_param, cudaStream_t st) {
   constexpr int UNIT = is_glu(ACT) ? 2 : 1;
-  static int resident[4];
-  static const cudaError_t prepared = ring_residency<NT>(rowdot_mma_kernel<T, TO, NT, ACT>, resident);
+  static DevicePrep prep;
+  const int (*resident)[4];
+  const cudaError_t prepared = prep.get([](int (&r)[4]) { return ring_residency<NT>(rowdot_mma_kernel<T, TO, NT, ACT>, r); }, resident);
   if (prepared != cudaSuccess) {
     set_error("rowdot_mma: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
   }
-  const RingPlan p = ring_plan(M / UNIT, UNIT, ceil_div(N, WR_K), resident);
+  const RingPlan p = ring_plan(M / UNIT, UNIT, ceil_div(N, WR_K), *resident);
   djv::launch_kernel_cluster(rowdot_mma_kernel<T, TO, NT, ACT>, dim3(p.clusters * p.S), dim3(WR_THREADS),
                              (size_t)WeightRing<NT>::BYTES, st, dim3(p.S), Y, W, X, idx, bias, M, N, ldw, idx64, B, act_param,
                              p.per, p.rest);
