@@ -84,6 +84,7 @@ __device__ __forceinline__ void qkv_batch_products(const __half *w, const __half
     __syncthreads();  // everybody's copies of this stage have landed, and the stage before has been read
     issue(it + QB_STAGES - 1);
     const uint32_t wb = base + (uint32_t)(it % QB_STAGES) * STAGE, xb = wb + W_BYTES;
+    float s[NT][4] = {};
 #pragma unroll
     for (int ks = kw; ks < QB_K / 16; ks += KW) {
       uint32_t a[4];
@@ -93,10 +94,12 @@ __device__ __forceinline__ void qkv_batch_products(const __half *w, const __half
         uint32_t b[4];
         const int row = j * 8 + br;
         ldmatrix_x4(b, xb + row * 128 + (((2 * ks + bc) ^ (row & 7)) << 4));
-        mma_m16n8k16(acc[j], a[0], a[1], a[2], a[3], b[0], b[1]);
-        mma_m16n8k16(acc[j + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+        mma_m16n8k16(s[j], a[0], a[1], a[2], a[3], b[0], b[1]);
+        mma_m16n8k16(s[j + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
       }
     }
+#pragma unroll
+    for (int j = 0; j < NT; ++j) add_sums(acc[j], s[j]);
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -264,8 +267,10 @@ out_proj_mma_kernel(__half *__restrict__ Y, const __half *__restrict__ W, const 
     for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
-        mma_m16n8k16(acc[j], lo[u].x, hi[u].x, lo[u].y, hi[u].y, x[u][j].x, x[u][j].y);
-        mma_m16n8k16(acc[j], lo[u].z, hi[u].z, lo[u].w, hi[u].w, x[u][j].z, x[u][j].w);
+        float s[4] = {};
+        mma_m16n8k16(s, lo[u].x, hi[u].x, lo[u].y, hi[u].y, x[u][j].x, x[u][j].y);
+        mma_m16n8k16(s, lo[u].z, hi[u].z, lo[u].w, hi[u].w, x[u][j].z, x[u][j].w);
+        add_sums(acc[j], s);
       }
   }
 #pragma unroll

@@ -45,17 +45,19 @@ static void launch_rowdot_dense(TO *Y, const T *W, const T *X, int M, int N, lon
 }
 
 // 16-bit element types only: tensor cores for 5 rows of x and more, and for 3 and 4 where the weights are large. bf16, us on the
-// CUDA cores / tensor cores for 4 rows: 2048 x 2048 3.8 / 5.0, 4096 x 4096 9.8 / 8.2, 11264 x 2048 12.9 / 10.8, 22016 x 4096
-// 39.9 / 29.2; for 2 rows 4096 x 4096 9.2 / 8.4, 11264 x 2048 9.8 / 10.8, 22016 x 4096 30.3 / 29.1, 50272 x 4096 62.4 / 64.
-static bool takes_mma(int B, int M, int N) { return B >= 5 || (B >= 3 && (long long)M * N >= 1ll << 24); }
+// CUDA cores / tensor cores for 4 rows: 4096 x 4096 9.8 / 8.0, 6144 x 4096 16.4 / 10.7, 22016 x 4096 39.8 / 29.3. With 3 and 4
+// rows the tensor cores' sums are in parts of 4 chunks, and rows are long: below 2560 columns the CUDA cores' are the nearer
+// ones (relative error of fp32 results, CUDA / tensor cores: 1024 columns 7.0e-8 / 7.5e-8, 2048 7.9 / 8.1, 2560 8.34 / 8.33,
+// 4096 9.6 / 9.0, 11008 14.2 / 10.0).
+static bool takes_mma(int B, int M, int N) { return B >= 5 || (B >= 3 && N >= 2560 && (long long)M * N >= 1ll << 24); }
 template <typename TO, int ACT>
 static int dense_mma(TO *Y, const bf16 *W, const bf16 *X, int B, int M, int N, long long ldw, float param, cudaStream_t st) {
-#define DJV_DM(NT_) launch_rowdot_mma<bf16, TO, NT_, ACT>(Y, W, X, nullptr, nullptr, M, N, ldw, 0, B, param, st)
+#define DJV_DM(NT_, PART_) launch_rowdot_mma<bf16, TO, NT_, ACT, PART_>(Y, W, X, nullptr, nullptr, M, N, ldw, 0, B, param, st)
   switch ((B + 7) / 8) {
-    case 1: return DJV_DM(1);
-    case 2: return DJV_DM(2);
-    case 3: return DJV_DM(3);
-    default: return DJV_DM(4);
+    case 1: return B < 5 ? DJV_DM(1, 4) : DJV_DM(1, 0);
+    case 2: return DJV_DM(2, 0);
+    case 3: return DJV_DM(3, 0);
+    default: return DJV_DM(4, 0);
   }
 #undef DJV_DM
 }

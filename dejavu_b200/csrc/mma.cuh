@@ -55,4 +55,11 @@ __device__ __forceinline__ void mma_m16n8k16_t<bf16>(float (&d)[4], uint32_t a0,
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// acc += s in fp32. The tensor cores cut off what does not fit beside the accumulator that they are given, always towards
+// zero, so a long chain of products in one accumulator drifts: a few products start from zero and join the rest here.
+__device__ __forceinline__ void add_sums(float (&acc)[4], const float (&s)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] += s[e];
+}
+
 }  // namespace djv

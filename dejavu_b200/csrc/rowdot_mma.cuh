@@ -67,7 +67,7 @@ struct RowdotSource {
   }
 };
 
-template <typename T, typename TO, int NT, int ACT>  // NT groups of 8 rows of x
+template <typename T, typename TO, int NT, int ACT, int PART>  // NT groups of 8 rows of x
 __global__ void __launch_bounds__(WR_THREADS, WR_BPS)
 rowdot_mma_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__ X, const void *__restrict__ idx,
                   const T *__restrict__ bias, int M, int N, long long ldw, int idx64, int B, float act_param, int per, int rest) {
@@ -88,23 +88,23 @@ rowdot_mma_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restri
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   RowdotSource<T, TO, ACT> src{Y, W, X, idx, bias, M, N, idx64, B, ldw, act_param, first, last, rows, S, rank};
-  weight_ring<T, NT>(src, tiles, chunks, B, wr_smem);
+  weight_ring<T, NT, PART>(src, tiles, chunks, B, wr_smem);
 }
 
 // (internal linkage: each library prepares its own copy of the kernel)
-template <typename T, typename TO, int NT, int ACT>
+template <typename T, typename TO, int NT, int ACT, int PART = 0>
 static int launch_rowdot_mma(TO *Y, const T *W, const T *X, const void *idx, const T *bias, int M, int N, long long ldw,
                              int idx64, int B, float act_param, cudaStream_t st) {
   constexpr int UNIT = is_glu(ACT) ? 2 : 1;
   static DevicePrep prep;
   const int (*resident)[4];
-  const cudaError_t prepared = prep.get([](int (&r)[4]) { return ring_residency<NT>(rowdot_mma_kernel<T, TO, NT, ACT>, r); }, resident);
+  const cudaError_t prepared = prep.get([](int (&r)[4]) { return ring_residency<NT>(rowdot_mma_kernel<T, TO, NT, ACT, PART>, r); }, resident);
   if (prepared != cudaSuccess) {
     set_error("rowdot_mma: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
   }
   const RingPlan p = ring_plan(M / UNIT, UNIT, ceil_div(N, WR_K), *resident);
-  djv::launch_kernel_cluster(rowdot_mma_kernel<T, TO, NT, ACT>, dim3(p.clusters * p.S), dim3(WR_THREADS),
+  djv::launch_kernel_cluster(rowdot_mma_kernel<T, TO, NT, ACT, PART>, dim3(p.clusters * p.S), dim3(WR_THREADS),
                              (size_t)WeightRing<NT>::BYTES, st, dim3(p.S), Y, W, X, idx, bias, M, N, ldw, idx64, B, act_param,
                              p.per, p.rest);
   count_launch();

@@ -9,6 +9,12 @@
 // added up (over the 4 warps that split a chunk's columns, then over the cluster through distributed shared memory, in rank
 // order) while the next tile's weights are on their way. Two blocks per multiprocessor, about 64 KB of weights each in flight.
 //
+// The tensor cores' sums are short: 16 columns with up to 8 rows of x, 32 with more, join the others in fp32 (add_sums). Kept in
+// the MMAs' accumulators from end to end of a row they were off by 1.0e-6 of the result at 4096 columns and 2.9e-6 at 11008;
+// now 1.2e-7 to 1.5e-7 and 1.8e-7. With PART, the sums of PART chunks join before they meet the rest (0.9e-7 and 1.0e-7):
+// where the CUDA cores, 1.0e-7 and 1.4e-7, had the product before. Cost with 8 rows of x 0 to 2 %, with 32 up to 5 %, of PART
+// another 0 to 4 %.
+//
 // Bound by HBM from about 20 MB of weights on: bf16, 8 rows of x, us before (a block of 8 warps per 16 rows, fed straight
 // from registers) / now, of which the weights at copy rate: 6144 x 4096 15.1 / 10.3 (7.7), 12352 x 4096 28.9 / 18.6 (15.5),
 // 22016 x 4096 35.3 / 29.5 (27.7), 50272 x 4096 77.7 / 65.7 (63.2); 16 rows, 4096 gathered rows of 12288 24.5 / 20.4 (15.5).
@@ -48,7 +54,7 @@ struct WeightRing {
   static_assert(STAGES >= 3, "");
 };
 
-template <typename T, int NT, class Source>
+template <typename T, int NT, int PART = 0, class Source>
 __device__ __forceinline__ void weight_ring(Source &src, int tiles, int chunks, int tokens, unsigned char *smem) {
   using R = WeightRing<NT>;
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -90,27 +96,44 @@ __device__ __forceinline__ void weight_ring(Source &src, int tiles, int chunks, 
   const int br = lane & 7, bc = WR_PPR / WR_KW * kw + (lane >> 3);
   const uint32_t a_off = (uint32_t)ar * WR_K * 2, b_off = R::W_BYTES + (uint32_t)br * WR_K * 2;
   int from = 0;
+  auto chunk = [&](float (&acc)[NT][4]) {  // the next one's products
+    cp_async_wait<R::STAGES - 2>();
+    __syncthreads();  // everybody's copies of this stage have landed, and the stage before has been read
+    issue();
+    const uint32_t st = base + (uint32_t)from * R::STAGE;
+    from = from + 1 == R::STAGES ? 0 : from + 1;
+#pragma unroll
+    for (int p = 0; p < WR_PPR / WR_KW; p += 4) {  // two steps of 16 columns
+      uint32_t a0[4], a1[4];
+      ldmatrix_x4(a0, st + a_off + (((ac + p) ^ (ar & 7)) << 4));
+      ldmatrix_x4(a1, st + a_off + (((ac + p + 2) ^ (ar & 7)) << 4));
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        uint32_t b[4];
+        ldmatrix_x4(b, st + b_off + j * 8 * WR_K * 2 + (((bc + p) ^ br) << 4));
+        float s[4] = {};
+        mma_m16n8k16_t<T>(s, a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
+        if (NT == 1) {
+          add_sums(acc[j], s);
+          s[0] = s[1] = s[2] = s[3] = 0.f;
+        }
+        mma_m16n8k16_t<T>(s, a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
+        add_sums(acc[j], s);
+      }
+    }
+  };
   for (int t = 0; t < tiles; ++t) {
     src.begin(t);
     float acc[NT][4] = {};
-    for (int c = 0; c < chunks; ++c) {
-      cp_async_wait<R::STAGES - 2>();
-      __syncthreads();  // everybody's copies of this stage have landed, and the stage before has been read
-      issue();
-      const uint32_t st = base + (uint32_t)from * R::STAGE;
-      from = from + 1 == R::STAGES ? 0 : from + 1;
+    if constexpr (PART == 0) {
+      for (int c = 0; c < chunks; ++c) chunk(acc);
+    } else {
+      for (int c = 0; c < chunks;) {
+        float part[NT][4] = {};
+#pragma unroll 1
+        for (const int stop = min(c + PART, chunks); c < stop; ++c) chunk(part);
 #pragma unroll
-      for (int p = 0; p < WR_PPR / WR_KW; p += 4) {  // two steps of 16 columns
-        uint32_t a0[4], a1[4];
-        ldmatrix_x4(a0, st + a_off + (((ac + p) ^ (ar & 7)) << 4));
-        ldmatrix_x4(a1, st + a_off + (((ac + p + 2) ^ (ar & 7)) << 4));
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          uint32_t b[4];
-          ldmatrix_x4(b, st + b_off + j * 8 * WR_K * 2 + (((bc + p) ^ br) << 4));
-          mma_m16n8k16_t<T>(acc[j], a0[0], a0[1], a0[2], a0[3], b[0], b[1]);
-          mma_m16n8k16_t<T>(acc[j], a1[0], a1[1], a1[2], a1[3], b[2], b[3]);
-        }
+        for (int j = 0; j < NT; ++j) add_sums(acc[j], part[j]);
       }
     }
     float *mine = red + (t & 1) * R::RED;

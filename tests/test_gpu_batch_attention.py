@@ -63,3 +63,30 @@ def test_output_projection_of_a_batch(cuda, B, nheads, hd, d, nnz):
     heads = torch.randperm(nheads, device=cuda, generator=g)[:nnz]
     want = torch.einsum("bhj,nhj->bn", x[:, heads].double(), w[:, heads].double()) + bias.double()
     near(ops.out_proj_sparse(x, w, heads.int(), bias), want)
+
+
+# An error of e of a result's size takes about e / 2^-12 of the results across the edge between two fp16 values. fp32 sums are off
+# by 1e-7 to 2e-7 here; sums left in the tensor cores' accumulators by 2e-6 (the projection) and 8e-7 (the output projection).
+def crossed(got, want):
+    return (got != want.half()).double().mean().item() * 2 ** -12
+
+
+def test_sums_of_the_projections_are_those_of_fp32(cuda):
+    from dejavu_b200 import _lib, ops
+
+    g = torch.Generator(device=cuda).manual_seed(1)
+    B, nheads, hd, d, S = 8, 12, 128, 9216, 16
+    f16 = {"dtype": torch.float16, "device": cuda}
+    w, x = (torch.randn(3, nheads, hd, d, device=cuda, generator=g) * d ** -0.5).half(), torch.randn(B, d, device=cuda, generator=g).half()
+    ring, q = torch.zeros(B, 16, d, **f16), torch.zeros(B, nheads, hd, **f16)
+    k, v = torch.zeros(B, nheads, hd // 8, S, 8, **f16), torch.zeros(B, nheads, S, hd, **f16)
+    state = torch.zeros(_lib.ATTN_STATE_HDR + 3 * nheads, dtype=torch.int32, device=cuda)
+    _lib.call("djv_attn_state_reset", state.data_ptr(), nheads, 0, ops._stream())
+    _lib.call("djv_attn_step_project_batch", q.data_ptr(), w.data_ptr(), None, x.data_ptr(), ring.data_ptr(), k.data_ptr(),
+              v.data_ptr(), state.data_ptr(), None, 0, d, nheads, hd, S, B, ops._stream())
+    want = torch.einsum("bd,chjd->cbhj", x.double(), w.double())
+    assert crossed(q, want[0]) <= 6e-7 and crossed(v[:, :, 0], want[2]) <= 6e-7
+    nheads, d = 32, 4096
+    w = (torch.randn(d, nheads, hd, device=cuda, generator=g) * d ** -0.5).half()
+    x, heads = torch.randn(16, nheads, hd, device=cuda, generator=g).half(), torch.arange(nheads, dtype=torch.int32, device=cuda)
+    assert crossed(ops.out_proj_sparse(x, w, heads), torch.einsum("bhj,nhj->bn", x.double(), w.double())) <= 5e-7

@@ -94,3 +94,21 @@ def test_routed_weights_streamed_for_several_rows(cuda, B, E, top, D, F, Fs):
             want[b] += unit(w[b, k] * x[b:b + 1].double(), gu[idx[b, k]], down[idx[b, k]])[0]
     # an activation on the edge of two bf16 values may round the other way: 2^-8 of itself, among F * (top + 1) that add up
     assert (got.double() - want).norm() <= 2e-3 * want.norm()
+
+
+# Distance of fp32 results from 64 bits. An addition rounds by about 2.4e-8 of the sum so far (2^-23 / sqrt(12), averaged over the
+# mantissa), which grows evenly: n in a row are off by 2.4e-8 * sqrt(n / 2) of the result, and the warps' and blocks' sums add 8
+# more; the products of an MMA that starts from zero are cut by 6e-8 to 7e-8. With 3 and 4 rows parts of 8 additions are joined,
+# up to 8 rows add every 16 columns of a warp's quarter, more rows every 32. Sums left in the tensor cores' accumulators are 1e-6
+# off at 4096 columns and 3e-6 at 11008.
+@pytest.mark.parametrize("B", [3, 4, 5, 8, 17, 32])
+@pytest.mark.parametrize("N,M", [(768, 50272), (2560, 8192), (4096, 4096), (4096, 22016), (11008, 8192)])
+def test_sums_of_several_rows_are_fp32_sums(cuda, B, N, M):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + N)
+    x = torch.randn(B, N, device=cuda, generator=g).bfloat16()
+    w = (torch.randn(M, N, device=cuda, generator=g) * N ** -0.5).bfloat16()
+    y = x.double() @ w.double().t()
+    n = 8 + N / 512 if B <= 4 else N / 64 if B <= 8 else N / 128
+    assert (ops.linear_gemv(x, w, torch.float32).double() - y).norm() <= (2.4e-8 * (n / 2 + 8) ** 0.5 + 7e-8) * y.norm()
