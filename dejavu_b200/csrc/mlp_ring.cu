@@ -591,23 +591,19 @@ int ring_max_clusters(size_t smem) {
 }
 
 template <int B, int MODE, int C>
-int ring_prepare() {
-  static int rc = [] {
-    cudaError_t e = cudaFuncSetAttribute(mlp_ring_kernel<B, MODE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         MR_SMEM_BUDGET + 8192);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return 1;
-    }
-    return 0;
-  }();
-  return rc;
+cudaError_t ring_prepare() {
+  static DevicePrep prep;
+  const int (*unused)[4];
+  return prep.get([](int (&)[4]) {
+    return cudaFuncSetAttribute(mlp_ring_kernel<B, MODE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, MR_SMEM_BUDGET + 8192);
+  }, unused);
 }
 
 template <int B, int MODE, int C>
 int ring_launch(RingArgs a, cudaStream_t st) {
-  if (ring_prepare<B, MODE, C>() != 0) {
-    set_error("mlp_ring: cannot raise the kernel's shared-memory limit");
+  const cudaError_t prepared = ring_prepare<B, MODE, C>();
+  if (prepared != cudaSuccess) {
+    set_error("mlp_ring: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
   }
   const int seg = a.N / C;

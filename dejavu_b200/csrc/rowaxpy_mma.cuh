@@ -264,23 +264,25 @@ inline size_t rowaxpy_mma_scratch_bytes(int B, int N, int M) {
   return 4096 + (p.rs > 1 ? (size_t)p.rs * B * N * sizeof(float) : 0);
 }
 
-// 1 <= B <= 32 (used from 3 rows up)
-inline int rowaxpy_mma(int B, __half *Y, const __half *W, const __half *X, const void *idx, const __half *bias,
+// 1 <= B <= 32 (used from 3 rows up; internal linkage: each library prepares its own copy of the kernels)
+static int rowaxpy_mma(int B, __half *Y, const __half *W, const __half *X, const void *idx, const __half *bias,
                        void *scratch, int M, int N, long long ldw, int idx64, cudaStream_t st) {
   const RowaxpyMmaPlan p = plan_rowaxpy_mma(M, N);
   float *partial = reinterpret_cast<float *>(reinterpret_cast<char *>(scratch) + 4096);  // (header: other kernels' counters)
   const dim3 grid(p.tiles, p.rs);
   constexpr size_t smem1 = RmSmem<1, RM_DEPTH1>::BYTES, smem2 = RmSmem<2, RM_DEPTH2>::BYTES;
   static_assert(smem1 <= 227 * 1024 && smem2 <= 227 * 1024, "shared memory of a block");
-  static const int prepared = [] {
-    cudaError_t e1 = cudaFuncSetAttribute(rowaxpy_mma_kernel<1, RM_DEPTH1>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-    cudaError_t e2 = cudaFuncSetAttribute(rowaxpy_mma_kernel<2, RM_DEPTH2>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-    if (e1 != cudaSuccess || e2 != cudaSuccess) cudaGetLastError();
-    return (e1 == cudaSuccess && e2 == cudaSuccess) ? 0 : 1;
-  }();
-  if (prepared != 0) return DJV_ERR_CUDA;
+  static DevicePrep prep;
+  const int (*unused)[4];
+  const cudaError_t prepared = prep.get([](int (&)[4]) {
+    const cudaError_t e = cudaFuncSetAttribute(rowaxpy_mma_kernel<1, RM_DEPTH1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(rowaxpy_mma_kernel<2, RM_DEPTH2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+  }, unused);
+  if (prepared != cudaSuccess) {
+    set_error("rowaxpy_mma: %s", cudaGetErrorString(prepared));
+    return DJV_ERR_CUDA;
+  }
   if (B <= 16)
     djv::launch_kernel(rowaxpy_mma_kernel<1, RM_DEPTH1>, grid, dim3(RM_THREADS), smem1, st, Y, W, X, idx, bias,
                        partial, M, N, ldw, idx64, B, p.rows_per_block);

@@ -348,15 +348,15 @@ static int launch_topk(int32_t *idx32, int64_t *idx64, const void *scores, int n
     const int per_b = (n + TC_C - 1) / TC_C;
     const size_t smem = ((size_t)per_b * (score_is_f32 ? 4 : 2) + 15) & ~(size_t)15;
     if (smem <= 200 * 1024) {
-      static const cudaError_t prep = [] {
-        cudaError_t a = cudaFuncSetAttribute(topk_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024);
-        cudaError_t b = cudaFuncSetAttribute(topk_cluster_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024);
-        return a != cudaSuccess ? a : b;
-      }();
-      if (prep != cudaSuccess) {
-        set_error("topk: cudaFuncSetAttribute: %s", cudaGetErrorString(prep));
+      static DevicePrep prep;
+      const int (*unused)[4];
+      const cudaError_t prepared = prep.get([](int (&)[4]) {
+        const cudaError_t e = cudaFuncSetAttribute(topk_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        return e != cudaSuccess ? e
+                                : cudaFuncSetAttribute(topk_cluster_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      }, unused);
+      if (prepared != cudaSuccess) {
+        set_error("topk: %s", cudaGetErrorString(prepared));
         return DJV_ERR_CUDA;
       }
       if (score_is_f32)

@@ -1,0 +1,87 @@
+"""What calls into the libraries prepare and launch, seen by a CUDA runtime that runs nothing (fake_cudart.cpp), in a process of
+its own that never loads the real one."""
+import ctypes as C
+import shutil
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+P = 1 << 20  # an aligned address that nobody reads
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from dejavu_b200 import build
+
+    build.build()
+    nvcc = Path(build._nvcc()).resolve()
+    folder = tmp_path_factory.mktemp("fake")
+    versions = folder / "versions"
+    versions.write_text("libcudart.so.12 { global: *; };\n")
+    out = folder / "libcudart.so.12"
+    subprocess.run([shutil.which("g++"), "-std=c++17", "-shared", "-fPIC", "-I", str(nvcc.parent.parent / "include"),
+                    str(ROOT / "tests" / "fake_cudart.cpp"), "-o", str(out), "-Wl,-soname,libcudart.so.12",
+                    f"-Wl,--version-script={versions}"], check=True)
+    return out
+
+
+PRELUDE = """
+import ctypes as C
+fake = C.CDLL({fake!r}, mode=C.RTLD_GLOBAL)
+fake.fake_notes.restype = C.c_char_p
+P = {P}
+L = C.c_longlong
+def load(name):
+    lib = C.CDLL({root!r} + "/dejavu_b200/" + name)
+    lib.djv_last_error.restype = C.c_char_p
+    return lib
+def done(lib, rc):
+    assert rc == 0, lib.djv_last_error()
+def notes():
+    out = [l.split() for l in fake.fake_notes().decode().splitlines()]
+    fake.fake_clear()
+    return [dict(what=l[0], device=int(l[1]), kernel=l[2], grid=int(l[3]) * int(l[4]) * int(l[5]), block=int(l[6]), smem=int(l[7]),
+                 cluster=int(l[8])) for l in out]
+ptr = C.c_void_p(P)
+"""
+
+
+def run(fake, body):
+    code = PRELUDE.format(fake=str(fake), root=str(ROOT), P=P) + body
+    r = subprocess.run([sys.executable, "-I", "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+CALLS = {
+    "fc2 of several rows": """
+for B in (3, 16, 17, 32):
+    done(lib, lib.djv_gather_transposed_gemv(ptr, ptr, ptr, ptr, None, B, 4096, 2048, L(4096), 0, ptr, C.c_size_t(1 << 30), None))
+""",
+    "products of several rows": """
+for B in (5, 16, 24, 32):
+    done(lib, lib.djv_gather_gemv(ptr, ptr, ptr, ptr, None, B, 4096, 8192, L(4096), 0, 1, None))
+""",
+    "sparse MLP in one pass": """
+for B in (1, 2, 4):
+    done(lib, lib.djv_mlp_sparse_fused(ptr, ptr, ptr, ptr, ptr, None, None, B, 4096, 512, 16384, L(4096), L(4096), 0, ptr, C.c_size_t(1 << 30), None))
+""",
+    "top-K of long vectors": """
+for f32 in (0, 1):
+    done(lib, lib.djv_topk(ptr, None, ptr, 200000, 512, f32, None))
+""",
+    "projections of a batch": """
+for hd in (32, 64, 128):
+    done(lib, lib.djv_attn_step_project_batch(ptr, ptr, None, ptr, ptr, ptr, ptr, ptr, None, 0, 512, 8, hd, 64, 8, None))
+""",
+}
+
+
+@pytest.mark.parametrize("what", CALLS)
+def test_kernels_are_prepared_on_every_device(fake, what):
+    """Attributes of a kernel belong to a device: what the first call sets on one does not serve the other."""
+    run(fake, 'lib = load("libdejavu_b200.so")\nfor device in (0, 1):\n    fake.fake_set_device(device)\n'
+        + "".join("    " + line + "\n" for line in CALLS[what].strip().splitlines())
+        + "    assert any(n['what'] == 'launch' and n['device'] == device and n['smem'] > 48 * 1024 for n in notes())\n")
