@@ -19,6 +19,7 @@ takes over.
 """
 from __future__ import annotations
 
+import inspect
 import os
 import time
 from dataclasses import dataclass, field
@@ -134,6 +135,15 @@ def update_graph_cache(model, cache, batch_size, seqlen_og, max_seqlen, tensor_p
     return cache
 
 
+def _asks_for_rows(model, rows, n) -> bool:
+    """Whether the model is asked for the logits of `rows` only. A class that selects them may have descendants whose forward does
+    not take the argument, or passes on whatever it gets: those are asked where it saves something, and may answer with all n."""
+    if not getattr(model, "selects_logit_rows", False):
+        return False
+    taken = inspect.signature(getattr(model, "forward", model)).parameters
+    return "logit_rows" in taken or (len(rows) < n and any(p.kind is p.VAR_KEYWORD for p in taken.values()))
+
+
 @torch.inference_mode()
 def step(model, params: InferenceParams, input_ids, position_ids=None, logit_rows=None):
     """Runs the next input_ids (B, n) of every sequence, from what the caches hold after params.sequence_len_offset
@@ -142,12 +152,11 @@ def step(model, params: InferenceParams, input_ids, position_ids=None, logit_row
     n = input_ids.size(1)
     if params.sequence_len_offset + n > params.max_sequence_len:
         raise ValueError(f"{params.sequence_len_offset} + {n} tokens exceed the cache of {params.max_sequence_len}")
-    if getattr(model, "selects_logit_rows", False):
-        logits = model(input_ids, position_ids=position_ids, inference_params=params, logit_rows=logit_rows).logits
-    else:
-        logits = model(input_ids, position_ids=position_ids, inference_params=params).logits
-        if logit_rows is not None:
-            logits = logits[:, list(logit_rows)]
+    rows = None if logit_rows is None else list(logit_rows)
+    asked = rows is not None and _asks_for_rows(model, rows, n)
+    logits = model(input_ids, position_ids=position_ids, inference_params=params, **({"logit_rows": rows} if asked else {})).logits
+    if rows is not None and not (asked and logits.size(1) == len(rows)):
+        logits = logits[:, rows]
     params.sequence_len_offset += n
     return logits
 

@@ -164,6 +164,43 @@ def test_pool_keeps_requests_apart_and_reuses_slots():
         pool.run("b", [1, 2], [])
 
 
+class Selecting:
+    selects_logit_rows = True
+
+    def forward(self, ids, position_ids=None, inference_params=None, logit_rows=None):
+        logits = ids[..., None].float()
+        return SimpleNamespace(logits=logits if logit_rows is None else logits[:, logit_rows])
+
+    def __call__(self, *args, **kwargs):
+        return self.forward(*args, **kwargs)
+
+
+class WithoutRows(Selecting):
+    def forward(self, ids, position_ids=None, inference_params=None):
+        return super().forward(ids, position_ids, inference_params)
+
+
+class PassingOn(Selecting):
+    def forward(self, ids, **kwargs):
+        return super().forward(ids, **kwargs)
+
+
+class Ignoring(Selecting):
+    def forward(self, ids, **kwargs):
+        return super().forward(ids)
+
+
+@pytest.mark.parametrize("kind", [Selecting, WithoutRows, PassingOn, Ignoring])
+@pytest.mark.parametrize("rows", [None, [3], [-1], (), [0, 2], [3, 2, 1, 0], [1, 1, 1, 1, 0]])
+def test_a_step_of_a_model_with_another_forward(kind, rows):
+    from dejavu_b200.generation import InferenceParams, step
+
+    ids = torch.tensor([[5, 6, 7, 8], [1, 2, 3, 4]])
+    params = InferenceParams(max_sequence_len=8, max_batch_size=2)
+    logits = step(kind(), params, ids, logit_rows=rows)
+    assert torch.equal(logits[..., 0].long(), ids if rows is None else ids[:, list(rows)]) and params.sequence_len_offset == 4
+
+
 def test_commands_explain_themselves(tmp_path):
     for cmd in ([str(ROOT / "bin" / "trace_run"), "--help"], [sys.executable, "-m", "dejavu_b200", "generate", "--help"],
                 [sys.executable, "-m", "dejavu_b200", "trace", "--help"]):
