@@ -254,10 +254,8 @@ class GPTLMHeadModel(nn.Module, GenerationMixin):
             elif rows != list(range(n)):
                 hidden_states = hidden_states[:, rows]
         B, L, d = hidden_states.shape
-        weight = self.lm_head.weight
-        if L == 1 and hidden_states.is_cuda and B <= 32 and (
-                n == 1 or (d % 8 == 0 and self.lm_head.bias is None and modules._inference_fp16(hidden_states, weight))):
-            lm_logits = ops.dense_gemv(hidden_states.reshape(B, d), weight).view(B, 1, -1)
+        if n == 1 and L == 1 and hidden_states.is_cuda and B <= 32:
+            lm_logits = ops.dense_gemv(hidden_states.view(B, d), self.lm_head.weight).view(B, 1, -1)
         else:
             lm_logits = self.lm_head(hidden_states)
         world = _world(self.process_group)

@@ -36,3 +36,19 @@ def test_logits_of_chosen_tokens(cuda, B, n, rows):
     assert out[1].shape == (B, len(rows), out[0].size(2))
     # two products of 256 terms in fp32, each rounded to fp16
     assert (out[1] - out[0][:, rows]).abs().le(2 ** -10 * out[0].abs().max() + 1e-5).all()
+
+
+def test_the_head_of_a_prompt_is_a_module_that_is_called(cuda):
+    from dejavu_b200.generation import InferenceParams, allocate_kv_cache, step
+    from dejavu_b200.gpt import GPTLMHeadModel, apply_sparsity_knobs, opt_config
+
+    cfg = apply_sparsity_knobs(opt_config("opt-125m", n_layer=2, n_embd=256, hidden_size=256, n_head=4, n_inner=1024, vocab_size=520,
+                                          max_position_embeddings=64, mlp_sp_dim=64, att_sp_dim=32), 256, 2, 2)
+    model = GPTLMHeadModel(cfg, device=cuda, dtype=torch.float16).eval().init_random(0, std=0.05)
+    model.lm_head.register_forward_hook(lambda head, args, result: 2 * result)
+    ids = torch.arange(5, device=cuda)[None]
+    out = []
+    for rows in (None, [4]):
+        ip = InferenceParams(max_sequence_len=5, max_batch_size=1, key_value_memory_dict=allocate_kv_cache(model, 1, 5, cuda))
+        out.append(step(model, ip, ids, logit_rows=rows))
+    assert (out[1] - out[0][:, [4]]).abs().le(2 ** -9 * out[0].abs().max() + 1e-5).all()  # (products of 256 terms, rounded to fp16)
