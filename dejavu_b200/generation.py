@@ -140,8 +140,15 @@ def _asks_for_rows(model, rows, n) -> bool:
     not take the argument, or passes on whatever it gets: those are asked where it saves something, and may answer with all n."""
     if not getattr(model, "selects_logit_rows", False):
         return False
-    taken = inspect.signature(getattr(model, "forward", model)).parameters
-    return "logit_rows" in taken or (len(rows) < n and any(p.kind is p.VAR_KEYWORD for p in taken.values()))
+    forward = getattr(model, "forward", None) or type(model).__call__
+    code = getattr(getattr(forward, "__func__", forward), "__code__", None)
+    if code is not None:  # (a signature object for every step would cost as much as several launches)
+        named = "logit_rows" in code.co_varnames[:code.co_argcount + code.co_kwonlyargcount]
+        any_name = bool(code.co_flags & inspect.CO_VARKEYWORDS)
+    else:
+        taken = inspect.signature(forward).parameters
+        named, any_name = "logit_rows" in taken, any(p.kind is p.VAR_KEYWORD for p in taken.values())
+    return named or (any_name and len(rows) < n)
 
 
 @torch.inference_mode()
