@@ -525,7 +525,7 @@ class ParallelMHASparseAttMlp(nn.Module):
             off = inference_params.sequence_len_offset
             assert off == 0 and L <= S
             # K cache (B, n, hd/8, S, 8), V cache (B, n, S, hd)   (mha_dejavu.py:385-447)
-            if (_inference_fp16(qkv, k_cache, v_cache) and hd in (32, 64, 128) and k_cache.size(0) == B
+            if (_inference_fp16(qkv, k_cache, v_cache) and hd in (32, 64, 128) and 1 <= L and k_cache.size(0) == B <= 65535
                     and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (qkv, k_cache, v_cache))):
                 ops.kv_store(k_cache, v_cache, qkv)
             else:

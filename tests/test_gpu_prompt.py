@@ -52,3 +52,14 @@ def test_the_head_of_a_prompt_is_a_module_that_is_called(cuda):
         ip = InferenceParams(max_sequence_len=5, max_batch_size=1, key_value_memory_dict=allocate_kv_cache(model, 1, 5, cuda))
         out.append(step(model, ip, ids, logit_rows=rows))
     assert (out[1] - out[0][:, [4]]).abs().le(2 ** -9 * out[0].abs().max() + 1e-5).all()  # (products of 256 terms, rounded to fp16)
+
+
+def test_a_prompt_without_tokens_leaves_empty_caches(cuda):
+    from dejavu_b200.generation import InferenceParams, allocate_kv_cache, step
+    from dejavu_b200.gpt import GPTLMHeadModel, apply_sparsity_knobs, opt_config
+
+    cfg = apply_sparsity_knobs(opt_config("opt-125m", n_layer=2, n_embd=256, hidden_size=256, n_head=4, n_inner=1024, vocab_size=520,
+                                          max_position_embeddings=64, mlp_sp_dim=64, att_sp_dim=32), 256, 2, 2)
+    model = GPTLMHeadModel(cfg, device=cuda, dtype=torch.float16).eval().init_random(0, std=0.05)
+    ip = InferenceParams(max_sequence_len=4, max_batch_size=1, key_value_memory_dict=allocate_kv_cache(model, 1, 4, cuda))
+    assert step(model, ip, torch.zeros(1, 0, dtype=torch.long, device=cuda)).shape == (1, 0, 520)
