@@ -67,6 +67,25 @@ def test_weights_streamed_for_several_rows(cuda, B, N, M):
     near(ops.gather_gemv(x.half(), w.half(), idx, bias, "relu"), want)
 
 
+# both sides of the line between the form without a ring and the ring; parts of a tile, of a 32-column block, of a split
+@pytest.mark.parametrize("B", [5, 8, 9, 16, 17, 25, 32])
+@pytest.mark.parametrize("N,M", [(8, 1), (40, 17), (512, 2048), (520, 257), (1024, 4096), (1032, 513), (2048, 1026), (4096, 2048), (4104, 512),
+                                 (264, 11265), (12288, 33)])
+def test_short_lists_of_several_tokens(cuda, B, N, M):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + N + M)
+    x = torch.randn(B, N, device=cuda, generator=g).half()
+    w = (torch.randn(M + 5, N, device=cuda, generator=g) * N ** -0.5).half()
+    bias = torch.randn(M + 5, device=cuda, generator=g).half()
+    idx = torch.randperm(M + 5, device=cuda, generator=g)[:M]
+    near(ops.gather_gemv(x, w, idx.int(), bias, "relu"), (x.double() @ w[idx].double().t() + bias[idx].double()).relu())
+    pairs = w[:(M + 1) // 2 * 2].bfloat16()
+    p = x.bfloat16().double() @ pairs.double().t()
+    near(ops.linear_gemv(x.bfloat16(), pairs, torch.float32), p)
+    near(ops.linear_gemv(x.bfloat16(), pairs, None, "silu_glu"), p[:, 0::2] * torch.sigmoid(p[:, 0::2]) * p[:, 1::2])
+
+
 @pytest.mark.parametrize("B,E,top,D,F,Fs", [(2, 1, 1, 8, 8, 0), (3, 5, 2, 136, 24, 40), (8, 8, 2, 512, 200, 328), (9, 40, 3, 264, 136, 8),
                                             (17, 4, 4, 1032, 72, 0), (32, 300, 1, 64, 16, 16)])
 def test_routed_weights_streamed_for_several_rows(cuda, B, E, top, D, F, Fs):

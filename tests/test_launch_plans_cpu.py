@@ -85,3 +85,26 @@ def test_kernels_are_prepared_on_every_device(fake, what):
     run(fake, 'lib = load("libdejavu_b200.so")\nfor device in (0, 1):\n    fake.fake_set_device(device)\n'
         + "".join("    " + line + "\n" for line in CALLS[what].strip().splitlines())
         + "    assert any(n['what'] == 'launch' and n['device'] == device and n['smem'] > 48 * 1024 for n in notes())\n")
+
+
+def test_short_lists_of_several_rows_fill_no_ring(fake):
+    run(fake, """
+lib = load("libdejavu_b200.so")
+def kernel(B, N, M):
+    done(lib, lib.djv_gather_gemv(ptr, ptr, ptr, ptr, None, B, N, M, L(N), 0, 1, None))
+    n = [n for n in notes() if n["what"] == "launch"]
+    assert len(n) == 1
+    return "short" if "rowdot_mma_short" in n[0]["kernel"] else "ring" if "rowdot_mma" in n[0]["kernel"] else "rowdot"
+for B in (9, 16, 32):
+    for N, M in ((768, 384), (1024, 1024), (2048, 2048), (4096, 1024), (12288, 512)):
+        assert kernel(B, N, M) == "short", (B, N, M)
+    for N, M in ((768, 8192), (4096, 4096), (12288, 4096)):
+        assert kernel(B, N, M) == "ring", (B, N, M)
+for B in (5, 8):
+    for N, M in ((768, 256), (512, 2048), (2048, 11264)):
+        assert kernel(B, N, M) == "short", (B, N, M)
+    for N, M in ((2048, 2048), (2048, 8192), (4096, 11264)):
+        assert kernel(B, N, M) == "ring", (B, N, M)
+for B in (1, 2):
+    assert kernel(B, 4096, 4096) == "rowdot"
+""")
