@@ -31,9 +31,22 @@ __global__ void attn_state_reset_kernel(int *st, int nheads, int prompt_len) {
 // Step 1 of djv_attn_step as a kernel of its own (see attn_prep_block).
 __global__ void __launch_bounds__(1024)
 attn_prep_kernel(int *__restrict__ st, const int *__restrict__ head_idx, int nnz,
-                 const __half *__restrict__ x, __half *__restrict__ x_ring, int d, int nheads, int S) {
+                 const __half *__restrict__ x, __half *__restrict__ x_ring, int d, int nheads, int S, int nseq,
+                 long long seq_ring) {
   pdl_prologue();
   attn_prep_block(st, head_idx, nnz, x, x_ring, d, nheads, S);
+  if (nseq > 1) {
+    // the other sequences of the batch share this state; each has its own window: x_ring[b][slot] = x[b]
+    __syncthreads();
+    if (st[ST_STATUS] != 0) return;
+    const int slot = st[ST_SLOT];
+    const int per = d / 8;
+    for (int c = threadIdx.x; c < (nseq - 1) * per; c += blockDim.x) {
+      const int b = 1 + c / per, k = c % per;
+      reinterpret_cast<uint4 *>(x_ring + (size_t)b * seq_ring + (size_t)slot * d)[k] =
+          reinterpret_cast<const uint4 *>(x + (size_t)b * d)[k];
+    }
+  }
 }
 
 __global__ void attn_finish_kernel(int *st) {
@@ -55,6 +68,7 @@ __global__ void attn_finish_kernel(int *st) {
 // the block sees the same set of token rows and the block-wide barriers are uniform.
 //   MODE 0: operator semantics (rows = batch_idx[i,:] >= 0, output y (T,3,nheads,hd))
 //   MODE 1: decode step (rows = bits of rowmask[i]; q of the current slot -> q_out, K/V -> caches)
+//   MODE 2: the same of a few sequences (see qkv_batch_takes)
 // ------------------------------------------------------------------------------------------
 constexpr int QKV_THREADS = 256;
 constexpr int QKV_WARPS = QKV_THREADS / WARP;
@@ -77,7 +91,17 @@ struct QkvArgs {
   const __half *x_cur;
   __half *x_ring_w;
   int early;  // MODE 1: the state is complete before this kernel can start; prefetch weights before the wait
+  // MODE 2: nseq sequences that share the state (same head selection, same window); elements between two
+  // sequences' windows (x), query rows (q_out) and caches. Block (., y) takes sequences y*QKV_SEQ_GROUP ..: their
+  // token rows go through the same pass over the weight rows, 16 at a time.
+  int nseq;
+  long long seq_x, seq_q, seq_k, seq_v;
 };
+constexpr int QKV_SEQ_GROUP = 8;  // sequences per block
+// a token row of MODE 2: (sequence << 4) | window slot
+__device__ __forceinline__ int row_seq(int code) { return code >> 4; }
+__device__ __forceinline__ int row_slot(int code) { return code & (DJV_KV_WINDOW - 1); }
+static_assert(DJV_KV_WINDOW == 16, "token-row codes keep the window slot in 4 bits");
 
 // ROWS weight rows against NB token rows: every activation chunk is loaded (through L1) once and used for
 // all ROWS weight rows, so L1 traffic per weight byte is NB / ROWS. Without that sharing a head with three
@@ -143,8 +167,10 @@ __device__ __forceinline__ void qkv_mma_rows(const QkvArgs &a, int qkv, int h, i
   for (int j = 0; j < NT; ++j) {
     xr[j] = nullptr;
     if (j * 8 + g < nrows) {
-      const int r = rows_s[j * 8 + g];
-      xr[j] = (MODE == 1 && a.x_cur != nullptr && r == cur_slot) ? a.x_cur : a.x + (size_t)r * a.d;
+      const int code = rows_s[j * 8 + g];
+      const int r = (MODE == 2) ? row_slot(code) : code;
+      const __half *xs = (MODE == 2) ? a.x + (size_t)row_seq(code) * a.seq_x : a.x;
+      xr[j] = (MODE >= 1 && a.x_cur != nullptr && r == cur_slot) ? a.x_cur : xs + (size_t)r * a.d;
     }
   }
 
@@ -197,17 +223,19 @@ __device__ __forceinline__ void qkv_mma_rows(const QkvArgs &a, int qkv, int h, i
     const int jj = jrow0 + tl * 16 + row;
     if (a.bias) sum += __half2float(a.bias[((size_t)qkv * a.nheads + h) * a.hd + jj]);
     const __half out = __float2half_rn(sum);
-    const int trow = rows_s[tok];
+    const int code = rows_s[tok];
+    const int trow = (MODE == 2) ? row_slot(code) : code;
+    const size_t sq = (MODE == 2) ? (size_t)row_seq(code) : 0;
     if (MODE == 0) {
       a.y[(((size_t)trow * 3 + qkv) * a.nheads + h) * a.hd + jj] = out;
     } else if (qkv == 1) {
       const int pos = base + trow;
-      a.k_cache[(((size_t)h * (a.hd / 8) + jj / 8) * a.S + pos) * 8 + jj % 8] = out;
+      a.k_cache[sq * a.seq_k + (((size_t)h * (a.hd / 8) + jj / 8) * a.S + pos) * 8 + jj % 8] = out;
     } else if (qkv == 2) {
       const int pos = base + trow;
-      a.v_cache[((size_t)h * a.S + pos) * a.hd + jj] = out;
+      a.v_cache[sq * a.seq_v + ((size_t)h * a.S + pos) * a.hd + jj] = out;
     } else {
-      a.q_out[(size_t)h * a.hd + jj] = out;
+      a.q_out[sq * a.seq_q + (size_t)h * a.hd + jj] = out;
     }
   }
 }
@@ -219,7 +247,7 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
   constexpr int GROUPS = QKV_WARPS / WPR;
   constexpr int RPB = GROUPS * ROWS;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (MODE == 1 && RPB >= 8 && a.early) {
+  if (MODE >= 1 && RPB >= 8 && a.early) {
     // The step was opened by an earlier, completed kernel (the caller's promise): the head this block works on
     // is known, so the first 4 KB of each of its weight rows are requested while the LayerNorm before this
     // kernel is still running.
@@ -240,7 +268,7 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int U = (ROWS == 1) ? 8 : (ROWS == 2 ? 4 : 2);  // ROWS * U = 8 weight loads in flight per lane
   __shared__ float red[QKV_WARPS][ROWS][8];
-  __shared__ int rows_s[DJV_KV_WINDOW];
+  __shared__ int rows_s[(MODE == 2 ? QKV_SEQ_GROUP : 1) * DJV_KV_WINDOW];
   __shared__ int nrows_s;
 
   const int jblocks = a.hd / RPB;
@@ -274,9 +302,12 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
         if (r >= 0) rows_s[n++] = r;
       }
     } else {
+      // the sequences of this block, sequence-major (all of them have the same pending window slots)
+      const int seq0 = MODE == 2 ? blockIdx.y * QKV_SEQ_GROUP : 0, seq1 = MODE == 2 ? min(a.nseq, seq0 + QKV_SEQ_GROUP) : 1;
       const unsigned m = (qkv == 0) ? (1u << slot) : (unsigned)st_rowmask(a.state, a.nheads)[i];
-      for (int s = 0; s <= slot; ++s)
-        if (m >> s & 1u) rows_s[n++] = s;
+      for (int sq = seq0; sq < seq1; ++sq)
+        for (int s = 0; s <= slot; ++s)
+          if (m >> s & 1u) rows_s[n++] = (sq << 4) | s;
     }
     nrows_s = n;
   }
@@ -286,8 +317,13 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
   if constexpr (RPB >= 8) {
     // full or half tensor-core tiles; measured faster than the CUDA-core path below even for one token row
     __shared__ float red_mma[QKV_WARPS * 2 * 16 * 8];
-    if (nrows <= 8) qkv_mma_rows<MODE, RPB, 1>(a, qkv, h, jb * RPB, nrows, rows_s, base, slot, red_mma);
-    else qkv_mma_rows<MODE, RPB, 2>(a, qkv, h, jb * RPB, nrows, rows_s, base, slot, red_mma);
+    // 16 token rows per pass over the block's weight rows
+    for (int r0 = 0; r0 < (MODE == 2 ? nrows : 1); r0 += 16) {
+      const int nr = MODE == 2 ? min(16, nrows - r0) : nrows;
+      if (MODE == 2 && r0 > 0) __syncthreads();  // the reduction buffer of the pass before has been read
+      if (nr <= 8) qkv_mma_rows<MODE, RPB, 1>(a, qkv, h, jb * RPB, nr, rows_s + r0, base, slot, red_mma);
+      else qkv_mma_rows<MODE, RPB, 2>(a, qkv, h, jb * RPB, nr, rows_s + r0, base, slot, red_mma);
+    }
     // (the CUDA-core path below is compiled for the one-row-per-block variant only)
   } else {
 
@@ -313,9 +349,11 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
     const uint4 *xp[NBMAX];
 #pragma unroll
     for (int r = 0; r < NBMAX; ++r) {
-      const int tr = rows_s[r0 + (r < nb ? r : 0)];
-      xp[r] = (MODE == 1 && a.x_cur != nullptr && tr == slot) ? reinterpret_cast<const uint4 *>(a.x_cur)
-                                                              : Xv + (size_t)tr * nchunks;
+      const int code = rows_s[r0 + (r < nb ? r : 0)];
+      const int tr = (MODE == 2) ? row_slot(code) : code;
+      const uint4 *xs = (MODE == 2) ? Xv + (size_t)row_seq(code) * (a.seq_x / 8) : Xv;
+      xp[r] = (MODE >= 1 && a.x_cur != nullptr && tr == slot) ? reinterpret_cast<const uint4 *>(a.x_cur)
+                                                              : xs + (size_t)tr * nchunks;
     }
     if (nb == 1) {
       const uint4 *x1[1] = {xp[0]};
@@ -370,17 +408,19 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
         const int j = j0 + jr;
         for (int r = 0; r < nb; ++r) {
           const __half out = __float2half_rn(acc[jr][r] + bv[jr]);
-          const int row = rows_s[r0 + r];
+          const int code = rows_s[r0 + r];
+          const int row = (MODE == 2) ? row_slot(code) : code;
+          const size_t sq = (MODE == 2) ? (size_t)row_seq(code) : 0;
           if (MODE == 0) {
             a.y[(((size_t)row * 3 + qkv) * a.nheads + h) * a.hd + j] = out;
           } else if (qkv == 0) {
-            a.q_out[(size_t)h * a.hd + j] = out;
+            a.q_out[sq * a.seq_q + (size_t)h * a.hd + j] = out;
           } else if (qkv == 1) {
             const int pos = base + row;
-            a.k_cache[(((size_t)h * (a.hd / 8) + j / 8) * a.S + pos) * 8 + j % 8] = out;
+            a.k_cache[sq * a.seq_k + (((size_t)h * (a.hd / 8) + j / 8) * a.S + pos) * 8 + j % 8] = out;
           } else {
             const int pos = base + row;
-            a.v_cache[((size_t)h * a.S + pos) * a.hd + j] = out;
+            a.v_cache[sq * a.seq_v + ((size_t)h * a.S + pos) * a.hd + j] = out;
           }
         }
       }
@@ -708,7 +748,7 @@ using namespace djv;
 // the largest that still gives every multiprocessor about two blocks. Very small calls put a whole block on
 // one row.
 template <int MODE>
-static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream_t st) {
+static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream_t st, int nseq = 1) {
   const long long sms = sm_count();
   // development knob, read at every launch: DJV_QKV_RPB (32, 16, 8 or 1: force the rows-per-block variant)
   const int force = env_int("DJV_QKV_RPB", 0);
@@ -717,7 +757,8 @@ static void launch_qkv(QkvArgs a, int capacity_heads, long long rows, cudaStream
   if (a.hd % rpb != 0) rpb = 8;
 #define DJV_QKV(WPR_, ROWS_)                                                                       \
   djv::launch_kernel(qkv_sparse_kernel<MODE, WPR_, ROWS_>,                                         \
-                     dim3(capacity_heads * 3 * (a.hd / ((QKV_WARPS / WPR_) * ROWS_))), QKV_THREADS, 0, st, a)
+                     dim3(capacity_heads * 3 * (a.hd / ((QKV_WARPS / WPR_) * ROWS_)), (nseq + QKV_SEQ_GROUP - 1) / QKV_SEQ_GROUP), \
+                     QKV_THREADS, 0, st, a)
   if (rpb == 32) DJV_QKV(1, 4);
   else if (rpb == 16) DJV_QKV(2, 4);
   else if (rpb == 8) DJV_QKV(2, 2);
@@ -921,14 +962,17 @@ static int attn_step_project(void *q_out, const void *wqkv, const void *bqkv, co
               "attn_step: pointers must be 16-byte aligned");
   DJV_REQUIRE(B == 1 || !step_is_open, "attn_step: a batch opens its step itself");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const long long seq_ring = (long long)DJV_KV_WINDOW * d;
   const int typical = head_idx ? (nnz > 0 ? nnz : 1) : nheads;
+  const bool together = B > 1 && qkv_batch_takes(B, typical, d, hd);
   if (!step_is_open) {
-    // (with several sequences the projection puts the token rows into their windows)
+    // (qkv_batch_kernel puts the token rows into their windows itself)
     djv::launch_kernel(attn_prep_kernel, 1, 1024, 0, st, state, head_idx, head_idx ? nnz : 0,
-                       B == 1 ? static_cast<const __half *>(x) : nullptr, static_cast<__half *>(x_ring), d, nheads, S);
+                       together ? nullptr : static_cast<const __half *>(x), static_cast<__half *>(x_ring), d, nheads, S,
+                       together ? 1 : B, seq_ring);
     count_launch();
   }
-  if (B > 1) {
+  if (together) {
     const QkvBatchArgs a{static_cast<const __half *>(wqkv), static_cast<const __half *>(bqkv), static_cast<const __half *>(x),
                          static_cast<__half *>(x_ring), state, static_cast<__half *>(q_out), static_cast<__half *>(k_cache),
                          static_cast<__half *>(v_cache), B, d, nheads, S};
@@ -948,12 +992,18 @@ static int attn_step_project(void *q_out, const void *wqkv, const void *bqkv, co
   a.k_cache = static_cast<__half *>(k_cache);
   a.v_cache = static_cast<__half *>(v_cache);
   a.S = S;
+  a.nseq = B;
+  a.seq_x = seq_ring;
+  a.seq_q = (long long)nheads * hd;
+  a.seq_k = (long long)nheads * hd * S;
+  a.seq_v = (long long)nheads * hd * S;
   if (step_is_open) {
     a.x_cur = static_cast<const __half *>(x);
     a.x_ring_w = static_cast<__half *>(x_ring);
     a.early = early_prefetch() ? 1 : 0;
   }
-  launch_qkv<1>(a, nheads, (long long)typical * 3 * hd, st);
+  if (B == 1) launch_qkv<1>(a, nheads, (long long)typical * 3 * hd, st);
+  else launch_qkv<2>(a, nheads, (long long)typical * 3 * hd, st, B);
   count_launch();
   return check_launch("attn_step_project");
 }

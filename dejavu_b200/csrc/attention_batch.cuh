@@ -1,7 +1,7 @@
 // The projections of a decode step of several sequences that share one lazy-K/V state, on the tensor cores
 // (mma.sync m16n8k16, fp16 in, fp32 accumulate): every selected head's weights are read from HBM once, whatever the batch.
 //
-//   qkv_batch_kernel   q, k, v of the heads in use: B x (1 + slots pending) token rows
+//   qkv_batch_kernel   q, k, v of the heads in use: B x (1 + slots pending) token rows (of 2 and 3 sequences: see qkv_batch_takes)
 //   out_proj_mma_kernel  output projection over the heads in use, up to 16 rows of the context
 #pragma once
 #include <cooperative_groups.h>
@@ -20,8 +20,9 @@ namespace djv {
 //
 // What bounds it: the weights from HBM, if the activations are not read too often. A block of 16 rows with all columns
 // (the form before) reads the token rows again for every 16 rows, and the weights again for every 16 token rows.
-// Splitting columns instead of rows over the device keeps the activations at 1 / 8 of that: 16 sequences, 12 of 32 heads of
-// 128, width 4096, mean over the steps of a window (16 to 256 token rows) 36.4 -> 28.5 us, 5.8 of them the weights at copy rate.
+// Splitting columns instead of rows over the device keeps the activations at 1 / 8 of that. The token rows of many sequences are
+// shared out over several clusters per head. 16 sequences, 12 of 32 heads of 128, 4096 wide, mean over the steps of a window (16 to
+// 256 token rows), with the step's opening: 38.3 -> 24.9 us, 5.8 of them the weights at copy rate.
 // -------------------------------------------------------------------------------------------
 constexpr int QB_THREADS = 256, QB_WARPS = QB_THREADS / WARP;
 constexpr int QB_K = 64;       // columns of a stage: 128 bytes of a row
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(QB_THREADS, 2) qkv_batch_kernel(QkvBatchArgs a
   const unsigned mask = (qkv == 0) ? (1u << slot) : (unsigned)st_rowmask(a.state, a.nheads)[i];
   if (status == 0) {  // nobody reads row `slot` of a window in this kernel: the current tokens are taken from x
     const int per = a.d / 8;
-    for (int b = gridDim.x - 1 - blockIdx.x; b < a.B; b += gridDim.x) {  // (the last blocks seldom have a head)
+    for (int b = gridDim.x - 1 - blockIdx.x + gridDim.x * blockIdx.y; b < a.B; b += gridDim.x * gridDim.y) {  // (the last blocks seldom have a head)
       const uint4 *src = reinterpret_cast<const uint4 *>(a.x + (size_t)b * a.d);
       uint4 *dst = reinterpret_cast<uint4 *>(a.x_ring + ((size_t)b * DJV_KV_WINDOW + slot) * a.d);
       for (int c = tid; c < per; c += QB_THREADS) dst[c] = src[c];
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(QB_THREADS, 2) qkv_batch_kernel(QkvBatchArgs a
   const __half *w = a.w + ((size_t)qkv * a.nheads + h) * HD * a.d;
   const __half *bias = a.bias ? a.bias + ((size_t)qkv * a.nheads + h) * HD : nullptr;
   float *red = reinterpret_cast<float *>(qb_ring);
-  for (int r0 = 0; r0 < a.B * pending; r0 += QB_TOKENS) {
+  for (int r0 = blockIdx.y * QB_TOKENS; r0 < a.B * pending; r0 += gridDim.y * QB_TOKENS) {
     const int nr = min(QB_TOKENS, a.B * pending - r0);
     if (tid < nr) {
       const int sq = (r0 + tid) / pending, s = (int)__fns(mask, 0, (r0 + tid) % pending + 1);
@@ -190,20 +191,36 @@ __global__ void __launch_bounds__(QB_THREADS, 2) qkv_batch_kernel(QkvBatchArgs a
   }
 }
 
-// Blocks per cluster: the blocks run in rounds of what is resident (two per multiprocessor; clusters of 8 leave about an
-// eighth of that empty), a round takes a block's column chunks and about 6 chunks' time for filling the ring and adding up.
-// Measured at heads of 128, width 4096, 16 token rows, us for clusters of 2 / 4 / 8: 12 heads 19.0 / 16.1 / 21.0 (64 rows
-// 31.4 / 25.2 / 24.0), 32 heads 26.7 / 31.9 / 34.0.
-inline int qkv_batch_split(int heads, int d, int hd) {
+// A few sequences stay with qkv_sparse_kernel, whose blocks take 8 to 32 rows with all columns each, so that a step is one wave of
+// loads: two, and three of middling width, unless the rows are so few that it would put a block on each. us a step with its opening,
+// qkv_sparse_kernel / qkv_batch_kernel, mean over a window: two sequences, 12 of 32 heads of 64, 2048 wide 10.4 / 11.1, 12 of 32 of
+// 128, 4096 wide 15.0 / 17.3, 16 of 40, 5120 wide 21.5 / 20.7, 24 of 72, 9216 wide 43.2 / 51.7, one head of 64, 768 wide 12.7 / 7.9;
+// three 11.4 / 11.4, 17.0 / 17.6, 24.9 / 21.2; four 12.3 / 11.6, 18.4 / 18.1, 28.2 / 23.0.
+inline bool qkv_batch_takes(int B, int heads, int d, int hd) {
+  return (long long)heads * 3 * hd < 2 * sm_count() || B > 3 || (B == 3 && (d <= 2048 || d > 4096));
+}
+
+// Blocks per cluster: the blocks run in rounds of what is resident, a round takes a block's column chunks, and the time of 4 to 6 of
+// them for filling the ring and adding up, 8 in clusters of 8. us at heads of 128, 16 sequences, clusters of 1 / 2 / 4 / 8: 4096
+// wide, 12 heads 82 / 49 / 32 / 28 (two sequences 31 / 20 / 17 / 20), 9216 wide, 24 heads 204 / 113 / 82 / 72 (65 / 45 / 53 / 52).
+// Clusters per head (grid.y), each with a share of the passes over token rows: a window leaves up to 16 rows for each sequence,
+// in a step with all heads for all of them. A cluster without rows is gone at once, and the weights come from L2 for all but the
+// first. us for 1 / 2 / 4: 4 of 12 heads of 64, 768 wide, 32 sequences 17.8 / 13.0 / 11.3 (qkv_sparse_kernel 17.0), 64 sequences
+// 29.5 / 20.1 / 14.7 (24.8); 12 of 32 of 128, 4096 wide, 16 sequences 31.6 / 24.9 / 24.7, 8 sequences 21.7 / 21.3 / 21.3.
+struct QkvBatchPlan {
+  int S, shares;
+};
+inline QkvBatchPlan qkv_batch_plan(int B, int heads, int d, int hd, const int (&resident)[4]) {
   const int chunks = ceil_div(d, QB_K), pairs = 3 * (heads > 0 ? heads : 1);
-  int best = 1;
+  QkvBatchPlan best{1, B < 8 ? 1 : B < 32 ? 2 : 4};
+  const int chunk = B < 4 ? 2 : 3;
   long long least = -1;
-  for (int S = 1; S <= 8 && S <= chunks && S * 4 <= hd; S *= 2) {
-    const int slots = S == 8 ? sm_count() * 7 / 4 : sm_count() * 2;
-    const long long cost = (long long)ceil_div(pairs * S, slots) * (ceil_div(chunks, S) + 6);
+  for (int i = 0, S = 1; i < 4 && S <= chunks && S * 4 <= hd; ++i, S *= 2) {
+    if (resident[i] < 1) continue;
+    const long long cost = (long long)ceil_div(pairs, resident[i]) * (chunk * ceil_div(chunks, S) + (S == 8 ? 18 : 12));
     if (least < 0 || cost < least) {
       least = cost;
-      best = S;
+      best.S = S;
     }
   }
   return best;
@@ -214,16 +231,16 @@ static int launch_qkv_batch(const QkvBatchArgs &a, int heads, cudaStream_t st) {
   constexpr size_t smem = QkvBatchSmem<HD>::BYTES;
   static_assert(smem <= 113 * 1024, "shared memory of two blocks");
   static DevicePrep prep;
-  const int (*unused)[4];
-  const cudaError_t prepared = prep.get([](int (&)[4]) {
-    return cudaFuncSetAttribute(qkv_batch_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }, unused);
+  const int (*resident)[4];
+  const cudaError_t prepared = prep.get([](int (&r)[4]) {
+    return cluster_residency(qkv_batch_kernel<HD>, QB_THREADS, (int)smem, 2, r);
+  }, resident);
   if (prepared != cudaSuccess) {
     set_error("attn_step: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
   }
-  const int S = qkv_batch_split(heads, a.d, HD);
-  djv::launch_kernel_cluster(qkv_batch_kernel<HD>, dim3(a.nheads * 3 * S), dim3(QB_THREADS), smem, st, dim3(S), a);
+  const QkvBatchPlan p = qkv_batch_plan(a.B, heads, a.d, HD, *resident);
+  djv::launch_kernel_cluster(qkv_batch_kernel<HD>, dim3(a.nheads * 3 * p.S, p.shares), dim3(QB_THREADS), smem, st, dim3(p.S), a);
   return DJV_OK;
 }
 

@@ -108,6 +108,27 @@ class DevicePrep {
   int resident_[MAX][4] = {};
 };
 
+// For a DevicePrep: lets `kernel` take `smem` bytes and asks how many clusters of 1, 2, 4, 8 blocks are resident at once. Clusters
+// stay inside a group of multiprocessors, so fewer of the larger ones fit than the multiprocessors have room for.
+template <typename... P>
+inline cudaError_t cluster_residency(void (*kernel)(P...), int threads, int smem, int per_sm, int (&resident)[4]) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1 << i;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(sm_count() * per_sm / 8 * 8);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaOccupancyMaxActiveClusters(&resident[i], kernel, &cfg);
+  }
+  return e;
+}
+
 // ---- device side --------------------------------------------------------------------------
 constexpr int WARP = 32;
 

@@ -15,7 +15,8 @@ def near(got, want):
 
 # token rows per pass (1 .. 64) and passes, columns that end inside a stage, fewer columns than a cluster has blocks
 @pytest.mark.parametrize("B,nheads,hd,d", [(2, 5, 32, 8), (3, 4, 64, 328), (5, 32, 128, 4096), (9, 3, 128, 1000), (16, 12, 64, 768),
-                                           (17, 2, 32, 72), (33, 2, 128, 136)])
+                                           (17, 2, 32, 72), (33, 2, 128, 136), (2, 12, 128, 768), (2, 30, 32, 72), (3, 12, 64, 2056),
+                                           (3, 9, 128, 4104), (47, 3, 64, 136)])
 def test_lazy_projection_of_a_batch(cuda, B, nheads, hd, d):
     from dejavu_b200 import _lib, ops
 

@@ -108,3 +108,19 @@ for B in (5, 8):
 for B in (1, 2):
     assert kernel(B, 4096, 4096) == "rowdot"
 """)
+
+
+def test_projections_of_few_and_of_many_sequences(fake):
+    run(fake, """
+lib = load("libdejavu_b200.so")
+def project(B, nheads, nnz, hd, d):
+    done(lib, lib.djv_attn_step_project_batch(ptr, ptr, None, ptr, ptr, ptr, ptr, ptr, ptr, nnz, d, nheads, hd, 64, B, None))
+    return [n for n in notes() if n["what"] == "launch"][-1]
+assert "qkv_sparse" in project(2, 32, 12, 128, 4096)["kernel"]
+assert "qkv_sparse" in project(3, 32, 12, 128, 4096)["kernel"]
+assert "qkv_batch" in project(2, 12, 1, 64, 768)["kernel"]
+assert "qkv_batch" in project(3, 72, 24, 128, 9216)["kernel"]
+for B, shares in ((7, 1), (16, 2), (64, 4)):
+    n = project(B, 12, 4, 64, 768)
+    assert "qkv_batch" in n["kernel"] and n["grid"] == 12 * 3 * n["cluster"] * shares, n
+""")
