@@ -31,8 +31,8 @@ template <int B, int ACT>
 static void launch_rowdot(const RowdotPlan &p, __half *Y, const __half *W, const __half *X,
                           const void *idx, const __half *bias, int M, int N, long long ldw,
                           int idx64, cudaStream_t st) {
-#define DJV_RD(WPR_, R_, U_)                                                                                            \
-  djv::launch_kernel(rowdot_kernel<__half, __half, B, ACT, WPR_, R_, U_>, p.grid, RD_THREADS, 0, st, Y, W, X, idx, bias, \
+#define DJV_RD(WPR_, R_, U_, BL_, SP_)                                                                                            \
+  djv::launch_kernel(rowdot_kernel<__half, __half, B, ACT, WPR_, R_, U_, BL_, SP_>, p.grid, RD_THREADS, 0, st, Y, W, X, idx, bias, \
                      M, N, ldw, idx64, (idx == nullptr || early_prefetch()) ? 1 : 0, 0.f, p.per_block, p.rest)
   DJV_ROWDOT(p, B, DJV_RD);
 #undef DJV_RD

@@ -35,8 +35,8 @@ template <typename T, typename TO, int B, int ACT>
 static void launch_rowdot_dense(TO *Y, const T *W, const T *X, int M, int N, long long ldw, float param,
                                 cudaStream_t st) {
   const RowdotPlan p = plan_rowdot(M, N / Chunk<T>::N, is_glu(ACT) ? 2 : 1, B);
-#define DJV_RD(WPR_, R_, U_)                                                                                            \
-  djv::launch_kernel(rowdot_kernel<T, TO, B, ACT, WPR_, R_, U_>, p.grid, RD_THREADS, 0, st, Y, W, X,                     \
+#define DJV_RD(WPR_, R_, U_, BL_, SP_)                                                                                            \
+  djv::launch_kernel(rowdot_kernel<T, TO, B, ACT, WPR_, R_, U_, BL_, SP_>, p.grid, RD_THREADS, 0, st, Y, W, X,                     \
                      static_cast<const void *>(nullptr), static_cast<const T *>(nullptr), M, N, ldw, 0, 1, param, \
                      p.per_block, p.rest)
   DJV_ROWDOT(p, B, DJV_RD);

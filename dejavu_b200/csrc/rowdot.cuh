@@ -42,19 +42,19 @@ __device__ __forceinline__ float apply_act_param(float v, float p) {
 constexpr int RD_THREADS = 256;
 constexpr int RD_WARPS = RD_THREADS / WARP;
 constexpr int RD_SPAN = 128;  // rows whose sums a block keeps before it finishes them
+constexpr int RD_FEW = 8;     // as many as a block with 4 chunks per row can have
 
 // Blocks per multiprocessor that the registers of a pass leave room for: ROWS * U 16-byte loads, ROWS * B sums.
 __host__ __device__ constexpr int rd_blocks(int B) { return B == 1 ? 4 : B == 2 ? 3 : B <= 4 ? 2 : 1; }
 
-template <typename T, typename TO, int B, int ACT, int WPR, int ROWS, int U>
-__global__ void __launch_bounds__(RD_THREADS, rd_blocks(B))
+template <typename T, typename TO, int B, int ACT, int WPR, int ROWS, int U, int BLOCKS, int SPAN>
+__global__ void __launch_bounds__(RD_THREADS, BLOCKS)
 rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__ X,
               const void *__restrict__ idx, const T *__restrict__ bias, int M, int N,
               long long ldw, int idx64, int early, float act_param, int per_block, int rest) {
   constexpr int UNIT = is_glu(ACT) ? 2 : 1;  // rows 2i, 2i + 1 of the matrix are the gate and up rows of output i
   constexpr int GROUPS = RD_WARPS / WPR;
   constexpr int GLANES = WARP * WPR;
-  constexpr int SPAN = U == 4 ? 2 : RD_SPAN;  // (with 4 chunks per row a block has two rows at most)
   __shared__ float red[B][SPAN][WPR];
 
   const int tid = threadIdx.x;
@@ -82,10 +82,13 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // the bias of the output that this thread finishes first, on its way while the products are made
-  const int outs0 = min(last - first, SPAN) / UNIT;
-  float bias0 = 0.f;
-  if (UNIT == 1 && bias != nullptr && tid < outs0 * B) bias0 = to_f(bias[load_index(idx, first + tid % outs0, idx64)]);
+  // The bias of the output that this thread finishes first: its row number is asked for together with those of the first pass,
+  // and it is on its way, unread, while that pass makes the products. (A thread without a row in that pass loads it at the end.)
+  constexpr int SO = SPAN / UNIT;  // outputs of a span, for every row of x
+  const int m_first = first + group * ROWS, m_bias = first + tid % SO;
+  long long bias_row = -1;
+  if (UNIT == 1 && bias != nullptr && m_first < last && m_bias < last && tid < SO * B) bias_row = load_index(idx, m_bias, idx64);
+  T bias0 = T(0.f);
 
   for (int s0 = first; s0 < last; s0 += SPAN) {  // (the same trips for all threads of the block)
     const int s1 = min(last, s0 + SPAN);
@@ -96,6 +99,7 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
         const long long r = m0 + j < s1 ? load_index(idx, m0 + j, idx64) : -1;
         wp[j] = r < 0 ? nullptr : reinterpret_cast<const uint4 *>(W + r * ldw);
       }
+      if (UNIT == 1 && m0 == m_first && bias_row >= 0) bias0 = bias[bias_row];
       float acc[ROWS][B];
 #pragma unroll
       for (int j = 0; j < ROWS; ++j)
@@ -133,8 +137,9 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
     }
     __syncthreads();
     const int outs = (s1 - s0) / UNIT;
-    for (int o = tid; o < outs * B; o += RD_THREADS) {
-      const int b = o / outs, i = o % outs;
+    for (int o = tid; o < SO * B; o += RD_THREADS) {
+      const int b = o / SO, i = o % SO;
+      if (i >= outs) continue;
       float v[UNIT];
 #pragma unroll
       for (int j = 0; j < UNIT; ++j) {
@@ -143,7 +148,7 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
 #pragma unroll
         for (int w2 = 0; w2 < WPR; ++w2) v[j] += red[b][row][w2];
         if (UNIT == 1 && bias != nullptr)
-          v[j] += s0 == first && o == tid ? bias0 : to_f(bias[load_index(idx, s0 + row, idx64)]);
+          v[j] += to_f(s0 == first && o == tid && bias_row >= 0 ? bias0 : bias[load_index(idx, s0 + row, idx64)]);
       }
       const size_t at = (size_t)b * units + s0 / UNIT + i;
       if constexpr (is_glu(ACT)) Y[at] = from_f<TO>(apply_glu<ACT>(v[0], v[1], act_param));
@@ -153,57 +158,85 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   }
 }
 
+// What a lane has under way of a pass: 4 rows x 2 chunks; 2 rows x 4 chunks where a block has few rows (RD_FEW_ROWS); for two rows
+// of x also those with a block more per multiprocessor (RD_FOUR_BLOCKS).
+enum RowdotForm { RD_FOUR_ROWS, RD_FEW_ROWS, RD_FOUR_BLOCKS };
+
 struct RowdotPlan {
   int wpr, grid, per_block, rest;
-  bool few;  // at most two rows per block: 2 rows x 4 chunks per lane instead of 4 x 2
+  RowdotForm form;
 };
 
-// A block with p rows makes ceil(p / (groups * 4)) passes of ceil(nchunks / (64 * wpr)) trips of the chunk loop, and a pass
-// costs about one trip on top (row pointers, sums of the warps, a block barrier at the end). The least of the four is
-// within 3 % of the best of them at every shape above; of equals the one with fewer lanes per row has more rows under way.
-inline RowdotPlan plan_rowdot(int M, int nchunks, int unit, int B) {
+// A block with p rows makes ceil(p / (groups * rows)) passes of ceil(nchunks / (32 * wpr * chunks)) trips of the chunk loop, and a
+// pass costs about one trip on top (row pointers, sums of the warps, a block barrier at the end). The least is within 3 % of the
+// best at every shape above; of equals the one with fewer lanes per row has more rows under way, but a block that is done after
+// one pass of few rows wants all its warps in it.
+inline long long rowdot_cost(int p, int nchunks, int rows, int &wpr) {
   static const int k_wpr = env_int("DJV_RD_WPR", 0);  // development knob
-  const int slots = sm_count() * rd_blocks(B), units = M / unit;
-  const int p = ceil_div(units, slots) * unit;
-  RowdotPlan r{};
-  r.few = B == 1 && p <= 2;
-  if (r.few)
-    for (r.wpr = 8; r.wpr > 1 && nchunks < WARP * r.wpr;) r.wpr /= 2;
   long long best = -1;
-  for (int wpr = 1; wpr <= 8 && !r.few; wpr *= 2) {
-    const int passes = ceil_div(p, RD_WARPS / wpr * 4);
-    const long long cost = (long long)passes * (ceil_div(nchunks, WARP * wpr * 2) + 1);
-    if (best < 0 || cost < best) {
+  for (int w = 1; w <= 8; w *= 2) {
+    const int at_once = RD_WARPS / w * rows;
+    const long long cost = (long long)ceil_div(p, at_once) * (ceil_div(nchunks, WARP * w * (8 / rows)) + 1);
+    if (best < 0 || cost < best || (rows == 2 && cost == best && p <= at_once && nchunks >= WARP * w)) {
       best = cost;
-      r.wpr = wpr;
+      wpr = w;
     }
   }
-  if (k_wpr > 0) r.wpr = k_wpr;
-  r.grid = max(1, min(slots, ceil_div(M, r.few ? 2 : unit)));
+  if (k_wpr > 0) wpr = k_wpr;
+  return best;
+}
+
+// Few rows: 2 per block, or up to 5 short ones with several rows of x. us, 4 x 2 / 2 x 4: two rows of x 512 x 12288 7.1 / 5.8,
+// 512 x 9216 6.3 / 5.5, 2048 x 1024 2.5 / 2.4; three 512 x 12288 6.6 / 5.8, 512 x 4096 3.9 / 3.4; but 1024 x 12288 7.8 / 8.3 (two),
+// 7.8 / 8.7 (three). A block more for two rows of x where that saves a tenth of the trips on a multiprocessor: 4096 x 4096
+// 9.3 / 8.2, 4096 x 12288 21.9 / 19.6; but 12352 x 4096 17.9 / 21.3, 6144 x 4096 10.3 / 11.2.
+inline RowdotPlan plan_rowdot(int M, int nchunks, int unit, int B) {
+  const int units = M / unit;
+  int slots = sm_count() * rd_blocks(B), p = ceil_div(units, slots) * unit;
+  RowdotPlan r{};
+  r.form = B <= 4 && (p <= 2 || (B > 1 && p <= 5 && nchunks <= 256)) ? RD_FEW_ROWS : RD_FOUR_ROWS;
+  const int q = r.form == RD_FEW_ROWS ? max(2, p) : p;
+  const long long cost = rowdot_cost(q, nchunks, r.form == RD_FEW_ROWS ? 2 : 4, r.wpr);
+  if (B == 2 && r.form == RD_FOUR_ROWS) {
+    const int more = sm_count() * 4;
+    int wpr;
+    if (rowdot_cost(ceil_div(units, more) * unit, nchunks, 2, wpr) * 4 * 10 <= cost * 3 * 9) {
+      r.form = RD_FOUR_BLOCKS;
+      r.wpr = wpr;
+      slots = more;
+    }
+  }
+  r.grid = max(1, min(slots, r.form == RD_FEW_ROWS ? ceil_div(M, q) : units));
   r.per_block = units / r.grid;
   r.rest = units % r.grid;
   return r;
 }
 
-// launch(WPR, ROWS, U) with compile-time arguments
-#define DJV_ROWDOT_WPR(plan, ROWS_, U_, LAUNCH)       \
-  do {                                                \
-    switch ((plan).wpr) {                             \
-      case 1: LAUNCH(1, ROWS_, U_); break;            \
-      case 2: LAUNCH(2, ROWS_, U_); break;            \
-      case 4: LAUNCH(4, ROWS_, U_); break;            \
-      default: LAUNCH(8, ROWS_, U_); break;           \
-    }                                                 \
+// launch(WPR, ROWS, U, BLOCKS, SPAN) with compile-time arguments
+#define DJV_ROWDOT_WPR(plan, ROWS_, U_, BLOCKS_, SPAN_, LAUNCH)       \
+  do {                                                                \
+    switch ((plan).wpr) {                                             \
+      case 1: LAUNCH(1, ROWS_, U_, BLOCKS_, SPAN_); break;            \
+      case 2: LAUNCH(2, ROWS_, U_, BLOCKS_, SPAN_); break;            \
+      case 4: LAUNCH(4, ROWS_, U_, BLOCKS_, SPAN_); break;            \
+      default: LAUNCH(8, ROWS_, U_, BLOCKS_, SPAN_); break;           \
+    }                                                                 \
   } while (0)
-#define DJV_ROWDOT(plan, B_, LAUNCH)                  \
-  do {                                                \
-    if constexpr ((B_) == 1) {                        \
-      if ((plan).few) {                               \
-        DJV_ROWDOT_WPR(plan, 2, 4, LAUNCH);           \
-        break;                                        \
-      }                                               \
-    }                                                 \
-    DJV_ROWDOT_WPR(plan, 4, 2, LAUNCH);               \
+#define DJV_ROWDOT(plan, B_, LAUNCH)                                                  \
+  do {                                                                                \
+    if constexpr ((B_) <= 4) {                                                        \
+      if ((plan).form == RD_FEW_ROWS) {                                               \
+        DJV_ROWDOT_WPR(plan, 2, 4, rd_blocks(B_), RD_FEW, LAUNCH);                    \
+        break;                                                                        \
+      }                                                                               \
+    }                                                                                 \
+    if constexpr ((B_) == 2) {                                                        \
+      if ((plan).form == RD_FOUR_BLOCKS) {                                            \
+        DJV_ROWDOT_WPR(plan, 2, 4, 4, RD_SPAN, LAUNCH);                               \
+        break;                                                                        \
+      }                                                                               \
+    }                                                                                 \
+    DJV_ROWDOT_WPR(plan, 4, 2, rd_blocks(B_), RD_SPAN, LAUNCH);                       \
   } while (0)
 
 }  // namespace djv

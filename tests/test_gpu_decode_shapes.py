@@ -67,6 +67,25 @@ def test_weights_streamed_for_several_rows(cuda, B, N, M):
     near(ops.gather_gemv(x.half(), w.half(), idx, bias, "relu"), want)
 
 
+# rows per block around where the forms of a pass change, fewer rows than warps, a bias that belongs to no row of the first pass
+@pytest.mark.parametrize("B", [2, 3, 4])
+@pytest.mark.parametrize("N,M", [(8, 1), (768, 385), (2048, 889), (2048, 1481), (2056, 1481), (4096, 593), (4104, 2049), (12288, 445), (3080, 4097)])
+def test_few_rows_of_a_few_tokens(cuda, B, N, M):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + N + M)
+    x = torch.randn(B, N, device=cuda, generator=g).half()
+    w = (torch.randn(M + 7, N, device=cuda, generator=g) * N ** -0.5).half()
+    bias = torch.randn(M + 7, device=cuda, generator=g).half()
+    idx = torch.randperm(M + 7, device=cuda, generator=g)[:M]
+    y = x.double() @ w.double().t()
+    near(ops.gather_gemv(x, w, idx, bias, "relu"), (y + bias.double())[:, idx].relu())
+    near(ops.dense_gemv(x, w), y)
+    pairs = w[:(M + 7) // 2 * 2].bfloat16()
+    p = x.bfloat16().double() @ pairs.double().t()
+    near(ops.linear_gemv(x.bfloat16(), pairs, None, "silu_glu"), p[:, 0::2] * torch.sigmoid(p[:, 0::2]) * p[:, 1::2])
+
+
 # both sides of the line between the form without a ring and the ring; parts of a tile, of a 32-column block, of a split
 @pytest.mark.parametrize("B", [5, 8, 9, 16, 17, 25, 32])
 @pytest.mark.parametrize("N,M", [(8, 1), (40, 17), (512, 2048), (520, 257), (1024, 4096), (1032, 513), (2048, 1026), (4096, 2048), (4104, 512),

@@ -110,6 +110,21 @@ for B in (1, 2):
 """)
 
 
+def test_rows_of_two_tokens_are_dealt_out_without_idle_warps(fake):
+    """(rows, chunks per row, blocks per multiprocessor) of the product's kernel, and that its blocks have all rows."""
+    run(fake, """
+import re
+lib = load("libdejavu_b200.so")
+for B, N, M, form in ((1, 12288, 512, "2,4,4"), (1, 4096, 4096, "4,2,4"), (2, 12288, 512, "2,4,3"), (2, 4096, 4096, "2,4,4"),
+                      (2, 12288, 4096, "2,4,4"), (2, 4096, 12352, "4,2,3"), (3, 4096, 512, "2,4,2"), (4, 12288, 512, "2,4,2"),
+                      (3, 12288, 1024, "4,2,2")):
+    done(lib, lib.djv_gather_gemv(ptr, ptr, ptr, ptr, None, B, N, M, L(N), 0, 1, None))
+    n, = notes()
+    rows, chunks, blocks = re.search("rowdot_kernelI.*Li[1248]ELi([24])ELi([24])ELi([0-9])ELi(?:8|128)EE", n["kernel"]).groups()
+    assert ",".join((rows, chunks, blocks)) == form and n["grid"] <= 148 * int(blocks), (B, N, M, n)
+""")
+
+
 def test_projections_of_few_and_of_many_sequences(fake):
     run(fake, """
 lib = load("libdejavu_b200.so")
