@@ -319,49 +319,100 @@ __global__ void __launch_bounds__(MO_THREADS) moe_decode_down_kernel(MoeDecodeAr
 // 8 sequences, 8 experts of 3648 x 4096 and the shared one, us: up 114 -> 87 (75 at copy rate), down 83 -> 51 (38). Before,
 // a block took 16 rows and all columns, with no loads under way while it found its experts or added up. (Finding a chunk's
 // expert by a division for every chunk cost the down stage 24 us.)
-constexpr int MM_B = 32;
+constexpr int MM_B = 32, MM_E = 1137;
 
-// every block finds for itself: list [n] of experts in use, place [E][MM_B] of an expert among a sequence's choices or -1
-__device__ __forceinline__ int moe_in_use(const MoeDecodeArgs &a, int *list, signed char *place, int *n_list) {
-  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP;
-  for (int i = tid; i < a.E * MM_B / 4; i += WR_THREADS) reinterpret_cast<int *>(place)[i] = -1;
+// Who chose what, in the shared memory that two blocks per multiprocessor leave behind their rings: the experts in use in
+// ascending order, a bit for every expert, and an expert's place among a sequence's choices, as a byte for every expert and sequence
+// where there is room for that, else as the sequences' choices, which are looked through. (Bytes for 32 sequences whatever their
+// number left room for one block from 57 experts on with 24 sequences, from 112 on with 8: 64 experts of 704 x 2048, 24 sequences,
+// 165 us so, 100 now; 112 of 512 x 1024, 8 sequences, 52 and 27.)
+template <int NT>
+struct MoeTable {
+  static constexpr int SEQS = NT * 8, BITS = (MM_E + 31) / 32 * 4, LIST = SEQS * MAX_TOP * 2, CHOICES = SEQS * MAX_TOP * 2;
+  static constexpr int BYTES = 115344 - WeightRing<NT>::BYTES;  // (two blocks of 115344 bytes are resident, two of 115648 are not)
+  static_assert(BYTES >= BITS + LIST + CHOICES, "");
+  static bool has_places(int E) { return E * SEQS <= BYTES - BITS - LIST; }
+};
+
+template <int NT, bool PLACES>
+struct MoeInUse {
+  const signed char *places;  // [E][SEQS]
+  const unsigned *choices;    // [B][pairs], two to a word
+  const short *list;          // [n] experts in use
+  int n, pairs;
+
+  // the expert's place among the sequence's choices, or -1
+  __device__ __forceinline__ int place(int e, int b) const {
+    if (PLACES) return places[e * MoeTable<NT>::SEQS + b];
+    int s = -1;
+    for (int k = 0; k < pairs; ++k) {
+      const unsigned two = choices[b * pairs + k];
+      if ((two & 0xffffu) == (unsigned)e) s = 2 * k;
+      if (two >> 16 == (unsigned)e) s = 2 * k + 1;
+    }
+    return s;
+  }
+};
+
+// every block finds for itself
+template <int NT, bool PLACES>
+__device__ __forceinline__ MoeInUse<NT, PLACES> moe_in_use(const MoeDecodeArgs &a, unsigned char *table, int *n_s) {
+  using Table = MoeTable<NT>;
+  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, pairs = (a.top + 1) / 2, words = (a.E + 31) / 32;
+  unsigned *bits = reinterpret_cast<unsigned *>(table);
+  short *list = reinterpret_cast<short *>(table + Table::BITS);
+  signed char *places = reinterpret_cast<signed char *>(table + Table::BITS + Table::LIST);
+  unsigned short *choices = reinterpret_cast<unsigned short *>(places);
+  for (int i = tid; i < words; i += WR_THREADS) bits[i] = 0u;
+  if (PLACES)
+    for (int i = tid; i < a.E * Table::SEQS / 4; i += WR_THREADS) reinterpret_cast<int *>(places)[i] = -1;
   __syncthreads();
   for (int b = warp; b < a.B; b += WR_WARPS) {
     int e;
     float v;
     warp_topk(a.z + (size_t)b * a.E, a.E, a.top, e, v);
-    if (lane < a.top) place[e * MM_B + b] = (signed char)lane;
+    if (lane < a.top) atomicOr(bits + e / 32, 1u << e % 32);
+    if (PLACES) {
+      if (lane < a.top) places[e * Table::SEQS + b] = (signed char)lane;
+    } else if (lane < 2 * pairs) {
+      choices[b * 2 * pairs + lane] = lane < a.top ? (unsigned short)e : (unsigned short)0xffff;
+    }
   }
   __syncthreads();
   if (warp == 0) {
     int n = 0;
-    for (int e0 = 0; e0 < a.E; e0 += WARP) {
-      bool used = false;
-      if (e0 + lane < a.E)
-        for (int b = 0; b < a.B; ++b) used |= place[(e0 + lane) * MM_B + b] >= 0;
-      const unsigned mask = __ballot_sync(0xffffffffu, used);
-      if (used) list[n + __popc(mask & ((1u << lane) - 1))] = e0 + lane;
-      n += __popc(mask);
+    for (int w0 = 0; w0 < words; w0 += WARP) {
+      unsigned m = w0 + lane < words ? bits[w0 + lane] : 0u;
+      int at = __popc(m);  // experts of this lane and those before it
+#pragma unroll
+      for (int o = 1; o < WARP; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += up;
+      }
+      const int all = __shfl_sync(0xffffffffu, at, WARP - 1);
+      at += n - __popc(m);
+      for (; m; m &= m - 1) list[at++] = (short)((w0 + lane) * 32 + __ffs(m) - 1);
+      n += all;
     }
-    if (lane == 0) *n_list = n;
+    if (lane == 0) *n_s = n;
   }
   __syncthreads();
-  return *n_list;
+  return {places, reinterpret_cast<const unsigned *>(choices), list, *n_s, pairs};
 }
 
+template <int NT, bool PLACES>
 struct MoeUpSource {
   const MoeDecodeArgs &a;
-  const int *list;
-  const signed char *place;
-  int n_list, slots, first, last, rows, S, rank;  // units (pairs of rows) of the cluster; weight rows of its tiles
+  const MoeInUse<NT, PLACES> used;
+  int slots, first, last, rows, S, rank;  // units (pairs of rows) of the cluster; weight rows of its tiles
   const bf16 *row[WR_WP];
   int k;
 
   // the expert of a unit (E: the shared one), and the unit's number in it
   __device__ __forceinline__ int expert(int &unit) const {
-    const int at = min(unit / a.F, n_list);
+    const int at = min(unit / a.F, used.n);
     unit -= at * a.F;
-    return at < n_list ? list[at] : a.E;
+    return at < used.n ? used.list[at] : a.E;
   }
   __device__ __forceinline__ void seek(int t, int c) {
     if (c == 0)
@@ -392,27 +443,27 @@ struct MoeUpSource {
   __device__ __forceinline__ void store(int t, int pair, int b, float2 v) const {
     int unit = first + t * rows / 2 + pair;
     if (2 * pair >= rows || unit >= last) return;
-    const int e = expert(unit), s = e == a.E ? a.top : place[e * MM_B + b];
+    const int e = expert(unit), s = e == a.E ? a.top : used.place(e, b);
     if (s < 0) return;
     const float wt = e == a.E ? 1.f : sigmoid_f(a.z[(size_t)b * a.E + e]);
     static_cast<bf16 *>(a.act)[((size_t)b * slots + s) * a.ld_act + unit] = from_f<bf16>(silu_glu(wt * v.x, wt * v.y));
   }
 };
 
+template <int NT, bool PLACES>
 struct MoeDownSource {
   const MoeDecodeArgs &a;
-  const int *list;
-  const signed char *place;
-  int n_list, slots, first, last, rows, S, rank;  // rows of the cluster, of its tiles
-  // the chunk's number in its expert, the expert's chunks, row length and place in the list (n_list: the shared one), and of
+  const MoeInUse<NT, PLACES> used;
+  int slots, first, last, rows, S, rank;  // rows of the cluster, of its tiles
+  // the chunk's number in its expert, the expert's chunks, row length and place in the list (used.n: the shared one), and of
   // the thread's pieces the rows of weights and of activations (xs: whether the sequence chose the expert)
   int j, kf, F, at, k;
   const bf16 *row[WR_WP], *act[(MM_B + WR_RP - 1) / WR_RP];
   bool xs[(MM_B + WR_RP - 1) / WR_RP];
 
   __device__ __forceinline__ void enter(int t) {
-    const bool shared = at == n_list;
-    const int e = shared ? a.E : list[at];
+    const bool shared = at == used.n;
+    const int e = shared ? a.E : used.list[at];
     F = shared ? a.F_shared : a.F;
     kf = ceil_div_dev(F, WR_K);
     const bf16 *base = shared ? static_cast<const bf16 *>(a.shared_down) : static_cast<const bf16 *>(a.w_down) + (size_t)e * a.D * a.F;
@@ -424,7 +475,7 @@ struct MoeDownSource {
 #pragma unroll
     for (int i = 0; i < (MM_B + WR_RP - 1) / WR_RP; ++i) {
       const int b = (int)threadIdx.x / WR_PPR + WR_RP * i;
-      const int s = b >= a.B ? -1 : shared ? a.top : place[e * MM_B + b];
+      const int s = b >= a.B ? -1 : shared ? a.top : used.place(e, b);
       xs[i] = s >= 0;
       act[i] = b < a.B ? static_cast<const bf16 *>(a.act) + ((size_t)b * slots + max(s, 0)) * a.ld_act : nullptr;
     }
@@ -437,7 +488,7 @@ struct MoeDownSource {
     } else {
       j += S;
     }
-    while (j >= kf && at < n_list) {  // (the list ends with the shared expert, or with the last chunk)
+    while (j >= kf && at < used.n) {  // (the list ends with the shared expert, or with the last chunk)
       j -= kf;
       ++at;
       enter(t);
@@ -462,16 +513,15 @@ struct MoeDownSource {
   }
 };
 
-template <int NT, bool UP>
+template <int NT, bool UP, bool PLACES>
 __global__ void __launch_bounds__(WR_THREADS, WR_BPS) moe_ring_kernel(MoeDecodeArgs a, int slots) {
   extern __shared__ __align__(128) unsigned char wr_smem[];
   __shared__ int n_s;
-  int *list = reinterpret_cast<int *>(wr_smem + WeightRing<NT>::BYTES);
-  signed char *place = reinterpret_cast<signed char *>(list + a.E);
   pdl_prologue();
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), cl = blockIdx.x / S, clusters = gridDim.x / S;
-  const int n = moe_in_use(a, list, place, &n_s);
+  const MoeInUse<NT, PLACES> used = moe_in_use<NT, PLACES>(a, wr_smem + WeightRing<NT>::BYTES, &n_s);
+  const int n = used.n;
   const bool shared = a.shared_gu != nullptr;
   const int units = UP ? n * a.F + (shared ? a.F_shared : 0) : a.D, per = units / clusters, rest = units % clusters;
   const int first = cl * per + min(cl, rest), last = first + per + (cl < rest ? 1 : 0), rows_all = (last - first) * (UP ? 2 : 1);
@@ -479,24 +529,20 @@ __global__ void __launch_bounds__(WR_THREADS, WR_BPS) moe_ring_kernel(MoeDecodeA
   const int all = UP ? ceil_div_dev(a.D, WR_K) : n * ceil_div_dev(a.F, WR_K) + (shared ? ceil_div_dev(a.F_shared, WR_K) : 0);
   const int chunks = rank < all ? (all - rank + S - 1) / S : 0;
   if constexpr (UP) {
-    MoeUpSource src{a, list, place, n, slots, first, last, rows, S, rank};
+    MoeUpSource<NT, PLACES> src{a, used, slots, first, last, rows, S, rank};
     weight_ring<bf16, NT>(src, tiles, chunks, a.B, wr_smem);
   } else {
-    MoeDownSource src{a, list, place, n, slots, first, last, rows, S, rank};
+    MoeDownSource<NT, PLACES> src{a, used, slots, first, last, rows, S, rank};
     weight_ring<bf16, NT>(src, tiles, chunks, a.B, wr_smem);
   }
 }
 
-template <int NT, bool UP>
+template <int NT, bool UP, bool PLACES>
 static int launch_ring(const MoeDecodeArgs &a, int slots, cudaStream_t st) {
   static DevicePrep prep;
   const int (*resident)[4];
-  const cudaError_t prepared = prep.get([](int (&r)[4]) {
-    const cudaError_t e = ring_residency<NT>(moe_ring_kernel<NT, UP>, r);
-    return e != cudaSuccess ? e
-                            : cudaFuncSetAttribute(moe_ring_kernel<NT, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   WeightRing<NT>::BYTES + 40 * 1024);
-  }, resident);
+  const cudaError_t prepared = prep.get([](int (&r)[4]) { return ring_residency<NT>(moe_ring_kernel<NT, UP, PLACES>, r, MoeTable<NT>::BYTES); },
+                                        resident);
   if (prepared != cudaSuccess) {
     set_error("moe_decode: %s", cudaGetErrorString(prepared));
     return DJV_ERR_CUDA;
@@ -505,16 +551,18 @@ static int launch_ring(const MoeDecodeArgs &a, int slots, cudaStream_t st) {
   const int n = a.E < a.B * a.top ? a.E : a.B * a.top, kf = ceil_div(a.F, WR_K), kf_shared = ceil_div(a.F_shared, WR_K);
   const RingPlan p = UP ? ring_plan(n * a.F + a.F_shared, 2, ceil_div(a.D, WR_K), *resident)
                         : ring_plan(a.D, 1, n * kf + kf_shared, *resident);
-  djv::launch_kernel_cluster(moe_ring_kernel<NT, UP>, dim3(p.clusters * p.S), dim3(WR_THREADS),
-                             WeightRing<NT>::BYTES + (size_t)a.E * (4 + MM_B), st, dim3(p.S), a, slots);
+  djv::launch_kernel_cluster(moe_ring_kernel<NT, UP, PLACES>, dim3(p.clusters * p.S), dim3(WR_THREADS),
+                             (size_t)(WeightRing<NT>::BYTES + MoeTable<NT>::BYTES), st, dim3(p.S), a, slots);
   count_launch();
   return DJV_OK;
 }
 
 template <int NT>
 static int launch_mma(const MoeDecodeArgs &a, int slots, bool up, bool down, cudaStream_t st) {
-  const int rc = up ? launch_ring<NT, true>(a, slots, st) : DJV_OK;
-  return rc || !down ? rc : launch_ring<NT, false>(a, slots, st);
+  const bool places = MoeTable<NT>::has_places(a.E);
+  const int rc = !up ? DJV_OK : places ? launch_ring<NT, true, true>(a, slots, st) : launch_ring<NT, true, false>(a, slots, st);
+  if (rc || !down) return rc;
+  return places ? launch_ring<NT, false, true>(a, slots, st) : launch_ring<NT, false, false>(a, slots, st);
 }
 
 template <typename T>
@@ -526,7 +574,7 @@ static int launch_decode(const MoeDecodeArgs &a, bool up, bool down, cudaStream_
                         aligned16(a.w_down) && aligned16(a.shared_down);
   if constexpr (sizeof(T) == 2) {
     // several rows share weights (both stages take this form or neither: they agree on where a choice's activations are)
-    if (a.B >= 2 && a.B <= MM_B && vec_up && vec_down && (size_t)a.E * (4 + MM_B) <= 40 * 1024) {
+    if (a.B >= 2 && a.B <= MM_B && vec_up && vec_down && a.E <= MM_E) {
       int rc;
       switch ((a.B + 7) / 8) {
         case 1: rc = launch_mma<1>(a, slots, up, down, st); break;

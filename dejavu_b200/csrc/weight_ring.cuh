@@ -211,25 +211,10 @@ inline RingPlan ring_plan(int units, int unit_rows, int chunks, const int (&resi
   return p;
 }
 
-// Prepares `kernel` and asks how many clusters of 1, 2, 4, 8 blocks are resident at once: clusters stay inside a group of
-// multiprocessors, so fewer of the larger ones fit than the multiprocessors have room for.
+// `more`: shared memory behind the ring
 template <int NT, typename... P>
-inline cudaError_t ring_residency(void (*kernel)(P...), int (&resident)[4]) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WeightRing<NT>::BYTES);
-  for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1 << i;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(sm_count() * WR_BPS / 8 * 8);
-    cfg.blockDim = dim3(WR_THREADS);
-    cfg.dynamicSmemBytes = WeightRing<NT>::BYTES;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaOccupancyMaxActiveClusters(&resident[i], kernel, &cfg);
-  }
-  return e;
+inline cudaError_t ring_residency(void (*kernel)(P...), int (&resident)[4], int more = 0) {
+  return cluster_residency(kernel, WR_THREADS, WeightRing<NT>::BYTES + more, WR_BPS, resident);
 }
 
 }  // namespace djv

@@ -106,7 +106,8 @@ def test_short_lists_of_several_tokens(cuda, B, N, M):
 
 
 @pytest.mark.parametrize("B,E,top,D,F,Fs", [(2, 1, 1, 8, 8, 0), (3, 5, 2, 136, 24, 40), (8, 8, 2, 512, 200, 328), (9, 40, 3, 264, 136, 8),
-                                            (17, 4, 4, 1032, 72, 0), (32, 300, 1, 64, 16, 16)])
+                                            (17, 4, 4, 1032, 72, 0), (32, 300, 1, 64, 16, 16), (24, 60, 5, 136, 64, 8),
+                                            (8, 130, 16, 264, 40, 0), (31, 1137, 16, 64, 8, 0), (2, 33, 15, 64, 24, 16)])
 def test_routed_weights_streamed_for_several_rows(cuda, B, E, top, D, F, Fs):
     from dejavu_b200 import ops
 

@@ -87,6 +87,24 @@ def test_kernels_are_prepared_on_every_device(fake, what):
         + "    assert any(n['what'] == 'launch' and n['device'] == device and n['smem'] > 48 * 1024 for n in notes())\n")
 
 
+def test_routed_products_count_on_blocks_that_fit(fake):
+    """The grid is what is resident with the shared memory that is launched, and that is two blocks per multiprocessor."""
+    run(fake, """
+lib = load("libdejavu_b200_routed.so")
+for E in (1, 8, 57, 112, 300, 1137):
+    for top in sorted({1, min(4, E), min(16, E)}):
+        for B in (2, 8, 16, 24, 32):
+            done(lib, lib.djv_moe_decode(1, ptr, ptr, ptr, ptr, ptr, ptr, ptr, None, None, None, B, E, top, 1024, 512, 0, 512, 3, None))
+            for n in notes():
+                if n["what"] == "launch":
+                    assert 2 * (n["smem"] + 1376) <= 228 * 1024 and n["grid"] <= 2 * 148, (E, top, B, n)
+                    asked.setdefault(n["kernel"], n["smem"])
+                else:
+                    asked[n["kernel"]] = n["smem"]
+                assert asked[n["kernel"]] == n["smem"], (E, top, B, n)
+""".replace("lib = load", "asked = {}\nlib = load", 1))
+
+
 def test_short_lists_of_several_rows_fill_no_ring(fake):
     run(fake, """
 lib = load("libdejavu_b200.so")
