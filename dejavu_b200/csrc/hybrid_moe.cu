@@ -325,7 +325,7 @@ constexpr int MM_B = 32, MM_E = 1137;
 // ascending order, a bit for every expert, and an expert's place among a sequence's choices, as a byte for every expert and sequence
 // where there is room for that, else as the sequences' choices, which are looked through. (Bytes for 32 sequences whatever their
 // number left room for one block from 57 experts on with 24 sequences, from 112 on with 8: 64 experts of 704 x 2048, 24 sequences,
-// 165 us so, 100 now; 112 of 512 x 1024, 8 sequences, 52 and 27.)
+// 171 us so, 101 now; 112 of 512 x 1024, 8 sequences, 52 and 26.)
 template <int NT>
 struct MoeTable {
   static constexpr int SEQS = NT * 8, BITS = (MM_E + 31) / 32 * 4, LIST = SEQS * MAX_TOP * 2, CHOICES = SEQS * MAX_TOP * 2;

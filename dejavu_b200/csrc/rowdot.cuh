@@ -34,10 +34,11 @@ __device__ __forceinline__ float apply_act_param(float v, float p) {
 // with U chunks in flight per lane per row. x is read through L1 (it is tiny and reused by every group); weights bypass L1.
 //
 // The grid is all blocks that are resident at once. Handing out rows in rounds instead (a grid of up to 6 blocks per
-// multiprocessor of which 4 fit) left a part of the blocks without work in the last round: bf16, 1 row of x, us before /
-// now: 12352 x 4096 23.6 / 16.9 (0.92 of the copy rate), 6144 x 4096 12.3 / 9.7, 22016 x 4096 gated 34.0 / 29.4,
-// 50272 x 4096 67.7 / 60.2, 11264 x 2048 gated 10.8 / 9.0; fp16 gathered, 4096 x 12288 19.1 / 18.5. Short lists are bound by
-// the chain launch, x and first weights, sums, store: 4096 x 4096 7.3 / 6.9, 2048 x 2048 2.8 either way.
+// multiprocessor of which 4 fit) left a part of the blocks without work in the last round: us before / now, bf16, 1 row of x:
+// 12352 x 4096 23.2 / 16.3 (0.95 of the copy rate), 6144 x 4096 12.2 / 9.3, 22016 x 4096 gated 32.9 / 29.1, 50272 x 4096 66.0 / 58.3,
+// 11264 x 2048 gated 8.9 / 9.1; 2 rows: 22016 x 4096 34.5 / 29.9, 4096 x 4096 8.3 / 8.1; fp16 gathered: 4096 x 12288 18.5 / 17.4 and
+// with 2 rows 19.2 / 18.8. (Runs of different days differ by up to 5 %.) Short lists are bound by the chain launch, row numbers, x
+// and first weights, sums, store: 2048 x 2048 2.8 / 2.9; gathered 384 x 768 2.5 / 2.7, 512 x 12288 with 2 rows 5.6 / 5.4.
 // -------------------------------------------------------------------------------------------
 constexpr int RD_THREADS = 256;
 constexpr int RD_WARPS = RD_THREADS / WARP;

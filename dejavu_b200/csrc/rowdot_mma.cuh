@@ -238,11 +238,13 @@ inline int rowdot_mma_short_split(int M, int N, int NT, int bps) {
   return S;
 }
 
-// Which form. us, short / ring, fp16 gathered with bias (bf16 with fp32 result in brackets where it differs), M x N:
-//   9 rows of x and more (16): 512 x 512 2.5 / 3.5, 1024 x 1024 4.1 / 5.2, 4096 x 1024 0.87 of the ring's, 6144 x 1024 1.37;
-//     2048 x 2048 0.81, 1024 x 4096 0.82, 512 x 12288 0.87; but 512 x 2048 1.04, 3072 x 2048 1.00 (1.06), 1024 x 12288 1.03.
-//   up to 8 rows (8): 256 x 1024 0.76, 2048 x 512 0.89, but 512 x 1024 1.02, 2048 x 1024 1.07, 1024 x 2048 1.15. And tiles that
-//     fill the resident blocks once, of short rows: 11264 x 2048 0.83 (0.96), 11264 x 768 0.73 (0.92); 8192 x 2048 1.19.
+// Which form. us, short / ring, bf16 with fp32 result, fp16 gathered with bias:
+//   16 rows of x: 512 x 512 2.0 / 2.6, 2.5 / 3.6; 1024 x 1024 3.6 / 4.9, 4.3 / 5.4; 4096 x 1024 4.2 / 4.5, 4.9 / 5.6; 2048 x 2048
+//     5.3 / 6.2, 6.1 / 7.6; 1024 x 4096 5.2 / 5.7, 6.0 / 7.4; 512 x 12288 6.5 / 7.4, 7.2 / 8.3. But 6144 x 1024 6.7 / 4.6, 8.3 / 6.1;
+//     512 x 2048 4.6 / 4.5, 5.4 / 5.2; 3072 x 2048 6.1 / 5.8, 6.9 / 6.9; 1024 x 12288 9.6 / 8.2, 10.5 / 10.2.
+//   8 rows: 256 x 1024 2.8 / 3.4, 3.1 / 4.1; 2048 x 512 2.8 / 3.1, 3.4 / 3.8; but 512 x 1024 4.2 / 3.9, 4.7 / 4.6; 2048 x 1024
+//     4.6 / 4.4, 5.4 / 5.0; 1024 x 2048 5.6 / 4.5, 6.5 / 5.6. And short rows whose tiles fill the resident blocks once: 11264 x 2048
+//     10.4 / 10.9, 11.1 / 13.3; 11264 x 768 5.4 / 5.9, 5.9 / 8.0; but 8192 x 2048 9.4 / 6.6, 10.1 / 8.5.
 inline bool rowdot_mma_is_short(int M, int N, int NT, int blocks) {
   if (NT > 1) return N <= 1024 ? M <= 4096 : N <= 4096 ? M > 512 && M <= 2048 : M <= 512;
   const int tiles = ceil_div(M, MS_ROWS);

@@ -7,7 +7,8 @@
 // are not copied: what is in their place meets no other row's sums, and copies of nothing took as long as copies (22016 x
 // 4096, 8 rows of x: 36 us with them, 29.5 without). The ring runs on from one tile to the next, so the sums of a tile are
 // added up (over the 4 warps that split a chunk's columns, then over the cluster through distributed shared memory, in rank
-// order) while the next tile's weights are on their way. Two blocks per multiprocessor, about 64 KB of weights each in flight.
+// order) while the next tile's weights are on their way. Two blocks per multiprocessor, each with 72, 48, 40 or 24 KB of weights in
+// flight for up to 8, 16, 24 and 32 rows of x: activations and sums take the rest.
 //
 // The tensor cores' sums are short: 16 columns with up to 8 rows of x, 32 with more, join the others in fp32 (add_sums). Kept in
 // the MMAs' accumulators from end to end of a row they were off by 1.0e-6 of the result at 4096 columns and 2.9e-6 at 11008;
@@ -17,8 +18,8 @@
 //
 // Bound by HBM from about 20 MB of weights on: bf16, 8 rows of x, us before (a block of 8 warps per 16 rows, fed straight
 // from registers) / now, of which the weights at copy rate: 6144 x 4096 15.1 / 10.3 (7.7), 12352 x 4096 28.9 / 18.6 (15.5),
-// 22016 x 4096 35.3 / 29.5 (27.7), 50272 x 4096 77.7 / 65.7 (63.2); 16 rows, 4096 gathered rows of 12288 24.5 / 20.4 (15.5).
-// Short lists cost a chain of latencies: 384 gathered rows of 768 3.4 / 4.2.
+// 22016 x 4096 34.6 / 29.3 (27.7), 50272 x 2048 41.3 / 33.6 (31.6); 16 rows, 4096 gathered rows of 12288 24.4 / 20.3 (15.5).
+// Short lists are over before a ring has been worth filling: those of the products take another form (rowdot_mma.cuh).
 //
 // What the weights are, which x meets them and where results go is the Source's business:
 //   seek(t, c)            the copies that follow are those of chunk c (of this block) of tile t; called in order

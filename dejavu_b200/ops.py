@@ -173,7 +173,7 @@ def dense_transposed_gemv(x: torch.Tensor, weight_t: torch.Tensor, bias: Optiona
 
 
 def _mlp_sparse_call(x, W1, W2t, idx, bias1, bias2):
-    """Both products of mlp_sparse behind one call into the library, one workspace for the hidden values and the result."""
+    """Both products of mlp_sparse behind one call into the library."""
     batch, N = x.shape
     M = idx.shape[0]
     lib = _lib.load()
