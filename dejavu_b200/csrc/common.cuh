@@ -144,6 +144,11 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
+// The same for `bytes` from p on, both multiples of 16: one instruction, whatever the size.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // 16-byte read-only load that does not pollute L1 (weights are streamed exactly once).
 __device__ __forceinline__ uint4 ld_stream16(const void *p) {
   uint4 v;

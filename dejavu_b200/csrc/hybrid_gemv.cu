@@ -37,7 +37,7 @@ static void launch_rowdot_dense(TO *Y, const T *W, const T *X, int M, int N, lon
   const RowdotPlan p = plan_rowdot(M, N / Chunk<T>::N, is_glu(ACT) ? 2 : 1, B);
 #define DJV_RD(WPR_, R_, U_, BL_, SP_)                                                                                            \
   djv::launch_kernel(rowdot_kernel<T, TO, B, ACT, WPR_, R_, U_, BL_, SP_>, p.grid, RD_THREADS, 0, st, Y, W, X,                     \
-                     static_cast<const void *>(nullptr), static_cast<const T *>(nullptr), M, N, ldw, 0, 1, param, \
+                     static_cast<const void *>(nullptr), static_cast<const T *>(nullptr), M, N, ldw, 0, p.ahead, param, \
                      p.per_block, p.rest)
   DJV_ROWDOT(p, B, DJV_RD);
 #undef DJV_RD

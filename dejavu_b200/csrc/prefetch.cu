@@ -11,10 +11,6 @@ namespace djv {
 constexpr int PF_THREADS = 256;
 constexpr unsigned PF_PIECE = 8192;  // bytes per bulk prefetch
 
-__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // rows idx[0..M) of up to 3 matrices that share the index list; a row is row_bytes contiguous bytes (a multiple
 // of 16) at base + idx * ld_bytes
 __global__ void __launch_bounds__(PF_THREADS)

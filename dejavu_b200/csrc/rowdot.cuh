@@ -45,6 +45,18 @@ constexpr int RD_WARPS = RD_THREADS / WARP;
 constexpr int RD_SPAN = 128;  // rows whose sums a block keeps before it finishes them
 constexpr int RD_FEW = 8;     // as many as a block with 4 chunks per row can have
 
+// What a block asks for before it waits for the kernel before it. Dense steps of one user are a chain of products and small kernels
+// between them, under which HBM would be idle: RD_AHEAD bytes per block, twice as many where that is an eighth of its rows, by bulk
+// prefetches (one thread an 8 KB piece). A decode step of 6 layers, 4096 wide, one / two rows of x, us: nothing 562.6 / 620.6, 16 rows
+// of 8 KB line by line 568.4 / 624.3, 8 KB in bulk 554.1 / 615.6, 16 KB 547.3 / 607.3, 32 KB 542.1 / 596.3; 12 layers, 2048 wide 472.3,
+// 464.9, 458.7, 451.7, 460.6; with routed experts, 2048 wide 568.1, 576.5, 564.5, 563.6, 569.9, 4096 wide 640.0, 646.0, 630.8, 629.9,
+// 636.2; this rule 543.6 / 597.2, 455.4, 566.1, 626.2. Lines are an instruction each, and with more bytes the loads of the kernel
+// before queue up behind them. In the sparse steps, whose side streams fill the gaps, neither form gains (8034 / 8019 us for 16
+// steps of 8 layers, 4096 wide, 13488 / 13365 of 4 layers, 9216 wide): those keep the lines.
+constexpr int RD_PIECE = 8192;
+constexpr int RD_AHEAD = 16384;
+constexpr int RD_AHEAD_LINES = -1;  // 8 KB of each of 16 rows, line by line, gathered ones included
+
 // Blocks per multiprocessor that the registers of a pass leave room for: ROWS * U 16-byte loads, ROWS * B sums.
 __host__ __device__ constexpr int rd_blocks(int B) { return B == 1 ? 4 : B == 2 ? 3 : B <= 4 ? 2 : 1; }
 
@@ -52,7 +64,7 @@ template <typename T, typename TO, int B, int ACT, int WPR, int ROWS, int U, int
 __global__ void __launch_bounds__(RD_THREADS, BLOCKS)
 rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__ X,
               const void *__restrict__ idx, const T *__restrict__ bias, int M, int N,
-              long long ldw, int idx64, int early, float act_param, int per_block, int rest) {
+              long long ldw, int idx64, int ahead, float act_param, int per_block, int rest) {
   constexpr int UNIT = is_glu(ACT) ? 2 : 1;  // rows 2i, 2i + 1 of the matrix are the gate and up rows of output i
   constexpr int GROUPS = RD_WARPS / WPR;
   constexpr int GLANES = WARP * WPR;
@@ -70,10 +82,16 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   const int last = first + (per_block + (bx < rest ? 1 : 0)) * UNIT;
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (early) {
-    // Weights are not produced by any kernel, and the index list is complete (identity, or the caller's promise): the
-    // first 8 KB of the block's rows are requested while the kernel before this one is still running. A prefetch can
-    // neither fault nor return a stale value, whatever the promise is worth.
+  if (ahead > 0) {
+    // Weights are not produced by any kernel of a step, and a prefetch could not return a stale value anyway.
+    const int row_bytes = nchunks * 16, pieces = (row_bytes + RD_PIECE - 1) / RD_PIECE;
+    const int total = (int)min((long long)(last - first) * pieces, max(1ll, (long long)ahead * pieces / row_bytes));
+    for (int p = tid; p < total; p += RD_THREADS) {
+      const int off = p % pieces * RD_PIECE;
+      bulk_prefetch_l2(reinterpret_cast<const char *>(W + (first + p / pieces) * ldw) + off, min(RD_PIECE, row_bytes - off));
+    }
+  } else if (ahead == RD_AHEAD_LINES) {
+    // The index list is complete (identity, or the caller's promise).
     constexpr int LINES = 64, MAX_ROWS = 16;
     const int row_lines = (int)min((long long)LINES, ((long long)N * (int)sizeof(T) + 127) / 128);
     for (int m = first + warp; m < min(last, first + MAX_ROWS); m += RD_WARPS) {
@@ -164,7 +182,7 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
 enum RowdotForm { RD_FOUR_ROWS, RD_FEW_ROWS, RD_FOUR_BLOCKS };
 
 struct RowdotPlan {
-  int wpr, grid, per_block, rest;
+  int wpr, grid, per_block, rest, ahead;
   RowdotForm form;
 };
 
@@ -210,6 +228,7 @@ inline RowdotPlan plan_rowdot(int M, int nchunks, int unit, int B) {
   r.grid = max(1, min(slots, r.form == RD_FEW_ROWS ? ceil_div(M, q) : units));
   r.per_block = units / r.grid;
   r.rest = units % r.grid;
+  r.ahead = (int)max((long long)RD_AHEAD, min(2ll * RD_AHEAD, (long long)r.per_block * unit * nchunks * 16 / 8));
   return r;
 }
 
