@@ -232,8 +232,7 @@ class GPTLMHeadModel(nn.Module, GenerationMixin):
     selects_logit_rows = True  # forward(logit_rows=...) computes logits at those tokens only
 
     def forward(self, input_ids, position_ids=None, inference_params=None, logit_rows=None):
-        # A decode step of several sequences runs kernels of several waves of blocks: programmatic dependent launch
-        # then costs more than it hides (see djv_set_programmatic_launch), so the step's kernels are launched plain.
+        # the decode step of several sequences can be launched plain (development knob; see djv_set_programmatic_launch)
         plain = (input_ids.is_cuda and input_ids.size(0) > 1 and input_ids.size(1) == 1
                  and not modules.BATCH_PROGRAMMATIC_LAUNCH)
         if plain:

@@ -61,9 +61,10 @@ L2_PREFETCH_MB = float(os.environ.get("DJV_L2_PREFETCH_MB", "100"))
 # batch > 1: the predictors run once, on the sum of the sequences' inputs (they are linear), instead of once per
 # sequence; "0": per sequence, logits added afterwards (development knob)
 SP_SUM_INPUTS = os.environ.get("DJV_SP_SUM_INPUTS", "1") != "0"
-# batch > 1: keep programmatic dependent launch for the decode step's kernels ("1"); default off, measured slower
-# (OPT-6.7B, 16 sequences: 6.3 ms per step with, 4.7 without; 4 sequences: 2.95 / 2.64) (development knob)
-BATCH_PROGRAMMATIC_LAUNCH = os.environ.get("DJV_BATCH_PDL", "0") != "0"
+# batch > 1: programmatic dependent launch for the decode step's kernels; "0": launched plain. us per step without / with it, 4
+# layers of 4096: 2 sequences 410 / 394, 4 412 / 390, 16 509 / 473; 6 layers of 2048: 2 sequences 321 / 295, 16 421 / 357. (It was slower
+# when kernels of several waves of blocks, and kernels of other libraries, stood in the chain.) (development knob)
+BATCH_PROGRAMMATIC_LAUNCH = os.environ.get("DJV_BATCH_PDL", "1") != "0"
 # batch > 1: the attention of all sequences runs through the batch entry points (one state, one launch per kernel
 # for the whole batch); "0": sequence by sequence through the batch-1 kernels (development knob)
 BATCHED_ATTENTION = os.environ.get("DJV_BATCHED_ATTENTION", "1") != "0"

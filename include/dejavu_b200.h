@@ -74,12 +74,11 @@ void djv_set_early_weight_prefetch(int enabled);
 /* Per calling thread, default 1. Every kernel of the library is launched with programmatic dependent launch and
  * lets its successor start (and wait) as soon as all its own blocks have started: the successor's launch latency
  * and prologue overlap the kernel's tail. That pays when kernels are short and fit the device in one wave (decode
- * with one sequence: OPT-66B 7.18 ms per token with it, 7.4 without). In decode steps of several sequences it was
- * measured to cost far more than it hides (OPT-6.7B, ms per step with / without: 2 sequences 4.58 / 2.37, 16
- * sequences 6.3 / 4.7). The step timeline shows why: successors launched early sit on the multiprocessors waiting,
- * and a kernel of another stream that they depend on through an event (in the batched step: the host framework's
- * own reduction kernels of the look-ahead predictor) finds no free slot for some 200 us per layer. 0 launches the
- * kernels of this thread as plain stream-ordered kernels. Never changes a result. */
+ * with one sequence: OPT-66B 7.18 ms per token with it, 7.4 without; of several sequences: OPT-6.7B width, 4 layers, us
+ * per step without / with it: 2 sequences 410 / 394, 16 sequences 509 / 473). Successors launched early sit on the
+ * multiprocessors waiting: where kernels of another stream that they depend on find no free slot, or kernels run in
+ * several waves of blocks, it can cost more than it hides. 0 launches the kernels of this thread as plain
+ * stream-ordered kernels. Never changes a result. */
 void djv_set_programmatic_launch(int enabled);
 
 /* ---------------------------------------------------------------------------------------------
