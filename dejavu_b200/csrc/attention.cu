@@ -86,8 +86,8 @@ struct QkvArgs {
   int *state;
   __half *q_out, *k_cache, *v_cache;
   int S;
-  // MODE 1 when the step was opened without the stash of x (djv_topk_attn_prep): the current token row is read
-  // from x_cur, and block 0 copies it into the window for later back-fills. Null otherwise.
+  // When the step was opened without the stash of x (djv_topk_attn_prep): the current token row (of MODE 2: (nseq, d) rows) is
+  // read from x_cur, and block 0 copies it into the window for later back-fills. Null otherwise.
   const __half *x_cur;
   __half *x_ring_w;
   int early;  // MODE 1: the state is complete before this kernel can start; prefetch weights before the wait
@@ -170,7 +170,8 @@ __device__ __forceinline__ void qkv_mma_rows(const QkvArgs &a, int qkv, int h, i
       const int code = rows_s[j * 8 + g];
       const int r = (MODE == 2) ? row_slot(code) : code;
       const __half *xs = (MODE == 2) ? a.x + (size_t)row_seq(code) * a.seq_x : a.x;
-      xr[j] = (MODE >= 1 && a.x_cur != nullptr && r == cur_slot) ? a.x_cur : xs + (size_t)r * a.d;
+      const __half *now = (MODE == 2) ? a.x_cur + (size_t)row_seq(code) * a.d : a.x_cur;
+      xr[j] = (MODE >= 1 && a.x_cur != nullptr && r == cur_slot) ? now : xs + (size_t)r * a.d;
     }
   }
 
@@ -285,9 +286,12 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
     base = a.state[ST_BASE];
     if (a.x_cur != nullptr && blockIdx.x == 0 && a.state[ST_STATUS] == 0) {
       // nobody reads window row `slot` in this kernel: the current token is taken from x_cur
-      const uint4 *src = reinterpret_cast<const uint4 *>(a.x_cur);
-      uint4 *dst = reinterpret_cast<uint4 *>(a.x_ring_w + (size_t)slot * a.d);
-      for (int c = threadIdx.x; c < a.d / 8; c += QKV_THREADS) dst[c] = src[c];
+      const int seq0 = MODE == 2 ? blockIdx.y * QKV_SEQ_GROUP : 0, seq1 = MODE == 2 ? min(a.nseq, seq0 + QKV_SEQ_GROUP) : 1;
+      for (int sq = seq0; sq < seq1; ++sq) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.x_cur + (size_t)sq * a.d);
+        uint4 *dst = reinterpret_cast<uint4 *>(a.x_ring_w + (size_t)sq * a.seq_x + (size_t)slot * a.d);
+        for (int c = threadIdx.x; c < a.d / 8; c += QKV_THREADS) dst[c] = src[c];
+      }
     }
   }
   if (i >= n_eff) return;
@@ -352,8 +356,8 @@ __global__ void __launch_bounds__(QKV_THREADS, 2) qkv_sparse_kernel(QkvArgs a) {
       const int code = rows_s[r0 + (r < nb ? r : 0)];
       const int tr = (MODE == 2) ? row_slot(code) : code;
       const uint4 *xs = (MODE == 2) ? Xv + (size_t)row_seq(code) * (a.seq_x / 8) : Xv;
-      xp[r] = (MODE >= 1 && a.x_cur != nullptr && tr == slot) ? reinterpret_cast<const uint4 *>(a.x_cur)
-                                                              : xs + (size_t)tr * nchunks;
+      const uint4 *now = reinterpret_cast<const uint4 *>(a.x_cur) + (MODE == 2 ? (size_t)row_seq(code) * nchunks : 0);
+      xp[r] = (MODE >= 1 && a.x_cur != nullptr && tr == slot) ? now : xs + (size_t)tr * nchunks;
     }
     if (nb == 1) {
       const uint4 *x1[1] = {xp[0]};
@@ -960,7 +964,6 @@ static int attn_step_project(void *q_out, const void *wqkv, const void *bqkv, co
   DJV_REQUIRE(S >= 1, "attn_step: cache capacity S=%d", S);
   DJV_REQUIRE(aligned16(wqkv) && aligned16(x) && aligned16(x_ring) && aligned16(k_cache) && aligned16(v_cache),
               "attn_step: pointers must be 16-byte aligned");
-  DJV_REQUIRE(B == 1 || !step_is_open, "attn_step: a batch opens its step itself");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const long long seq_ring = (long long)DJV_KV_WINDOW * d;
   const int typical = head_idx ? (nnz > 0 ? nnz : 1) : nheads;
@@ -1022,6 +1025,14 @@ extern "C" int djv_attn_step_project_batch(void *q_out, const void *wqkv, const 
                                            int B, void *stream) {
   return attn_step_project(q_out, wqkv, bqkv, x, x_ring, k_cache, v_cache, state, head_idx, nnz, d, nheads, hd, S, B,
                            0, stream);
+}
+
+extern "C" int djv_attn_step_project_batch_opened(void *q_out, const void *wqkv, const void *bqkv, const void *x,
+                                                  void *x_ring, void *k_cache, void *v_cache, int32_t *state,
+                                                  const int32_t *head_idx, int nnz, int d, int nheads, int hd, int S,
+                                                  int B, void *stream) {
+  return attn_step_project(q_out, wqkv, bqkv, x, x_ring, k_cache, v_cache, state, head_idx, nnz, d, nheads, hd, S, B,
+                           1, stream);
 }
 
 static int attn_step_attend(void *ctx, const void *q, const void *k_cache, const void *v_cache, int32_t *state,

@@ -570,7 +570,7 @@ class ParallelMHASparseAttMlp(nn.Module):
             assert k_cache.is_contiguous() and v_cache.is_contiguous()
             bb = self._batch_buffers(x.device, S, B)
             state = bb["state"]
-            call("djv_attn_step_project_batch", bb["q"].data_ptr(), self.Wqkv.weight.data_ptr(),
+            call("djv_attn_step_project_batch_opened" if step_is_open else "djv_attn_step_project_batch", bb["q"].data_ptr(), self.Wqkv.weight.data_ptr(),
                  None if bias is None else bias.data_ptr(), xf.data_ptr(), bb["x_ring"].data_ptr(),
                  k_cache.data_ptr(), v_cache.data_ptr(), state.data_ptr(),
                  None if head_idx is None else head_idx.data_ptr(), nnz, d, n, hd, S, B, ops._stream())
@@ -673,11 +673,11 @@ class ParallelMHASparseAttMlp(nn.Module):
                 nxt = self.next_mixer if (decoding and FUSE_STEP_OPEN) else None
                 with _side(x, "att", after=residual) as done:
                     scores = self.sp(residual)
-                    if nxt is not None and nxt.sparse_attention and scores.dim() == 1 and x.size(0) == 1:
-                        # the selection is for the next layer's attention: open its decode step in the same
-                        # kernel, so that layer starts with its QKV projection
+                    if nxt is not None and nxt.sparse_attention and scores.dim() == 1 and (x.size(0) == 1 or BATCHED_ATTENTION):
+                        # the selection is for the next layer's attention: open its decode step (of a batch: the one
+                        # that its sequences share) in the same kernel, so that layer starts with its QKV projection
                         S_next = inference_params.key_value_memory_dict[nxt.layer_idx][1].shape[2]
-                        state = nxt._decode_buffers(x.device, S_next)[0]["state"]
+                        state = nxt._decode_buffers(x.device, S_next, x.size(0))[0]["state"]
                         idx = ops.topk_indices_open_step(scores, self.att_k, state, S_next)
                         idx._step_opened_for = nxt
                     else:

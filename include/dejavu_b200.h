@@ -296,6 +296,12 @@ int djv_attn_step_project(void *q_out, const void *wqkv, const void *bqkv, const
 int djv_attn_step_project_batch(void *q_out, const void *wqkv, const void *bqkv, const void *x, void *x_ring,
                                 void *k_cache, void *v_cache, int32_t *state, const int32_t *head_idx, int nnz,
                                 int d, int nheads, int hd, int S, int B, void *stream);
+/* The same behind a djv_topk_attn_prep on `state` (head_idx, nnz: the list that it made, for the shape of the launch): no
+ * opening launch; the projection puts the tokens x (B,d) into their windows. */
+int djv_attn_step_project_batch_opened(void *q_out, const void *wqkv, const void *bqkv, const void *x,
+                                       void *x_ring, void *k_cache, void *v_cache, int32_t *state,
+                                       const int32_t *head_idx, int nnz, int d, int nheads, int hd, int S, int B,
+                                       void *stream);
 int djv_attn_step_attend_batch(void *ctx, const void *q, const void *k_cache, const void *v_cache, int32_t *state,
                                int B, int nheads, int hd, int S, float softmax_scale, void *scratch,
                                size_t scratch_bytes, void *stream);

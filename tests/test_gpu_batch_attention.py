@@ -53,6 +53,31 @@ def test_lazy_projection_of_a_batch(cuda, B, nheads, hd, d):
     assert state[3].item() == 0
 
 
+# qkv_sparse_kernel (two and three sequences, one row per block where d or hd leave few) and qkv_batch_kernel
+@pytest.mark.parametrize("B,nheads,hd,d,nnz", [(2, 30, 32, 72, 12), (3, 32, 128, 4096, 12), (9, 40, 128, 264, 33), (2, 4, 64, 136, 1), (17, 3, 32, 72, 3)])
+def test_step_opened_by_the_selection_of_heads(cuda, B, nheads, hd, d, nnz):
+    """The selection opens the step and the projection stashes the tokens: the same bits as with a launch that does both first."""
+    from dejavu_b200 import _lib, ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + d)
+    S, f16 = 40, {"dtype": torch.float16, "device": cuda}
+    w, bias = (torch.randn(3, nheads, hd, d, device=cuda, generator=g) * d ** -0.5).half(), torch.randn(3, nheads, hd, generator=g, **f16)
+    sides = [(torch.zeros(B, nheads, hd, **f16), torch.zeros(B, 16, d, **f16), torch.zeros(B, nheads, hd // 8, S, 8, **f16),
+              torch.zeros(B, nheads, S, hd, **f16), torch.zeros(_lib.ATTN_STATE_HDR + 3 * nheads, dtype=torch.int32, device=cuda)) for _ in range(2)]
+    for side in sides:
+        _lib.call("djv_attn_state_reset", side[4].data_ptr(), nheads, 3, ops._stream())
+    for t in range(35):
+        x = torch.randn(B, d, device=cuda, generator=g).half()
+        scores = torch.randn(nheads, device=cuda, generator=g).half()
+        lists = ops.topk_indices(scores, nnz, torch.int32), ops.topk_indices_open_step(scores, nnz, sides[1][4], S)
+        for (q, ring, k, v, state), heads, entry in zip(sides, lists, ("", "_opened")):
+            _lib.call("djv_attn_step_project_batch" + entry, q.data_ptr(), w.data_ptr(), bias.data_ptr(), x.data_ptr(), ring.data_ptr(),
+                      k.data_ptr(), v.data_ptr(), state.data_ptr(), heads.data_ptr(), nnz, d, nheads, hd, S, B, ops._stream())
+        for a, b in zip(*sides):
+            assert torch.equal(a, b), t
+        assert torch.equal(sides[1][1][:, t % 16], x)
+
+
 @pytest.mark.parametrize("B", [4, 5, 8, 9, 15, 16])
 @pytest.mark.parametrize("nheads,hd,d,nnz", [(4, 32, 128, 4), (7, 64, 384, 5), (32, 128, 4096, 12), (40, 128, 256, 33), (6, 32, 128, 0)])
 def test_output_projection_of_a_batch(cuda, B, nheads, hd, d, nnz):
