@@ -91,6 +91,20 @@ def test_output_projection_of_a_batch(cuda, B, nheads, hd, d, nnz):
     near(ops.out_proj_sparse(x, w, heads.int(), bias), want)
 
 
+# splits given up for blocks that fit at once: one pass and several per block, parts without tokens
+@pytest.mark.parametrize("B,nheads,hd,S,length", [(16, 32, 64, 300, 290), (4, 40, 128, 700, 513), (300, 4, 32, 200, 199), (3, 32, 128, 1100, 1), (1, 72, 128, 2100, 2099)])
+def test_attention_of_a_batch(cuda, B, nheads, hd, S, length):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B + S)
+    q, k, v = (torch.randn(B, nheads, n, hd, device=cuda, generator=g).half() for n in (1, S, S))
+    got = ops.decode_attention(q[:, :, 0], k.view(B, nheads, S, hd // 8, 8).transpose(2, 3).contiguous(), v, None, length, hd ** -0.5)
+    p = (q.double() @ k[:, :, :length].double().transpose(2, 3) * hd ** -0.5).softmax(-1)
+    # weights by __expf of fp32 scores: 2^-21 each beside the rounding of the result
+    err = (got.double() - (p @ v[:, :, :length].double())[:, :, 0]).abs().max().item()
+    assert err <= 2 ** -11 * 4 + 1e-5, err
+
+
 # An error of e of a result's size takes about e / 2^-12 of the results across the edge between two fp16 values. fp32 sums are off
 # by 1e-7 to 2e-7 here; sums left in the tensor cores' accumulators by 2e-6 (the projection) and 8e-7 (the output projection).
 def crossed(got, want):
