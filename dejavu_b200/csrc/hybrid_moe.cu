@@ -8,6 +8,7 @@
 
 #include "../../include/dejavu_b200_routed.h"
 #include "hybrid_moe.cuh"
+#include "rowdot.cuh"
 #include "weight_ring.cuh"
 
 namespace djv {
@@ -565,6 +566,219 @@ static int launch_mma(const MoeDecodeArgs &a, int slots, bool up, bool down, cud
   return places ? launch_ring<NT, false, true>(a, slots, st) : launch_ring<NT, false, false>(a, slots, st);
 }
 
+// ---- decode, one row --------------------------------------------------------------------------------------------------
+// The chosen experts' rows and the shared one's are dealt out evenly over the resident blocks, as the dense products' are
+// (rowdot.cuh): a block per 8 outputs and expert, and 8 rows of the result per block, left a last round nearly empty, and a lane walked
+// the experts one after another. Every block has a part of the shared expert, which it begins with: its rows are known while
+// the router is still running, and are asked for ahead. Bound by HBM from about 50 MB on, below by the chain router scores, choices,
+// weights, sums. A decode step, us before / now: 12 layers 2048 wide, 8 experts of 1856 and a shared one 566 / 540 (up 10.3 / 9.5
+// of 7.0 at copy rate, down 9.5 / 5.8 of 3.5), 6 layers 4096 wide, experts of 3648 626 / 597.
+constexpr int M1_SPAN = 64;  // outputs whose sums a block keeps before it finishes them
+
+template <typename T, int WPR>
+__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_up_kernel(MoeDecodeArgs a, int slots) {
+  constexpr int GROUPS = MO_WARPS / WPR, GLANES = WARP * WPR, U = 2, AT_ONCE = GROUPS * 2;
+  static_assert(M1_SPAN % AT_ONCE == 0, "");
+  __shared__ float red[M1_SPAN][2][WPR], weight_s[M1_SPAN];
+  __shared__ T *out_s[M1_SPAN];
+  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, group = warp / WPR, wig = warp % WPR, glane = wig * WARP + lane;
+  const int nch = a.D / Chunk<T>::N, grid = gridDim.x, bx = blockIdx.x;
+  auto part = [&](int n, int at, int &first, int &count) {  // of n outputs
+    const int per = n / grid, rest = n % grid;
+    first = at * per + min(at, rest);
+    count = per + (at < rest ? 1 : 0);
+  };
+  int fs, ns, fe, ne;
+  part(a.F_shared, bx, fs, ns);
+  part(a.top * a.F, grid - 1 - bx, fe, ne);  // (those with one more are others than above)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int row_bytes = nch * 16, rows_ahead = min(2 * ns, max(1, RD_AHEAD / row_bytes));
+  for (int r = tid; r < rows_ahead; r += MO_THREADS)
+    for (int off = 0; off < row_bytes; off += RD_PIECE)
+      bulk_prefetch_l2(reinterpret_cast<const char *>(static_cast<const T *>(a.shared_gu) + ((size_t)2 * fs + r) * a.D) + off,
+                       min(RD_PIECE, row_bytes - off));
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int e_l = 0;  // of place `lane`: the expert, and its score
+  float v_l = 0.f;
+  bool known = false;
+  if (bx == 0 && warp == 0) {
+    warp_topk(a.z, a.E, a.top, e_l, v_l);
+    known = true;
+    if (lane < a.top) a.chosen[lane] = e_l;
+  }
+  const uint4 *xv = static_cast<const uint4 *>(a.x);
+  const int n = ns + ne;
+  for (int s0 = 0; s0 < n; s0 += M1_SPAN) {
+    const int s1 = min(n, s0 + M1_SPAN);
+    for (int i0 = s0 + group * 2; i0 < s1; i0 += AT_ONCE) {
+      const uint4 *wp[2] = {nullptr, nullptr};  // gate row; the up row is behind it
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = i0 + q;
+        if (i >= s1) continue;
+        const T *w;
+        T *out = static_cast<T *>(a.act);
+        float wt = 1.f;
+        if (i < ns) {
+          w = static_cast<const T *>(a.shared_gu) + (size_t)2 * (fs + i) * a.D;
+          out += (size_t)a.top * a.ld_act + fs + i;
+        } else {
+          if (!known) {
+            warp_topk(a.z, a.E, a.top, e_l, v_l);
+            known = true;
+          }
+          const int u = fe + i - ns, s = u / a.F, o = u - s * a.F;
+          wt = sigmoid_f(__shfl_sync(0xffffffffu, v_l, s));
+          w = static_cast<const T *>(a.w_gu) + ((size_t)__shfl_sync(0xffffffffu, e_l, s) * a.F + o) * 2 * a.D;
+          out += (size_t)s * a.ld_act + o;
+        }
+        wp[q] = reinterpret_cast<const uint4 *>(w);
+        if (wig == 0 && lane == 0) {
+          weight_s[i - s0] = wt;
+          out_s[i - s0] = out;
+        }
+      }
+      float acc[4] = {};
+      for (int c0 = glane; c0 < nch; c0 += GLANES * U) {
+        uint4 v[4][U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + u * GLANES;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            v[r][u] = c < nch && wp[r / 2] != nullptr ? ld_stream16(wp[r / 2] + (r % 2) * nch + c) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + u * GLANES;
+          if (c < nch) {
+            const uint4 x = ld_cached16(xv + c);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[r] = dot_chunk<T>(v[r][u], x, acc[r]);
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float t = warp_sum(acc[r]);
+        if (lane == 0 && i0 + r / 2 < s1) red[i0 + r / 2 - s0][r % 2][wig] = t;
+      }
+    }
+    __syncthreads();
+    if (tid < s1 - s0) {
+      float g = 0.f, u = 0.f;
+#pragma unroll
+      for (int k = 0; k < WPR; ++k) {
+        g += red[tid][0][k];
+        u += red[tid][1][k];
+      }
+      *out_s[tid] = from_f<T>(silu_glu(weight_s[tid] * g, weight_s[tid] * u));
+    }
+    if (s1 < n) __syncthreads();
+  }
+}
+
+template <typename T, int WPR>
+__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_down_kernel(MoeDecodeArgs a, int slots) {
+  constexpr int GROUPS = MO_WARPS / WPR, GLANES = WARP * WPR, U = 2, AT_ONCE = GROUPS * 4, N = Chunk<T>::N;
+  static_assert(M1_SPAN % AT_ONCE == 0, "");
+  __shared__ float red[M1_SPAN][WPR];
+  __shared__ const T *base_s[MAX_TOP];  // row 0 of a choice's weights
+  const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, group = warp / WPR, wig = warp % WPR, glane = wig * WARP + lane;
+  const int grid = gridDim.x, bx = blockIdx.x, per = a.D / grid, rest = a.D % grid;
+  const int first = bx * per + min(bx, rest), last = first + per + (bx < rest ? 1 : 0);
+  const int nf = a.F / N, nfs = a.F_shared / N, nch = nfs + a.top * nf;  // chunks of a row: the shared expert's, the choices'
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (nfs > 0) {
+    const int row_bytes = nfs * 16, rows_ahead = min(last - first, max(1, RD_AHEAD / row_bytes));
+    for (int r = tid; r < rows_ahead; r += MO_THREADS)
+      for (int off = 0; off < row_bytes; off += RD_PIECE)
+        bulk_prefetch_l2(reinterpret_cast<const char *>(static_cast<const T *>(a.shared_down) + (size_t)(first + r) * a.F_shared) + off,
+                         min(RD_PIECE, row_bytes - off));
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (tid < a.top) base_s[tid] = static_cast<const T *>(a.w_down) + (size_t)a.chosen[tid] * a.D * a.F;
+  __syncthreads();
+  for (int s0 = first; s0 < last; s0 += M1_SPAN) {
+    const int s1 = min(last, s0 + M1_SPAN);
+    for (int m0 = s0 + group * 4; m0 < s1; m0 += AT_ONCE) {
+      float acc[4] = {};
+      for (int c0 = glane; c0 < nch; c0 += GLANES * U) {
+        uint4 v[4][U];
+        const uint4 *xp[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int c = c0 + u * GLANES;
+          const T *w = static_cast<const T *>(a.shared_down), *act = static_cast<const T *>(a.act);
+          int F = a.F_shared, k = c;  // chunk k of its part of the row
+          if (c < nfs) {
+            act += (size_t)a.top * a.ld_act;
+          } else if (c < nch) {
+            const int s = (c - nfs) / nf;
+            k = c - nfs - s * nf;
+            F = a.F;
+            w = base_s[s];
+            act += (size_t)s * a.ld_act;
+          }
+          xp[u] = reinterpret_cast<const uint4 *>(act) + k;
+          const T *row = w + (size_t)m0 * F + k * N;
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            v[r][u] = c < nch && m0 + r < s1 ? ld_stream16(row + (size_t)r * F) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (c0 + u * GLANES < nch) {
+            const uint4 x = ld_cached16(xp[u]);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[r] = dot_chunk<T>(v[r][u], x, acc[r]);
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float t = warp_sum(acc[r]);
+        if (lane == 0 && m0 + r < s1) red[m0 + r - s0][wig] = t;
+      }
+    }
+    __syncthreads();
+    if (tid < s1 - s0) {
+      float y = 0.f;
+#pragma unroll
+      for (int k = 0; k < WPR; ++k) y += red[tid][k];
+      a.y[s0 + tid] = y + (a.init ? a.init[s0 + tid] : 0.f);
+    }
+    if (s1 < last) __syncthreads();
+  }
+}
+
+// As plan_rowdot: the lanes that share a row by passes x trips.
+template <typename T>
+static int launch_one(const MoeDecodeArgs &a, int slots, bool up, bool down, cudaStream_t st) {
+  constexpr int N = Chunk<T>::N;
+  const int resident = 4 * sm_count();
+  int wpr = 1;
+#define DJV_GO(KERNEL_, GRID_)                                                                                       \
+  switch (wpr) {                                                                                                     \
+    case 1: djv::launch_kernel(KERNEL_<T, 1>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
+    case 2: djv::launch_kernel(KERNEL_<T, 2>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
+    case 4: djv::launch_kernel(KERNEL_<T, 4>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
+    default: djv::launch_kernel(KERNEL_<T, 8>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;               \
+  }                                                                                                                  \
+  count_launch();
+  if (up) {
+    const int units = a.top * a.F + a.F_shared, grid = min(resident, units);
+    rowdot_cost(2 * ceil_div(units, grid), a.D / N, 4, wpr);
+    DJV_GO(moe_one_up_kernel, grid)
+  }
+  if (down) {
+    const int grid = min(resident, a.D);
+    rowdot_cost(ceil_div(a.D, grid), a.F_shared / N + a.top * (a.F / N), 4, wpr);
+    DJV_GO(moe_one_down_kernel, grid)
+  }
+#undef DJV_GO
+  return check_launch("moe_decode");
+}
+
 template <typename T>
 static int launch_decode(const MoeDecodeArgs &a, bool up, bool down, cudaStream_t st) {
   const int slots = a.top + (a.shared_gu ? 1 : 0), fmax = a.F > a.F_shared || !a.shared_gu ? a.F : a.F_shared;
@@ -572,6 +786,7 @@ static int launch_decode(const MoeDecodeArgs &a, bool up, bool down, cudaStream_
   const bool vec_up = a.D % N == 0 && aligned16(a.x) && aligned16(a.w_gu) && aligned16(a.shared_gu);
   const bool vec_down = a.F % N == 0 && (!a.shared_gu || a.F_shared % N == 0) && a.ld_act % N == 0 && aligned16(a.act) &&
                         aligned16(a.w_down) && aligned16(a.shared_down);
+  if (a.B == 1 && vec_up && vec_down && (long long)a.top * a.F + a.F_shared <= (1 << 28)) return launch_one<T>(a, slots, up, down, st);
   if constexpr (sizeof(T) == 2) {
     // several rows share weights (both stages take this form or neither: they agree on where a choice's activations are)
     if (a.B >= 2 && a.B <= MM_B && vec_up && vec_down && a.E <= MM_E) {

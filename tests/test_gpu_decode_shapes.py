@@ -135,6 +135,13 @@ def test_routed_weights_streamed_for_several_rows(cuda, B, E, top, D, F, Fs):
     assert (got.double() - want).norm() <= 2e-3 * want.norm()
 
 
+# one row: fewer outputs than blocks, a block's outputs on both sides of a pass and of what it keeps, experts of few and of many chunks
+@pytest.mark.parametrize("E,top,D,F,Fs", [(1, 1, 8, 8, 0), (5, 2, 136, 24, 40), (8, 2, 2048, 1856, 1856), (40, 16, 264, 136, 8), (4, 4, 1032, 72, 0),
+                                          (300, 1, 64, 16, 20000), (3, 2, 40, 30008, 0), (1024, 3, 8, 8, 16), (2, 2, 9224, 600, 328), (4, 1, 76000, 16, 8)])
+def test_routed_weights_of_one_row(cuda, E, top, D, F, Fs):
+    test_routed_weights_streamed_for_several_rows(cuda, 1, E, top, D, F, Fs)
+
+
 # Distance of fp32 results from 64 bits. An addition rounds by about 2.4e-8 of the sum so far (2^-23 / sqrt(12), averaged over the
 # mantissa), which grows evenly: n in a row are off by 2.4e-8 * sqrt(n / 2) of the result, and the warps' and blocks' sums add 8
 # more; the products of an MMA that starts from zero are cut by 6e-8 to 7e-8. With 3 and 4 rows parts of 8 additions are joined,
