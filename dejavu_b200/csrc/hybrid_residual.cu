@@ -22,20 +22,34 @@ struct HyperArgs {
   int D, vocab;
 };
 
-template <typename T, int S, int V>  // V columns at a time: 4 (16-byte accesses) or 1
+// V columns at a time: 4 (16-byte accesses) or 1. NI: D <= NI * V * blockDim.x, everything a thread reads is on its way before anything
+// is stored (stores could alias the loads behind them, which otherwise wait: a row of 4096 alone took two trips to L2 for its two groups
+// of columns); 0: any D, group by group. A decode step, us before / now: 8 layers 4096 wide (17 boundaries) 701 / 688, 12 layers 2048
+// wide 454 / 448.
+template <typename T, int S, int V, int NI>
 __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
-  extern __shared__ float u_s[];  // D
+  extern __shared__ float u_s[];  // NI == 0: D
   __shared__ float coef[S * S + 2 * S];
   __shared__ float red[HS_THREADS / WARP];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int tid = threadIdx.x;
-  // the coefficients are weights: no kernel of the step writes them
+  const int tid = threadIdx.x, D = a.D;
+  constexpr int W = NI > 0 ? NI : 1;
+  // the coefficients and the norm's weights: no kernel of the step writes them
   if (tid < S * S) coef[tid] = a.y ? a.mix[tid] : (tid / S == tid % S ? 1.f : 0.f);
   if (tid >= 64 && tid < 64 + S) coef[S * S + tid - 64] = a.y ? a.w_out[tid - 64] : 0.f;
   if (tid >= 96 && tid < 96 + S) coef[S * S + S + tid - 96] = a.w_in ? a.w_in[tid - 96] : 1.f;
+  float gamma[W][V];
+  if constexpr (NI > 0) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int c = (i * (int)blockDim.x + tid) * V + v;
+        gamma[i][v] = a.gamma && c < D ? __ldg(a.gamma + c) : 0.f;
+      }
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
-  const int D = a.D;
   const int row = a.row_list ? a.row_list[blockIdx.x] : blockIdx.x;
   const float *x = a.x_in ? a.x_in + (size_t)row * S * D : nullptr;
   const T *e = nullptr;
@@ -43,10 +57,7 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
     const long long id = a.ids[row];
     e = static_cast<const T *>(a.embed) + (size_t)(id < 0 ? 0 : (id >= a.vocab ? a.vocab - 1 : id)) * D;
   }
-  float ss = 0.f;
-#pragma unroll 2
-  for (int c = tid * V; c < D; c += blockDim.x * V) {
-    float xs[S][V], yv[V], u[V];
+  auto load = [&](int c, float (&xs)[S][V], float (&yv)[V]) {
     if (x) {
 #pragma unroll
       for (int s = 0; s < S; ++s) {
@@ -66,7 +77,7 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
       }
     }
 #pragma unroll
-    for (int v = 0; v < V; ++v) yv[v] = u[v] = 0.f;
+    for (int v = 0; v < V; ++v) yv[v] = 0.f;
     if (a.y) {
       if (V == 4) {
         const float4 t = *reinterpret_cast<const float4 *>(a.y + (size_t)row * D + c);
@@ -75,6 +86,11 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
         yv[0] = a.y[(size_t)row * D + c];
       }
     }
+  };
+  float ss = 0.f;
+  auto update = [&](int c, const float (&xs)[S][V], const float (&yv)[V], float (&u)[V]) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) u[v] = 0.f;
 #pragma unroll
     for (int t = 0; t < S; ++t) {
       float nv[V];
@@ -95,9 +111,38 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
       }
     }
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      u_s[c + v] = u[v];
-      ss = fmaf(u[v], u[v], ss);
+    for (int v = 0; v < V; ++v) ss = fmaf(u[v], u[v], ss);
+  };
+  T *h = static_cast<T *>(a.h) + (size_t)blockIdx.x * D;
+  auto store = [&](int c, const T (&o)[V]) {
+    if (V == 4 && sizeof(T) == 2)
+      *reinterpret_cast<uint2 *>(h + c) = *reinterpret_cast<const uint2 *>(o);
+    else if (V == 4)
+      *reinterpret_cast<uint4 *>(h + c) = *reinterpret_cast<const uint4 *>(o);
+    else
+      h[c] = o[0];
+  };
+  float u[W][V];
+  if constexpr (NI > 0) {
+    float xs[NI][S][V], yv[NI][V];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = (i * (int)blockDim.x + tid) * V;
+      if (c < D) load(c, xs[i], yv[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = (i * (int)blockDim.x + tid) * V;
+      if (c < D) update(c, xs[i], yv[i], u[i]);
+    }
+  } else {
+#pragma unroll 2
+    for (int c = tid * V; c < D; c += blockDim.x * V) {
+      float xs[S][V], yv[V];
+      load(c, xs, yv);
+      update(c, xs, yv, u[0]);
+#pragma unroll
+      for (int v = 0; v < V; ++v) u_s[c + v] = u[0][v];
     }
   }
   if (!a.gamma) return;
@@ -107,17 +152,23 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   float tot = 0.f;
   for (int w = 0; w < blockDim.x / WARP; ++w) tot += red[w];
   const float rstd = 1.f / sqrtf(tot / (float)D + a.eps);
-  T *h = static_cast<T *>(a.h) + (size_t)blockIdx.x * D;
-  for (int c = tid * V; c < D; c += blockDim.x * V) {  // the same columns this thread wrote into u_s
-    T o[V];
+  if constexpr (NI > 0) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) o[v] = from_f<T>(u_s[c + v] * rstd * a.gamma[c + v]);
-    if (V == 4 && sizeof(T) == 2)
-      *reinterpret_cast<uint2 *>(h + c) = *reinterpret_cast<uint2 *>(o);
-    else if (V == 4)
-      *reinterpret_cast<uint4 *>(h + c) = *reinterpret_cast<uint4 *>(o);
-    else
-      h[c] = o[0];
+    for (int i = 0; i < NI; ++i) {
+      const int c = (i * (int)blockDim.x + tid) * V;
+      if (c >= D) continue;
+      T o[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) o[v] = from_f<T>(u[i][v] * rstd * gamma[i][v]);
+      store(c, o);
+    }
+  } else {
+    for (int c = tid * V; c < D; c += blockDim.x * V) {  // the same columns this thread wrote into u_s
+      T o[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) o[v] = from_f<T>(u_s[c + v] * rstd * a.gamma[c + v]);
+      store(c, o);
+    }
   }
 }
 
@@ -129,12 +180,20 @@ static int launch_hyper(const HyperArgs &a, int R, int S, cudaStream_t st) {
   const int most = R > 2 * sm_count() ? HS_THREADS / 2 : HS_THREADS;
   if (threads > most) threads = most;
   if (threads < 128) threads = 128;
-  const size_t smem = (size_t)a.D * 4;
+  // of few rows a thread keeps all its columns; of many, group by group: more blocks per multiprocessor are worth more then
+  const int ni = R > 2 * sm_count() ? 0 : ceil_div(a.D, V * threads);
+#define DJV_HS_NI(S_, NI_)                                                                              \
+  {                                                                                                     \
+    const size_t smem = NI_ ? 0 : (size_t)a.D * 4;                                                      \
+    if (smem > 48 * 1024)                                                                               \
+      cudaFuncSetAttribute(hyper_step_kernel<T, S_, V, NI_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    djv::launch_kernel(hyper_step_kernel<T, S_, V, NI_>, R, threads, smem, st, a);                      \
+  }
 #define DJV_HS(S_)                                                                                      \
   case S_:                                                                                              \
-    if (smem > 48 * 1024)                                                                               \
-      cudaFuncSetAttribute(hyper_step_kernel<T, S_, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    djv::launch_kernel(hyper_step_kernel<T, S_, V>, R, threads, smem, st, a);                           \
+    if (V == 4 && S_ <= 4 && ni == 1) DJV_HS_NI(S_, (V == 4 && S_ <= 4 ? 1 : 0))                        \
+    else if (V == 4 && S_ <= 4 && ni == 2) DJV_HS_NI(S_, (V == 4 && S_ <= 4 ? 2 : 0))                   \
+    else DJV_HS_NI(S_, 0)                                                                               \
     break
   switch (S) {
     DJV_HS(1);
@@ -147,6 +206,7 @@ static int launch_hyper(const HyperArgs &a, int R, int S, cudaStream_t st) {
     DJV_HS(8);
   }
 #undef DJV_HS
+#undef DJV_HS_NI
   count_launch();
   return check_launch("hyper_step");
 }

@@ -285,6 +285,13 @@ def test_gated_linear_attention_portions_and_decoding(dtype, aligned, heads, dk,
         close(state[b], states[b], torch.float32, 2e-5)
 
 
+# a thread's columns in registers (one group of 4 each, two, their edges), group by group, and all of many rows group by group
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("S,D,n", [(4, 2048, 1), (4, 2052, 2), (3, 4096, 1), (4, 4100, 1), (1, 512, 1), (2, 3000, 3), (5, 2048, 1), (4, 2048, 300)])
+def test_hyper_step_of_few_rows(dtype, S, D, n):
+    test_hyper_step(dtype, S, D, n)
+
+
 # ---- whole models --------------------------------------------------------------------------------------------------
 
 _models: dict = {}
