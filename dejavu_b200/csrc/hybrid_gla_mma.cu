@@ -27,14 +27,14 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 
 // rows x cols of bf16 from global (row stride ld) into shared memory, zeros up to pad_rows / pad_cols. 16-byte chunks.
 __device__ __forceinline__ void stage_rows(bf16 *dst, int pitch, const bf16 *src, long long ld, int rows, int cols,
-                                           int pad_cols) {
+                                           int pad_cols, int limit = GC) {
   const int chunks = pad_cols / 8, step = GLA_THREADS / chunks;  // (pad_cols <= 256)
   const int r0 = threadIdx.x / chunks, c = threadIdx.x - r0 * chunks;
   if (r0 >= step) return;
   const bool inside = c * 8 < cols;
   const bf16 *s = src + (size_t)r0 * ld + c * 8;
   uint32_t d = smem_addr(dst + r0 * pitch + c * 8);
-  for (int r = r0; r < GC; r += step, s += (size_t)step * ld, d += step * pitch * 2) {
+  for (int r = r0; r < limit; r += step, s += (size_t)step * ld, d += step * pitch * 2) {
     const bool ok = inside && r < rows;
     cp_async16_zfill(d, ok ? s : src, ok ? 16 : 0);
   }
@@ -181,16 +181,22 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_state_kernel(Gla
 // ---- a chunk's outputs -----------------------------------------------------------------------------------------------
 // scores of 16 query rows (block I) against 8 keys from key j0 on, relative to the sum `ref` before the block:
 // q_t exp(B_t - ref) . k_s exp(ref - B_s); the second exponent is <= 0 for keys before the block
-template <int NT>  // n-tiles of 8 value columns per warp
+// A block takes MB of the chunk's 4 blocks of 16 rows: all of them where there are many chunks and heads, fewer where the device would
+// be left idle (the incoming state is then read and split once per block). us, 8 heads of 128 / 256, 64 / 32 / 16 rows: 130 tokens 37 / 36 / 31, 333
+// 46 / 36 / 31, 700 44 / 34 / 42, 1000 43 / 32 / 42, 2000 48 / 58 / 76.
+template <int NT, int MB>  // n-tiles of 8 value columns per warp
 __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaArgs a) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   __shared__ float ssq[GW][GC];
   pdl_prologue();
   const int tid = threadIdx.x, lane = tid % WARP, warp = tid / WARP;
-  const int ci = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  constexpr int PARTS = GC / 16 / MB, WPB = GW / MB;  // blocks per chunk; warps that share 16 rows
+  const int ci = blockIdx.x / PARTS, I0 = MB == GC / 16 ? 0 : blockIdx.x % PARTS * MB, h = blockIdx.y, b = blockIdx.z;
+  const int keys = (I0 + MB) * 16;  // as many rows of the chunk as the last of this block's sees
   const int dk = a.dk, dv = a.dv, dkp = up16(dk), dvp = up16(dv);
   const int kp = dkp + 8, vp = dvp + 8, bp = dkp + 4, ap = GC + 8;
   const int t0 = ci * GC, cl = min(GC, a.n - t0);
+  if (I0 * 16 >= cl) return;
   bf16 *qs = reinterpret_cast<bf16 *>(sm_raw), *ks = qs + GC * kp, *vs = ks + GC * kp;
   float *bs = reinterpret_cast<float *>(vs + GC * vp);            // [GC][bp]
   bf16 *a_hi = reinterpret_cast<bf16 *>(bs), *a_lo = a_hi + GC * ap;  // over bs, once the sums are used up
@@ -201,18 +207,18 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   const float *S = a.contrib + (((size_t)b * a.H + h) * a.nc + ci) * (size_t)dk * dv;
   for (int i = tid * 32; i < dk * dv; i += GLA_THREADS * 32) prefetch_l2(S + i);
   const int gate_lines = (dv + 63) / 64;  // and the gates
-  for (int i = tid; i < cl * gate_lines; i += GLA_THREADS)
-    prefetch_l2(rows + (size_t)(i / gate_lines) * a.ld + goff + i % gate_lines * 64);
-  stage_rows(qs, kp, rows + qoff, a.ld, cl, dk, dkp);
-  stage_rows(ks, kp, rows + koff, a.ld, cl, dk, dkp);
-  stage_rows(vs, vp, rows + voff, a.ld, cl, dv, dvp);
+  for (int i = tid; i < (min(cl, keys) - I0 * 16) * gate_lines; i += GLA_THREADS)
+    prefetch_l2(rows + (size_t)(I0 * 16 + i / gate_lines) * a.ld + goff + i % gate_lines * 64);
+  stage_rows(qs, kp, rows + qoff, a.ld, cl, dk, dkp, keys);
+  stage_rows(ks, kp, rows + koff, a.ld, cl, dk, dkp, keys);
+  stage_rows(vs, vp, rows + voff, a.ld, cl, dv, dvp, keys);
   {
     const float *cum = a.cum + (((size_t)b * a.n + t0) * a.H + h) * dk;
     const int per = dkp / 4, step = GLA_THREADS / per;  // dk % 8 == 0
     const int r0 = tid / per, c = (tid - r0 * per) * 4;
     if (r0 < step) {
 #pragma unroll 4
-      for (int t = r0; t < GC; t += step) {
+      for (int t = r0; t < keys; t += step) {
         // (rows past the end repeat the last sum; columns past the end are zero)
         const bool ok = c < dk;
         cp_async16_zfill(smem_addr(bs + t * bp + c), ok ? cum + (size_t)min(t, cl - 1) * a.H * dk + c : cum, ok ? 16 : 0);
@@ -223,10 +229,10 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   cp_async_wait<0>();
   __syncthreads();
 
-  // scores: two warps per block of 16 rows, key tiles of 8 alternate between them
+  // scores: WPB warps per block of 16 rows, key tiles of 8 alternate between them
   const int g = lane / 4, t4 = lane % 4, lm = lane % 8, lq = lane / 8;
-  const int I = warp / 2, r0 = I * 16;
-  constexpr int MAXT = GC / 16;  // key tiles per warp
+  const int I = I0 + warp / WPB, wi = warp % WPB, r0 = I * 16;
+  constexpr int MAXT = GC / 8 / WPB;  // key tiles per warp
   float sc[MAXT][4];
 #pragma unroll
   for (int x = 0; x < MAXT; ++x)
@@ -258,7 +264,7 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
     }
 #pragma unroll
     for (int x = 0; x < MAXT; ++x) {
-      const int j0 = (2 * x + warp % 2) * 8;
+      const int j0 = (WPB * x + wi) * 8;
       if (j0 < r0 + (mild ? 16 : 0)) {
         uint32_t kh[2], kl[2];
         auto key = [&](int c, const float2 &r, uint32_t &hi, uint32_t &lo) {
@@ -275,22 +281,24 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
     }
   }
   if (!mild) {
-    // decays too strong for a common reference inside the block: every pair by itself (the tile j0 is x = I here)
-    const int j0 = r0 + (warp % 2) * 8;
-    float d[4] = {0.f, 0.f, 0.f, 0.f};
+    // decays too strong for a common reference inside the block: every pair of it by itself (a warp has one of its two tiles, or none)
+    const int tile = 2 * I + wi % 2, j0 = tile * 8;
+    if (tile % WPB == wi) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int t = r0 + g + (e / 2) * 8, s = j0 + t4 * 2 + e % 2;
-      if (s <= t)
-        for (int c = 0; c < dk; ++c)
-          d[e] = fmaf(to_f(qs[t * kp + c]) * a.scale * to_f(ks[s * kp + c]), __expf(bs[t * bp + c] - bs[s * bp + c]), d[e]);
-    }
-#pragma unroll
-    for (int x = 0; x < MAXT; ++x)
-      if (x == I) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[x][e] = d[e];
+      for (int e = 0; e < 4; ++e) {
+        const int t = r0 + g + (e / 2) * 8, s = j0 + t4 * 2 + e % 2;
+        if (s <= t)
+          for (int c = 0; c < dk; ++c)
+            d[e] = fmaf(to_f(qs[t * kp + c]) * a.scale * to_f(ks[s * kp + c]), __expf(bs[t * bp + c] - bs[s * bp + c]), d[e]);
       }
+#pragma unroll
+      for (int x = 0; x < MAXT; ++x)
+        if (x == tile / WPB) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[x][e] = d[e];
+        }
+    }
   }
   __syncthreads();
   // queries for the incoming state: q exp(B_t), split, over q and k
@@ -298,7 +306,7 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   const int kt0 = tid / kc, c2 = (tid - kt0 * kc) * 2;
   if (kt0 < kstep) {
 #pragma unroll 4
-    for (int t = kt0; t < GC; t += kstep) {
+    for (int t = I0 * 16 + kt0; t < keys; t += kstep) {
       const float2 q = b2f(*reinterpret_cast<const uint32_t *>(qs + t * kp + c2));
       const float2 s = *reinterpret_cast<const float2 *>(bs + t * bp + c2);
       uint32_t hi, lo;
@@ -310,7 +318,7 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   __syncthreads();
 #pragma unroll
   for (int x = 0; x < MAXT; ++x) {
-    const int s = (2 * x + warp % 2) * 8 + t4 * 2;
+    const int s = (WPB * x + wi) * 8 + t4 * 2;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int t = r0 + g + e * 8;
@@ -322,11 +330,11 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   }
   __syncthreads();
 
-  // outputs: a warp takes NT * 8 value columns of all 64 rows
+  // outputs: a warp takes NT * 8 value columns of all rows
   const int n0 = warp * NT * 8;
-  float acc[GC / 16][NT][4];
+  float acc[MB][NT][4];
 #pragma unroll
-  for (int m = 0; m < GC / 16; ++m)
+  for (int m = 0; m < MB; ++m)
 #pragma unroll
     for (int x = 0; x < NT; ++x)
 #pragma unroll
@@ -347,10 +355,10 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
       split2(v[2], v[3], sh[x][1], sl[x][1]);
     }
 #pragma unroll
-    for (int m = 0; m < GC / 16; ++m) {
+    for (int m = 0; m < MB; ++m) {
       uint32_t qh[4], ql[4];
-      ldmatrix_x4(qh, smem_addr(qs + (m * 16 + lrow) * kp + k0 + lcol));
-      ldmatrix_x4(ql, smem_addr(ks + (m * 16 + lrow) * kp + k0 + lcol));
+      ldmatrix_x4(qh, smem_addr(qs + ((I0 + m) * 16 + lrow) * kp + k0 + lcol));
+      ldmatrix_x4(ql, smem_addr(ks + ((I0 + m) * 16 + lrow) * kp + k0 + lcol));
 #pragma unroll
       for (int x = 0; x < NT; ++x) {
         mma_bf16(acc[m][x], qh, sh[x][0], sh[x][1]);
@@ -361,6 +369,7 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
   }
 #pragma unroll
   for (int s0 = 0; s0 < GC; s0 += 16) {
+    if (s0 >= keys) break;
     uint32_t bv[NT][2];
 #pragma unroll
     for (int x = 0; x < NT; ++x) {
@@ -371,10 +380,11 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
       bv[x][1] = r[1];
     }
 #pragma unroll
-    for (int m = s0 / 16; m < GC / 16; ++m) {
+    for (int m = 0; m < MB; ++m) {
+      if (I0 + m < s0 / 16) continue;
       uint32_t ph[4], pl[4];
-      ldmatrix_x4(ph, smem_addr(a_hi + (m * 16 + lrow) * ap + s0 + lcol));
-      ldmatrix_x4(pl, smem_addr(a_lo + (m * 16 + lrow) * ap + s0 + lcol));
+      ldmatrix_x4(ph, smem_addr(a_hi + ((I0 + m) * 16 + lrow) * ap + s0 + lcol));
+      ldmatrix_x4(pl, smem_addr(a_lo + ((I0 + m) * 16 + lrow) * ap + s0 + lcol));
 #pragma unroll
       for (int x = 0; x < NT; ++x) {
         mma_bf16(acc[m][x], ph, bv[x][0], bv[x][1]);
@@ -383,18 +393,18 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
     }
   }
   // norm over the head's values, gate (whose loads are in flight while the sums meet)
-  uint32_t gates[GC / 16][2][NT];
+  uint32_t gates[MB][2][NT];
 #pragma unroll
-  for (int m = 0; m < GC / 16; ++m)
+  for (int m = 0; m < MB; ++m)
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
       for (int x = 0; x < NT; ++x) {
-        const int t = m * 16 + g + e * 8, j = n0 + x * 8 + t4 * 2;
+        const int t = (I0 + m) * 16 + g + e * 8, j = n0 + x * 8 + t4 * 2;
         gates[m][e][x] = (t < cl && j < dv) ? *reinterpret_cast<const uint32_t *>(rows + (size_t)t * a.ld + goff + j) : 0;
       }
 #pragma unroll
-  for (int m = 0; m < GC / 16; ++m)
+  for (int m = 0; m < MB; ++m)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       float s = 0.f;
@@ -409,14 +419,14 @@ __global__ void __launch_bounds__(GLA_THREADS, 2) gla_mma_chunk_out_kernel(GlaAr
     }
   __syncthreads();
 #pragma unroll
-  for (int m = 0; m < GC / 16; ++m)
+  for (int m = 0; m < MB; ++m)
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int t = m * 16 + g + e * 8;
+      const int t = (I0 + m) * 16 + g + e * 8;
       if (t >= cl) continue;
       float tot = 0.f;
 #pragma unroll
-      for (int w = 0; w < GW; ++w) tot += ssq[w][t];
+      for (int w = 0; w < GW; ++w) tot += ssq[w][m * 16 + g + e * 8];
       const float rn = 1.f / sqrtf(tot / (float)dv + a.eps);
       bf16 *out = static_cast<bf16 *>(a.out) + (((size_t)b * a.n + t0 + t) * a.H + h) * dv;
 #pragma unroll
@@ -459,11 +469,19 @@ int gla_mma_chunk_state(const GlaArgs &a, cudaStream_t st) {
 
 int gla_mma_chunk_out(const GlaArgs &a, cudaStream_t st) {
   const size_t smem = mma_out_smem(a.dk, a.dv);
-  const dim3 grid(a.nc, a.H, a.B);
-#define DJV_GO(NT_)                                                                                              \
-  {                                                                                                              \
-    cudaFuncSetAttribute(gla_mma_chunk_out_kernel<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    djv::launch_kernel(gla_mma_chunk_out_kernel<NT_>, grid, dim3(GLA_THREADS), smem, st, a);                     \
+  // as few rows per block as are one wave of two blocks per multiprocessor
+  const long long chunks = (long long)a.nc * a.H * a.B, slots = 2 * sm_count();
+  const int mb = chunks * 4 <= slots ? 1 : chunks * 2 <= slots ? 2 : 4;
+#define DJV_GO_MB(NT_, MB_)                                                                                           \
+  {                                                                                                                   \
+    cudaFuncSetAttribute(gla_mma_chunk_out_kernel<NT_, MB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    djv::launch_kernel(gla_mma_chunk_out_kernel<NT_, MB_>, dim3(a.nc * (4 / MB_), a.H, a.B), dim3(GLA_THREADS), smem, st, a); \
+  }
+#define DJV_GO(NT_)                   \
+  {                                   \
+    if (mb == 1) DJV_GO_MB(NT_, 1)    \
+    else if (mb == 2) DJV_GO_MB(NT_, 2) \
+    else DJV_GO_MB(NT_, 4)            \
   }
   const int nt = ceil_div(a.dv, 64);
   if (nt == 1) DJV_GO(1)
@@ -471,6 +489,7 @@ int gla_mma_chunk_out(const GlaArgs &a, cudaStream_t st) {
   else if (nt == 3) DJV_GO(3)
   else DJV_GO(4)
 #undef DJV_GO
+#undef DJV_GO_MB
   count_launch();
   return check_launch("gla_prefill");
 }

@@ -285,6 +285,27 @@ def test_gated_linear_attention_portions_and_decoding(dtype, aligned, heads, dk,
         close(state[b], states[b], torch.float32, 2e-5)
 
 
+@pytest.mark.parametrize("dk,dv,tau", [(128, 256, 8.0), (64, 40, 0.3), (128, 256, 0.1), (16, 200, 4.0)])
+def test_gated_linear_attention_is_the_same_whatever_a_block_takes(dk, dv, tau):
+    """Blocks take 16, 32 or 64 rows of a chunk by the number of chunks: heads that are copies of one another (1, 24 and 60 of
+    them, of 4 chunks) have the same outputs bit by bit, decays strong and mild."""
+    from dejavu_b200 import ops
+
+    g, n, rank = gen(dk + dv), 230, 4
+    q, k, v, gate = (rnd(g, n, d, dtype=torch.bfloat16) for d in (dk, dk, dv, dv))
+    low, a2, bias, norm = rnd(g, n, rank, dtype=torch.bfloat16), rnd(g, dk, rank), 2.0 + 2.0 * rnd(g, dk), 1 + 0.3 * rnd(g, dv)
+    first = None
+    for H_ in (1, 24, 60):
+        rows = torch.cat([t.repeat(1, H_) for t in (q, k, v, gate)] + [low], 1)
+        buf = torch.zeros(n, (rows.shape[1] + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")
+        buf[:, :rows.shape[1]] = dev(rows, torch.bfloat16)
+        state = torch.zeros(1, H_, dk, dv, device="cuda")
+        out = ops.gated_linear_attention(buf, dev(a2.repeat(H_, 1)), dev(bias.repeat(H_)), tau, dev(norm), 1e-5, dk ** -0.5, state,
+                                         torch.zeros(1, dtype=torch.int64, device="cuda"), n).view(n, H_, dv)
+        first = out[:, 0] if first is None else first
+        assert torch.equal(out, first[:, None].expand_as(out)), H_
+
+
 # a thread's columns in registers (one group of 4 each, two, their edges), group by group, and all of many rows group by group
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("S,D,n", [(4, 2048, 1), (4, 2052, 2), (3, 4096, 1), (4, 4100, 1), (1, 512, 1), (2, 3000, 3), (5, 2048, 1), (4, 2048, 300)])
