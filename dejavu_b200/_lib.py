@@ -138,9 +138,31 @@ ROUTED_SIGNATURES = {
 SHARED = ("djv_hyper_step", "djv_residual_step", "djv_dense_gemv", "djv_glu", "djv_softcap", "djv_rotary",
           "djv_window_timeouts")
 
+# Signatures by their letters, result first: i int, p pointer, l long long, z size_t, f float. Those of the status and size functions
+# that `call` and `query` see are compiled into _calls (build.py), one binding for each.
+_LETTERS = {_i: "i", _vp: "p", _ll: "l", _sz: "z", _f: "f"}
+
+
+def _signature(fn_name: str) -> str:
+    for table in (SIGNATURES, HYBRID_SIGNATURES, ROUTED_SIGNATURES):
+        if fn_name in table:
+            res, args = table[fn_name]
+            return "".join(_LETTERS.get(t, "?") for t in (res, *args))
+    raise AttributeError(fn_name)
+
+
+KINDS = {k: n for n, k in enumerate(sorted({_signature(f) for t in (SIGNATURES, HYBRID_SIGNATURES, ROUTED_SIGNATURES) for f in t
+                                            if _signature(f)[0] in "iz" and "?" not in _signature(f)}))}
+
 _lib = None
 _hybrid = None
 _routed = None
+_bound: dict = {}  # function name -> what `call` and `query` call, for the libraries loaded so far
+
+try:  # generated and compiled by build.py; without it every call goes through ctypes
+    from . import _calls
+except ImportError:
+    _calls = None
 
 
 def _open(path, signatures) -> C.CDLL:
@@ -154,6 +176,7 @@ def _open(path, signatures) -> C.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+    _bound.clear()
     return lib
 
 
@@ -196,9 +219,30 @@ def check(fn_name: str, status: int, lib=None) -> None:
         raise DejavuKernelError(fn_name, status, msg)
 
 
+def _bind(fn_name: str):
+    """The function as the compiled binding has it. That takes integers, floats and None; for anything else it answers
+    NotImplemented without having called, and ctypes, which also takes its own types, decides."""
+    fn = getattr(_library_of(fn_name), fn_name)
+    kind = KINDS.get(_signature(fn_name))
+    if _calls is not None and kind is not None and _calls.KINDS == " ".join(KINDS):
+        fn = _calls.bind(kind, C.cast(fn, _vp).value)
+    _bound[fn_name] = fn
+    return fn
+
+
 def call(fn_name: str, *args) -> None:
-    lib = _library_of(fn_name)
-    check(fn_name, getattr(lib, fn_name)(*args), lib)
+    """Calls a function that returns a status, and raises if that is not OK."""
+    status = (_bound.get(fn_name) or _bind(fn_name))(*args)
+    if status != OK:
+        if status is NotImplemented:
+            status = getattr(_library_of(fn_name), fn_name)(*args)
+        check(fn_name, status, _library_of(fn_name))
+
+
+def query(fn_name: str, *args) -> int:
+    """Calls a function that returns a size."""
+    value = (_bound.get(fn_name) or _bind(fn_name))(*args)
+    return getattr(_library_of(fn_name), fn_name)(*args) if value is NotImplemented else value
 
 
 def launch_count() -> int:

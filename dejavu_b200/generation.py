@@ -193,7 +193,8 @@ class SequencePool:
         params = self.live[request]
         if params.sequence_len_offset and len(tokens) > 1 and not getattr(self.model, "takes_portions", False):
             raise ValueError("this model takes a prompt in one piece")
-        ids = torch.tensor([tokens], dtype=torch.long, device=self.device)
+        # (a blocking copy would wait for the portion before this one)
+        ids = torch.tensor([tokens], dtype=torch.long).to(self.device, non_blocking=True)
         pos = torch.full((1, 1), params.sequence_len_offset, dtype=torch.long, device=self.device)
         first = params.sequence_len_offset == 0 and len(tokens) > 1  # (models number a prompt's tokens themselves)
         return step(self.model, params, ids, None if first else pos, logit_rows)[0]

@@ -124,7 +124,8 @@ class HybridDecoder(nn.Module, GenerationMixin):
             rows, R = None, n
         else:
             R = len(logit_rows)
-            rows = torch.tensor([b * n + t for b in range(B) for t in logit_rows], dtype=torch.int32, device=dev)
+            rows = torch.tensor([b * n + t for b in range(B) for t in logit_rows], dtype=torch.int32)
+            rows = rows.to(dev, non_blocking=True)  # (a blocking copy would wait for all the work before it)
         h = self.hidden(input_ids.reshape(-1).contiguous(), inference_params.key_value_memory_dict, pos, n, past, rows,
                         collect)
         if R == 0:

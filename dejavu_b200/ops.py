@@ -17,7 +17,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import call
+from ._lib import call, query
 
 _ACTIVATIONS = ["id", "relu", "gelu", "gelu_approx", "squared_relu"]
 
@@ -25,7 +25,7 @@ _scratch_cache: dict = {}
 
 
 def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())  # (without a Stream object for each call)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # (without a Stream object for each call)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -132,9 +132,8 @@ def gather_transposed_gemv(
         assert x.dtype == bias.dtype, f"Input and bias must have the same dtype, got {x.dtype} and {bias.dtype}"
     idx, idx64 = _idx_args(idx)
     output = torch.empty(batch, N, device=x.device, dtype=x.dtype)
-    lib = _lib.load()
-    need = max(lib.djv_gather_transposed_gemv_scratch_bytes(batch, N, M),
-               lib.djv_mlp_sparse_fused_scratch_bytes(batch, N, M) if batch <= 4 else 0)
+    need = max(query("djv_gather_transposed_gemv_scratch_bytes", batch, N, M),
+               query("djv_mlp_sparse_fused_scratch_bytes", batch, N, M) if batch <= 4 else 0)
     scratch = _scratch(need, x.device)
     if push_comm is not None and M >= 1 and batch <= 4:
         seq = push_comm.next_seq()
@@ -159,7 +158,7 @@ def dense_transposed_gemv(x: torch.Tensor, weight_t: torch.Tensor, bias: Optiona
     assert weight_t.stride(1) == 1 and x.dtype == weight_t.dtype == torch.float16
     x = x.contiguous()
     output = torch.empty(batch, N, device=x.device, dtype=x.dtype)
-    need = _lib.load().djv_gather_transposed_gemv_scratch_bytes(batch, N, M)
+    need = query("djv_gather_transposed_gemv_scratch_bytes", batch, N, M)
     scratch = _scratch(need, x.device)
     if push_comm is not None and batch <= 4:
         seq = push_comm.next_seq()
@@ -176,10 +175,9 @@ def _mlp_sparse_call(x, W1, W2t, idx, bias1, bias2):
     """Both products of mlp_sparse behind one call into the library."""
     batch, N = x.shape
     M = idx.shape[0]
-    lib = _lib.load()
-    need = lib.djv_gather_transposed_gemv_scratch_bytes(batch, N, M)
+    need = query("djv_gather_transposed_gemv_scratch_bytes", batch, N, M)
     if batch <= 4:
-        need = max(need, lib.djv_mlp_sparse_fused_scratch_bytes(batch, N, M))
+        need = max(need, query("djv_mlp_sparse_fused_scratch_bytes", batch, N, M))
     stream = _stream()
     scratch = _scratch(need, x.device, stream)
     hidden, output = x.new_empty(batch, M), x.new_empty(batch, N)
@@ -202,12 +200,13 @@ def mlp_sparse(x, W1, W2t, idx, bias1=None, bias2=None, push_comm=None, fused=Fa
         assert x.dtype == W1.dtype == W2t.dtype == torch.float16 and W1.stride(1) == 1 and W2t.stride(1) == 1
         assert W1.shape[1] == N and W2t.shape[1] == N
     if not fused:
-        tensors = [t for t in (x, W1, W2t, bias1, bias2) if t is not None]
-        if (push_comm is None and 1 <= batch <= _lib.MAX_BATCH and W1.shape[1] == N == W2t.shape[1] and W1.stride(1) == 1
-                and W2t.stride(1) == 1 and all(t.is_cuda and t.dtype == torch.float16 for t in tensors)
-                and idx.is_cuda and idx.dtype in (torch.int32, torch.int64) and idx.is_contiguous() and x.is_contiguous()
-                and (bias1 is None or (bias1.shape == W1.shape[:1] and bias1.is_contiguous()))
-                and (bias2 is None or (bias2.shape == (N,) and bias2.is_contiguous()))):
+        f16 = torch.float16
+        (Z, N1), (_, N2) = W1.shape, W2t.shape
+        if (push_comm is None and 1 <= batch <= _lib.MAX_BATCH and N1 == N == N2 and W1.stride(1) == 1 and W2t.stride(1) == 1
+                and x.dtype is f16 and W1.dtype is f16 and W2t.dtype is f16 and idx.dtype in (torch.int32, torch.int64)
+                and x.is_cuda and W1.is_cuda and W2t.is_cuda and idx.is_cuda and idx.is_contiguous() and x.is_contiguous()
+                and (bias1 is None or (bias1.dtype is f16 and bias1.is_cuda and bias1.shape == (Z,) and bias1.is_contiguous()))
+                and (bias2 is None or (bias2.dtype is f16 and bias2.is_cuda and bias2.shape == (N,) and bias2.is_contiguous()))):
             return _mlp_sparse_call(x, W1, W2t, idx, bias1, bias2)
         # other forms, and what is refused: one product at a time
         x = gather_gemv(x, W1, idx, bias1, activation="relu")
@@ -222,7 +221,7 @@ def mlp_sparse(x, W1, W2t, idx, bias1=None, bias2=None, push_comm=None, fused=Fa
         bias2 = bias2.contiguous()
         assert bias2.shape == (N,) and bias2.dtype == x.dtype
     output = torch.empty(batch, N, device=x.device, dtype=x.dtype)
-    need = _lib.load().djv_mlp_sparse_fused_scratch_bytes(batch, N, M)
+    need = query("djv_mlp_sparse_fused_scratch_bytes", batch, N, M)
     scratch = _scratch(need, x.device)
     call("djv_mlp_sparse_fused", output.data_ptr(), W1.data_ptr(), W2t.data_ptr(), x.data_ptr(), idx.data_ptr(),
          _ptr(bias1), _ptr(bias2), batch, N, M, W1.shape[0], W1.stride(0), W2t.stride(0), idx64,
@@ -249,7 +248,7 @@ def mlp_sparse_after_exchange(comm, partial, residual, norm_weight, norm_bias, e
     idx, idx64 = _idx_args(idx)
     out = torch.empty(batch, N, device=partial.device, dtype=partial.dtype)
     r = torch.empty(batch, N, device=partial.device, dtype=partial.dtype)
-    need = _lib.load().djv_mlp_sparse_fused_scratch_bytes(batch, N, M)
+    need = query("djv_mlp_sparse_fused_scratch_bytes", batch, N, M)
     scratch = _scratch(need, partial.device)
     seq_out = comm.next_seq() if push else -1
     call("djv_mlp_sparse_fused_exchange", comm.handle, seq_in, _lib.EXCHANGE_REFILL, seq_out,
@@ -507,7 +506,7 @@ def decode_attention(q, k_cache, v_cache, head_idx, length: int, softmax_scale: 
         head_idx = head_idx.contiguous()
         nnz = head_idx.shape[0]
     ctx = torch.empty_like(q)
-    need = _lib.load().djv_decode_attn_scratch_bytes(max(nnz, 1), B, hd, S)
+    need = query("djv_decode_attn_scratch_bytes", max(nnz, 1), B, hd, S)
     scratch = _scratch(need, q.device)
     call("djv_decode_attn", ctx.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _ptr(head_idx),
          nnz, B, nheads, hd, S, length, float(softmax_scale), scratch.data_ptr(), scratch.numel(), _stream())
@@ -649,7 +648,7 @@ def gated_linear_attention(proj, a2, a2_bias, tau: float, norm, eps: float, scal
     if n == 1:
         call("djv_gla_decode", *args, H, dk, dv, _stream())
     else:
-        need = _lib.load_hybrid().djv_gla_scratch_bytes(code, b, n, H, dk, dv)
+        need = query("djv_gla_scratch_bytes", code, b, n, H, dk, dv)
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=proj.device)
         call("djv_gla_prefill", *args, n, H, dk, dv, scratch.data_ptr(), scratch.numel(), _stream())
     return out
@@ -687,7 +686,7 @@ def residual_step(x, y, gamma_y, gamma, eps: float, dtype, *, base: float = 0.0,
 
 def mlstm_state(batch: int, heads: int, dk: int, dv: int, device) -> torch.Tensor:
     """State of a matrix memory: S (dk, dv), n (dk) and m of every head, one fp32 row each."""
-    return torch.zeros(batch, heads, _lib.load_routed().djv_mlstm_state_floats(dk, dv), dtype=torch.float32, device=device)
+    return torch.zeros(batch, heads, query("djv_mlstm_state_floats", dk, dv), dtype=torch.float32, device=device)
 
 
 def mlstm(proj, gates, bias_i, bias_f, cap: float, norm, eps: float, scale: float, state, pos, n: int, dk: int, dv: int,
@@ -708,7 +707,7 @@ def mlstm(proj, gates, bias_i, bias_f, cap: float, norm, eps: float, scale: floa
     if n == 1:
         call("djv_mlstm_decode", *args, H, dk, dv, _stream())
     else:
-        need = _lib.load_routed().djv_mlstm_scratch_bytes(code, b, n, H, dk, dv)
+        need = query("djv_mlstm_scratch_bytes", code, b, n, H, dk, dv)
         scratch = torch.empty(max(need, 256), dtype=torch.uint8, device=proj.device)
         call("djv_mlstm_prefill", *args, n, H, dk, dv, scratch.data_ptr(), scratch.numel(), _stream())
     return out
@@ -770,7 +769,7 @@ def latent_attention_decode(proj, uk, uv, norm, eps: float, freqs, ring, gate, p
     _require_cuda(proj, uk, uv, ring, pos, gate)
     _f32(norm, freqs)
     dev = ring.device
-    floats = _lib.load_routed().djv_latent_scratch_floats(b, heads, rank, min(window, cap))
+    floats = query("djv_latent_scratch_floats", b, heads, rank, min(window, cap))
     qc, sums = scratch or (torch.empty(b, heads, width, dtype=ring.dtype, device=dev),
                            torch.empty(floats, dtype=torch.float32, device=dev))
     out = torch.empty(b, heads * dv, dtype=ring.dtype, device=dev)

@@ -113,3 +113,28 @@ def test_operators_refuse_cpu_tensors():
     with pytest.raises(RuntimeError, match="no CPU path"):
         ops.gather_gemv(torch.zeros(1, 64, dtype=torch.float16), torch.zeros(8, 64, dtype=torch.float16),
                         torch.arange(4))
+
+
+def test_compiled_bindings_answer_as_ctypes_does():
+    """Sizes and statuses through the generated bindings, and what only ctypes can decide (its own types, too many bits, wrong ones)."""
+    import ctypes as C
+
+    import pytest
+
+    from dejavu_b200 import _lib
+
+    assert _lib._calls is not None and _lib._calls.KINDS == " ".join(_lib.KINDS)
+    lib = _lib.load()
+    assert isinstance(_lib._bind("djv_topk"), type(len))
+    for args in ((3, 4096, 512), (0, 8, 1), (32, 12288, 4096)):
+        assert _lib.query("djv_gather_transposed_gemv_scratch_bytes", *args) == lib.djv_gather_transposed_gemv_scratch_bytes(*args)
+    for pointer in (None, 0, C.c_void_p(None)):
+        with pytest.raises(_lib.DejavuKernelError, match="null scores"):
+            _lib.call("djv_topk", None, None, pointer, 1, 1, 0, None)
+    with pytest.raises(_lib.DejavuKernelError, match=r"K=2 outside \[0,1\]"):  # more bits than an int has: cut to 1, as ctypes does
+        _lib.call("djv_topk", 64, None, 64, 2 ** 40 + 1, 2, 0, None)
+    for wrong in ((1.5, None, None, 1, 1, 0, None), (None, None, "", 1, 1, 0, None), (None,)):
+        with pytest.raises((C.ArgumentError, TypeError)):
+            _lib.call("djv_topk", *wrong)
+    with pytest.raises(AttributeError):
+        _lib.call("djv_no_such_function")
