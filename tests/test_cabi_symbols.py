@@ -133,7 +133,7 @@ def test_compiled_bindings_answer_as_ctypes_does():
             _lib.call("djv_topk", None, None, pointer, 1, 1, 0, None)
     with pytest.raises(_lib.DejavuKernelError, match=r"K=2 outside \[0,1\]"):  # more bits than an int has: cut to 1, as ctypes does
         _lib.call("djv_topk", 64, None, 64, 2 ** 40 + 1, 2, 0, None)
-    for wrong in ((1.5, None, None, 1, 1, 0, None), (None, None, "", 1, 1, 0, None), (None,)):
+    for wrong in ((1.5, None, None, 1, 1, 0, None), (None, None, [], 1, 1, 0, None), (None,)):
         with pytest.raises((C.ArgumentError, TypeError)):
             _lib.call("djv_topk", *wrong)
     with pytest.raises(AttributeError):
