@@ -158,11 +158,7 @@ _lib = None
 _hybrid = None
 _routed = None
 _bound: dict = {}  # function name -> what `call` and `query` call, for the libraries loaded so far
-
-try:  # generated and compiled by build.py; without it every call goes through ctypes
-    from . import _calls
-except ImportError:
-    _calls = None
+_calls = None  # the compiled bindings, once they are there
 
 
 def _open(path, signatures) -> C.CDLL:
@@ -222,8 +218,14 @@ def check(fn_name: str, status: int, lib=None) -> None:
 def _bind(fn_name: str):
     """The function as the compiled binding has it. That takes integers, floats and None; for anything else it answers
     NotImplemented without having called, and ctypes, which also takes its own types, decides."""
+    global _calls
     fn = getattr(_library_of(fn_name), fn_name)
     kind = KINDS.get(_signature(fn_name))
+    if _calls is None:
+        try:  # generated and compiled by build.py; without them every call goes through ctypes
+            from . import _calls
+        except ImportError:
+            pass
     if _calls is not None and kind is not None and _calls.KINDS == " ".join(KINDS):
         fn = _calls.bind(kind, C.cast(fn, _vp).value)
     _bound[fn_name] = fn

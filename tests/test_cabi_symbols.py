@@ -115,17 +115,13 @@ def test_operators_refuse_cpu_tensors():
                         torch.arange(4))
 
 
-def test_compiled_bindings_answer_as_ctypes_does():
+def test_compiled_bindings_answer_as_ctypes_does(lib):
     """Sizes and statuses through the generated bindings, and what only ctypes can decide (its own types, too many bits, wrong ones)."""
     import ctypes as C
 
-    import pytest
-
     from dejavu_b200 import _lib
 
-    assert _lib._calls is not None and _lib._calls.KINDS == " ".join(_lib.KINDS)
-    lib = _lib.load()
-    assert isinstance(_lib._bind("djv_topk"), type(len))
+    assert isinstance(_lib._bind("djv_topk"), type(len)) and _lib._calls.KINDS == " ".join(_lib.KINDS)
     for args in ((3, 4096, 512), (0, 8, 1), (32, 12288, 4096)):
         assert _lib.query("djv_gather_transposed_gemv_scratch_bytes", *args) == lib.djv_gather_transposed_gemv_scratch_bytes(*args)
     for pointer in (None, 0, C.c_void_p(None)):
