@@ -32,12 +32,15 @@ def build(cfg, cuda, seed=0, local_exchange=False):
 
 
 def record_selections(model):
+    from dejavu_b200.modules import _wait_ready
+
     rec = []
 
     def hook(layer_idx):
         def fn(_m, _inp, out):
             mlp_idx = out[1]
             att_idx = out[2] if len(out) > 2 else None
+            _wait_ready(att_idx)  # made on a side stream; nothing on this one has waited for it yet
             rec[-1][layer_idx] = {"mlp_idx": None if mlp_idx is None else mlp_idx.cpu(),
                                   "att_idx": None if att_idx is None else att_idx.cpu()}
         return fn
