@@ -52,10 +52,13 @@ constexpr int RD_FEW = 8;     // as many as a block with 4 chunks per row can ha
 // 464.9, 458.7, 451.7, 460.6; with routed experts, 2048 wide 568.1, 576.5, 564.5, 563.6, 569.9, 4096 wide 640.0, 646.0, 630.8, 629.9,
 // 636.2; this rule 543.6 / 597.2, 455.4, 566.1, 626.2. Lines are an instruction each, and with more bytes the loads of the kernel
 // before queue up behind them. In the sparse steps, whose side streams fill the gaps, neither form gains (8034 / 8019 us for 16
-// steps of 8 layers, 4096 wide, 13488 / 13365 of 4 layers, 9216 wide): those keep the lines.
+// steps of 8 layers, 4096 wide, 13488 / 13365 of 4 layers, 9216 wide): those, fp16, keep the lines.
 constexpr int RD_PIECE = 8192;
 constexpr int RD_AHEAD = 16384;
-constexpr int RD_AHEAD_LINES = -1;  // 8 KB of each of 16 rows, line by line, gathered ones included
+template <typename T>
+constexpr bool is_half = false;
+template <>
+constexpr bool is_half<__half> = true;
 
 // Blocks per multiprocessor that the registers of a pass leave room for: ROWS * U 16-byte loads, ROWS * B sums.
 __host__ __device__ constexpr int rd_blocks(int B) { return B == 1 ? 4 : B == 2 ? 3 : B <= 4 ? 2 : 1; }
@@ -82,7 +85,7 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   const int last = first + (per_block + (bx < rest ? 1 : 0)) * UNIT;
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (ahead > 0) {
+  if constexpr (!is_half<T>) {
     // Weights are not produced by any kernel of a step, and a prefetch could not return a stale value anyway.
     const int row_bytes = nchunks * 16, pieces = (row_bytes + RD_PIECE - 1) / RD_PIECE;
     const int total = (int)min((long long)(last - first) * pieces, max(1ll, (long long)ahead * pieces / row_bytes));
@@ -90,8 +93,8 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
       const int off = p % pieces * RD_PIECE;
       bulk_prefetch_l2(reinterpret_cast<const char *>(W + (first + p / pieces) * ldw) + off, min(RD_PIECE, row_bytes - off));
     }
-  } else if (ahead == RD_AHEAD_LINES) {
-    // The index list is complete (identity, or the caller's promise).
+  } else if (ahead) {
+    // The index list is complete (identity, or the caller's promise): 8 KB of each of 16 rows, line by line.
     constexpr int LINES = 64, MAX_ROWS = 16;
     const int row_lines = (int)min((long long)LINES, ((long long)N * (int)sizeof(T) + 127) / 128);
     for (int m = first + warp; m < min(last, first + MAX_ROWS); m += RD_WARPS) {
