@@ -21,6 +21,7 @@ MAX_BATCH = 32
 KV_WINDOW = 16
 EXCHANGE_REFILL = 1
 ATTN_STATE_HDR = 8
+SCRATCH_HEAD = 4096  # bytes of a workspace that have to be zero before its first use
 
 
 class DejavuKernelError(RuntimeError):

@@ -69,6 +69,7 @@ class DecodingCGCache:
     logits: Optional[torch.Tensor] = None
     next_token: Optional[torch.Tensor] = None
     launches_per_step: int = 0
+    workspaces: list = field(default_factory=list)
 
     def run(self, new_input_ids, new_position_ids):
         self.input_ids.copy_(new_input_ids)
@@ -104,7 +105,11 @@ def update_graph_cache(model, cache, batch_size, seqlen_og, max_seqlen, tensor_p
     cache.position_ids = torch.full((batch_size, 1), seqlen_og, dtype=torch.long, device=device)
     # the decode state must describe a decodable position while warming up
     model.reset_decode_state(seqlen_og, device, max_seqlen, batch_size)
-    s = torch.cuda.Stream()
+    # captured on a high-priority stream: when a main-chain kernel and look-ahead work on a side stream both
+    # have blocks waiting for a multiprocessor, the main chain goes first. The steps before run there too, so that what is made once
+    # for each stream (workspaces) is there when the capture begins and no replay makes it again.
+    priority = int(os.environ.get("DJV_MAIN_PRIORITY", "-1"))  # development knob; 0 = same as the side streams
+    s = torch.cuda.Stream(device=device, priority=priority)
     s.wait_stream(torch.cuda.current_stream())
     def step():
         cache.logits = model(cache.input_ids, position_ids=cache.position_ids,
@@ -122,14 +127,12 @@ def update_graph_cache(model, cache, batch_size, seqlen_og, max_seqlen, tensor_p
             torch.distributed.barrier()
     torch.cuda.current_stream().wait_stream(s)
     graph = torch.cuda.CUDAGraph()
-    from . import _lib
+    from . import _lib, ops
 
     launches_before = _lib.launch_count()
-    # captured on a high-priority stream: when a main-chain kernel and look-ahead work on a side stream both
-    # have blocks waiting for a multiprocessor, the main chain goes first
-    priority = int(os.environ.get("DJV_MAIN_PRIORITY", "-1"))  # development knob; 0 = same as the side streams
-    with torch.cuda.graph(graph, stream=torch.cuda.Stream(device=device, priority=priority)):
+    with torch.cuda.graph(graph, stream=s):
         step()
+    cache.workspaces = ops.take_workspaces(s.cuda_stream)  # the graph's own from here on, as long as it may be replayed
     cache.launches_per_step = _lib.launch_count() - launches_before  # kernels of libdejavu_b200 per replay
     cache.graph = graph
     return cache

@@ -39,14 +39,21 @@ def _require_cuda(*tensors):
 
 
 def _scratch(nbytes: int, device: torch.device, stream: Optional[int] = None) -> torch.Tensor:
-    """Zero-initialised per-(device, stream) workspace; the kernels leave their counters zeroed."""
+    """Per-(device, stream) workspace. Its head, where the kernels keep counters, starts as zeros and is left so by them; what is
+    behind it is written before it is read."""
     key = (device.index, _stream() if stream is None else stream)
     buf = _scratch_cache.get(key)
     if buf is None or buf.numel() < nbytes:
         size = max(nbytes, 1 << 20)
-        buf = torch.zeros(size, dtype=torch.uint8, device=device)
+        buf = torch.empty(size, dtype=torch.uint8, device=device)
+        buf[:_lib.SCRATCH_HEAD].zero_()
         _scratch_cache[key] = buf
     return buf
+
+
+def take_workspaces(stream: int) -> list:
+    """The workspaces of a stream, which then gets new ones: a captured graph keeps those that it was captured with."""
+    return [_scratch_cache.pop(key) for key in [k for k in _scratch_cache if k[1] == stream]]
 
 
 def _idx_args(idx: torch.Tensor):
