@@ -333,7 +333,7 @@ class ParallelFusedMLPDejavu(nn.Module):
             assert x.size(1) == 1
             assert self.activation == "relu", "the sparse path applies ReLU (gather_gemv.py:655)"
             # idx came from a side stream and the main stream has waited on its event already
-            with ops.indices_ready(EARLY_PREFETCH and getattr(idx, "_ready_event", None) is not None):
+            with ops.indices_ready(EARLY_PREFETCH and getattr(idx, "_ready_event", None) is not None, self.fc1.weight.shape[0]):
                 out = ops.mlp_sparse(x.view(x.size(0), -1), self.fc1.weight, self.fc2.weight_t, idx, self.fc1.bias,
                                      self.fc2.bias, push_comm=self.push_comm)
             out = out.view(x.size(0), 1, -1)

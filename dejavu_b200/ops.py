@@ -435,14 +435,15 @@ def batch_sum(x: torch.Tensor) -> torch.Tensor:
 
 
 @contextlib.contextmanager
-def indices_ready(ready: bool = True):
+def indices_ready(ready: bool = True, rows: int = 1):
     """Inside this block the caller promises that the index lists / attention state passed to the operators
     are complete before the kernels can start (produced on another stream and joined with an event): the
     kernels then prefetch their weight rows while the kernel launched before them is still running
-    (see djv_set_early_weight_prefetch)."""
+    (see djv_set_early_weight_prefetch). `rows`: how many rows the matrices have that the lists name rows of; a gathered
+    product asks ahead only for rows below it."""
     lib = _lib.load()
     if ready:
-        lib.djv_set_early_weight_prefetch(1)
+        lib.djv_set_early_weight_prefetch(max(1, rows))
     try:
         yield
     finally:

@@ -98,6 +98,24 @@ def test_mlp_sparse_fused_with_early_weight_stream(cuda):
     assert torch.equal(got, want) and filler is not None
 
 
+@pytest.mark.parametrize("batch", [1, 2, 3])
+def test_rows_are_asked_for_ahead_within_the_matrix(cuda, batch):
+    """A list that is made just before its product, in memory that held anything: what is asked for too early changes nothing."""
+    from dejavu_b200 import ops
+
+    gen = torch.Generator().manual_seed(11)
+    W1, W2t, b1, b2, x, _ = [t.to(cuda) for t in _mlp_inputs(gen, 4096, 1024, 300, batch, "rand32")]
+    scores = torch.randn(4096, generator=gen).to(cuda)
+    want = ops.mlp_sparse(x, W1, W2t, ops.topk_indices(scores, 300, torch.int32), b1, b2)
+    for _ in range(3):
+        old = torch.full((300,), 0x7F7F7F7F, dtype=torch.int32, device=cuda)
+        del old  # (its memory is the next list's)
+        idx = ops.topk_indices(scores, 300, torch.int32)
+        with ops.indices_ready(True, 4096):
+            got = ops.mlp_sparse(x, W1, W2t, idx, b1, b2)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("Z,N,M,B", [(6144, 12288, 512, 1), (4608, 9216, 200, 3), (1024, 256, 64, 4)])
 def test_ring_pipeline_runs_fc1_and_fc2_alone(cuda, monkeypatch, Z, N, M, B):
     """The same pipeline behind djv_gather_gemv / djv_gather_transposed_gemv (development knob)."""
