@@ -265,3 +265,32 @@ def test_state_dict_keys_follow_the_reference(cuda):
     assert sd["transformer.layers.0.mlp.fc2.weight"].shape == (256, 1024)
     assert sd["transformer.layers.0.mixer.Wqkv.weight"].shape == (768, 256)
     assert model.transformer.layers[0].mixer.mlp_k == 256 and model.transformer.layers[0].mixer.att_k == 2
+
+
+@pytest.mark.parametrize("B,mlp_K,att_K", [(1, 256, 2), (1, 1024, 2), (1, 256, 4), (3, 256, 2)])
+def test_last_look_ahead_is_for_those_who_listen(cuda, B, mlp_K, att_K):
+    """The predictors of the last layer run only where something could see what they say; the logits are the same bits."""
+    from dejavu_b200 import _lib
+    from dejavu_b200.generation import InferenceParams, allocate_kv_cache
+
+    cfg = tiny_config(mlp_K, att_K)
+    model = build(cfg, cuda)
+    ids = torch.randint(0, cfg.vocab_size, (B, 5), generator=torch.Generator().manual_seed(1)).to(cuda)
+    seen, got, launches = [], [], []
+    for listen in (False, True, False):
+        handle = model.transformer.layers[-1].mixer.register_forward_hook(lambda *a: seen.append(a[2][2:])) if listen else None
+        ip = InferenceParams(max_sequence_len=24, max_batch_size=B, key_value_memory_dict=allocate_kv_cache(model, B, 24, cuda))
+        with torch.inference_mode():
+            model(ids, inference_params=ip)
+            before = _lib.launch_count()
+            for t in range(18):
+                ip.sequence_len_offset = 5 + t
+                pos = torch.full((B, 1), 5 + t, device=cuda)
+                got.append(model(ids[:, :1] + t, position_ids=pos, inference_params=ip).logits)
+        launches.append(_lib.launch_count() - before)
+        if handle is not None:
+            handle.remove()
+    assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(got[:18], got[18:36], got[36:]))
+    assert launches[0] == launches[2] < launches[1]
+    if att_K < 4:
+        assert len(seen) == 19 and all(s[0] is not None and s[0].numel() == att_K for s in seen[1:])
