@@ -834,7 +834,7 @@ extern "C" int djv_out_proj_sparse(void *y, const void *w, const void *x, const 
   if (B > OP_MAX_B) {
 #define DJV_OM(HD_, NT_)                                                                                                   \
   djv::launch_kernel(out_proj_mma_kernel<HD_, NT_>, dim3(ceil_div(d, OM_ROWS)), dim3(OM_THREADS), 0, st, Y, W, X, head_idx, \
-                     n_active_dev, bi, B, d, nheads, nnz)
+                     n_active_dev, bi, B, d, nheads, nnz, early_prefetch() ? 1 : 0)
     if (hd == 128) B <= 8 ? DJV_OM(128, 1) : DJV_OM(128, 2);
     else if (hd == 64) B <= 8 ? DJV_OM(64, 1) : DJV_OM(64, 2);
     else B <= 8 ? DJV_OM(32, 1) : DJV_OM(32, 2);

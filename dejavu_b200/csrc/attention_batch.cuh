@@ -249,6 +249,8 @@ static int launch_qkv_batch(const QkvBatchArgs &a, int heads, cudaStream_t st) {
 // 8 warps split the 32-column pieces of the heads in use. Lane (g, t) loads 16 contiguous bytes of weight rows g and
 // g + 8 and of context rows g and g + 8: the order along k is the same on both sides. (CUDA cores in slices of 8 and 4
 // rows, each reading the weights again, took 23.6 us at 16 rows, 12 of 32 heads of 128, width 4096; this 8.2.)
+// With the caller's word that the heads are known, the weights are asked for under the attention kernel: 16 steps of 8 layers with
+// 16 sequences 11621 -> 11481 us.
 // -------------------------------------------------------------------------------------------
 constexpr int OM_THREADS = 256, OM_WARPS = OM_THREADS / WARP, OM_ROWS = 16;
 
@@ -256,9 +258,17 @@ template <int HD, int NT>
 __global__ void __launch_bounds__(OM_THREADS)
 out_proj_mma_kernel(__half *__restrict__ Y, const __half *__restrict__ W, const __half *__restrict__ X,
                     const int *__restrict__ head_idx, const int *__restrict__ n_active_dev, const __half *__restrict__ bias,
-                    int B, int d, int nheads, int nnz) {
+                    int B, int d, int nheads, int nnz, int early) {
   __shared__ float red[OM_WARPS][NT][OM_ROWS][8];
-  pdl_prologue();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (early) {  // the heads are known: their columns of the block's rows, while the attention before this kernel is still running
+    const int n_pf = n_active_dev ? min(nnz, *n_active_dev) : nnz;
+    for (int o = threadIdx.x; o < n_pf * OM_ROWS; o += OM_THREADS) {
+      const int n = blockIdx.x * OM_ROWS + o % OM_ROWS, h = head_idx[o / OM_ROWS];
+      if (n < d && h >= 0 && h < nheads) bulk_prefetch_l2(W + ((size_t)n * nheads + h) * HD, HD * 2);
+    }
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int PIECES = HD / 32, U = NT == 1 ? 6 : 4;
   const int tid = threadIdx.x, warp = tid / WARP, lane = tid % WARP, g = lane / 4, t = lane % 4;
   const int n0 = blockIdx.x * OM_ROWS;

@@ -583,9 +583,12 @@ class ParallelMHASparseAttMlp(nn.Module):
             n_eff_ptr = state.data_ptr() + 4 * 2
             for b0 in range(0, B, 16):  # (djv_out_proj_sparse takes up to 16 rows per call)
                 nb = min(16, B - b0)
-                call("djv_out_proj_sparse", out[b0].data_ptr(), self.out_proj.weight.data_ptr(),
-                     bb["ctx"][b0].data_ptr(), eff_heads_ptr, n_eff_ptr, None if ob is None else ob.data_ptr(), nb, d,
-                     n, hd, n, ops._stream())
+                # (up to 4 rows finish so soon that asking ahead only delays the attention: 4 sequences, 9216 wide, 2 layers,
+                # 16 steps 11066 us with, 11026 without)
+                with ops.indices_ready(early and nb > 4):
+                    call("djv_out_proj_sparse", out[b0].data_ptr(), self.out_proj.weight.data_ptr(),
+                         bb["ctx"][b0].data_ptr(), eff_heads_ptr, n_eff_ptr, None if ob is None else ob.data_ptr(), nb, d,
+                         n, hd, n, ops._stream())
             return out.view(B, 1, d)
 
         def project(i, b):

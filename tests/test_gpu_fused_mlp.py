@@ -98,7 +98,7 @@ def test_mlp_sparse_fused_with_early_weight_stream(cuda):
     assert torch.equal(got, want) and filler is not None
 
 
-@pytest.mark.parametrize("batch", [1, 2, 3])
+@pytest.mark.parametrize("batch", [1, 2, 3, 9, 16])
 def test_rows_are_asked_for_ahead_within_the_matrix(cuda, batch):
     """A list that is made just before its product, in memory that held anything: what is asked for too early changes nothing."""
     from dejavu_b200 import ops
@@ -114,6 +114,20 @@ def test_rows_are_asked_for_ahead_within_the_matrix(cuda, batch):
         with ops.indices_ready(True, 4096):
             got = ops.mlp_sparse(x, W1, W2t, idx, b1, b2)
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("batch,d,nheads,hd", [(5, 264, 3, 32), (8, 512, 8, 64), (9, 1024, 8, 128), (16, 40, 12, 64)])
+def test_columns_of_heads_are_asked_for_ahead(cuda, batch, d, nheads, hd):
+    from dejavu_b200 import ops
+
+    gen = torch.Generator().manual_seed(d)
+    x, w, b = rand(gen, (batch, nheads, hd)).to(cuda), rand(gen, (d, nheads, hd)).to(cuda), rand(gen, (d,)).to(cuda)
+    heads = torch.randperm(nheads, generator=gen)[: max(1, nheads // 2)].to(torch.int32).to(cuda)
+    want = ops.out_proj_sparse(x, w, heads, b)
+    torch.cuda.synchronize()
+    with ops.indices_ready(True):
+        got = ops.out_proj_sparse(x * 1, w, heads, b)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("Z,N,M,B", [(6144, 12288, 512, 1), (4608, 9216, 200, 3), (1024, 256, 64, 4)])
