@@ -34,22 +34,21 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, D = a.D;
   constexpr int W = NI > 0 ? NI : 1;
-  // the coefficients and the norm's weights: no kernel of the step writes them
-  if (tid < S * S) coef[tid] = a.y ? a.mix[tid] : (tid / S == tid % S ? 1.f : 0.f);
-  if (tid >= 64 && tid < 64 + S) coef[S * S + tid - 64] = a.y ? a.w_out[tid - 64] : 0.f;
-  if (tid >= 96 && tid < 96 + S) coef[S * S + S + tid - 96] = a.w_in ? a.w_in[tid - 96] : 1.f;
-  float gamma[W][V];
-  if constexpr (NI > 0) {
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const int c = (i * (int)blockDim.x + tid) * V + v;
-        gamma[i][v] = a.gamma && c < D ? __ldg(a.gamma + c) : 0.f;
-      }
-  }
+  // every operand may come from the product just before, the coefficients and the norm's weights too
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  __syncthreads();
+  float k = 0.f;  // a coefficient per thread, on its way together with the columns
+  int ki = -1;
+  if (tid < S * S) {
+    ki = tid;
+    k = a.y ? a.mix[tid] : (tid / S == tid % S ? 1.f : 0.f);
+  } else if (tid >= 64 && tid < 64 + S) {
+    ki = S * S + tid - 64;
+    k = a.y ? a.w_out[tid - 64] : 0.f;
+  } else if (tid >= 96 && tid < 96 + S) {
+    ki = S * S + S + tid - 96;
+    k = a.w_in ? a.w_in[tid - 96] : 1.f;
+  }
+  float gamma[W][V];
   const int row = a.row_list ? a.row_list[blockIdx.x] : blockIdx.x;
   const float *x = a.x_in ? a.x_in + (size_t)row * S * D : nullptr;
   const T *e = nullptr;
@@ -129,13 +128,19 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
     for (int i = 0; i < NI; ++i) {
       const int c = (i * (int)blockDim.x + tid) * V;
       if (c < D) load(c, xs[i], yv[i]);
+#pragma unroll
+      for (int v = 0; v < V; ++v) gamma[i][v] = a.gamma && c < D ? a.gamma[c + v] : 0.f;
     }
+    if (ki >= 0) coef[ki] = k;
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int c = (i * (int)blockDim.x + tid) * V;
       if (c < D) update(c, xs[i], yv[i], u[i]);
     }
   } else {
+    if (ki >= 0) coef[ki] = k;
+    __syncthreads();
 #pragma unroll 2
     for (int c = tid * V; c < D; c += blockDim.x * V) {
       float xs[S][V], yv[V];

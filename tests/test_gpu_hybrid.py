@@ -313,6 +313,35 @@ def test_hyper_step_of_few_rows(dtype, S, D, n):
     test_hyper_step(dtype, S, D, n)
 
 
+@pytest.mark.parametrize("S,D,n", [(4, 2048, 1), (4, 4096, 1), (2, 3000, 2), (4, 4100, 1), (1, 257, 3), (4, 2048, 300)])
+def test_hyper_step_takes_operands_from_the_product_before(S, D, n):
+    """Coefficients and norm weights that the kernel in front makes, in memory that held those of the step before."""
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(D + n)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    x, y, N, K = draw(n, S, D), draw(n, D), 8192, S * S + 2 * S
+    w_gamma, w_coef = (draw(m, N).mul_(N ** -0.5).bfloat16() for m in (D, K))
+    fixed = draw(D), draw(K)
+    inputs = [draw(1, N).bfloat16() for _ in range(2)]
+
+    def boundary(gamma, k):
+        out = torch.empty_like(x)
+        h = ops.hyper_step(x, y, k[:S * S], k[S * S:S * S + S], k[S * S + S:], gamma, 1e-5, torch.bfloat16, x_out=out)
+        return h, out
+
+    made = [tuple(ops.linear_gemv(c, w, torch.float32)[0] for w in (w_gamma, w_coef)) for c in inputs]
+    torch.cuda.synchronize()
+    want = [(boundary(m[0], fixed[1]), boundary(fixed[0], m[1])) for m in made]
+    torch.cuda.synchronize()
+    for t in range(20):
+        c = inputs[t % 2]
+        by_gamma = boundary(ops.linear_gemv(c, w_gamma, torch.float32)[0], fixed[1])
+        by_coef = boundary(fixed[0], ops.linear_gemv(c, w_coef, torch.float32)[0])
+        for got, ref in zip((by_gamma, by_coef), want[t % 2]):
+            assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1]), t
+
+
 # ---- whole models --------------------------------------------------------------------------------------------------
 
 _models: dict = {}
