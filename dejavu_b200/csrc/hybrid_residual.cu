@@ -34,7 +34,18 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, D = a.D;
   constexpr int W = NI > 0 ? NI : 1;
-  // every operand may come from the product just before, the coefficients and the norm's weights too
+  // Every operand may come from the product just before, the coefficients and the norm's weights too: they are read behind the wait.
+  // Ahead of it they are only brought into L2, from where the other weights of a step have driven them.
+  if (NI > 0 && a.gamma != nullptr && tid % 8 == 0) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = (i * (int)blockDim.x + tid) * V;
+      if (c < D) prefetch_l2(a.gamma + c);
+    }
+  }
+  if (a.y != nullptr && tid == 1) prefetch_l2(a.mix);
+  if (a.y != nullptr && tid == 2) prefetch_l2(a.w_out);
+  if (a.w_in != nullptr && tid == 3) prefetch_l2(a.w_in);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   float k = 0.f;  // a coefficient per thread, on its way together with the columns
   int ki = -1;
