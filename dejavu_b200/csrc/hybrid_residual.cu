@@ -274,13 +274,14 @@ __global__ void __launch_bounds__(512) residual_step_kernel(ResidualArgs a) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x, D = a.D;
   constexpr int W = NI > 0 ? NI : 1;
-  float gy[W][4], gh[W][4];  // norm weights: no kernel of the step writes them
-  if constexpr (NI > 0 && NI <= 2) {
+  float gy[W][4], gh[W][4];
+  // the norms' weights: as in hyper_step_kernel, brought into L2 ahead of the wait and read behind it
+  if (NI > 0 && NI <= 2 && tid % 8 == 0) {
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int c = (i * blockDim.x + tid) * 4;
-      if (c < D && a.gamma_y) load4(a.gamma_y + c, gy[i]);
-      if (c < D && a.gamma) load4(a.gamma + c, gh[i]);
+      if (c < D && a.gamma_y) prefetch_l2(a.gamma_y + c);
+      if (c < D && a.gamma) prefetch_l2(a.gamma + c);
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -306,6 +307,8 @@ __global__ void __launch_bounds__(512) residual_step_kernel(ResidualArgs a) {
         if (x) load4(x + c, xv[i]);
         else load4(e + c, xv[i]);
         if (y) load4(y + c, yv[i]);
+        if (NI <= 2 && a.gamma_y) load4(a.gamma_y + c, gy[i]);
+        if (NI <= 2 && a.gamma) load4(a.gamma + c, gh[i]);
       }
     }
     for (int k = 0; k < np; ++k) {

@@ -86,6 +86,29 @@ def test_residual_step(dtype, D, n, k):
     assert ops.residual_step(dev(x), None, None, dev(gh), eps, dtype, rows=rows[:0].cuda()).shape == (0, D)
 
 
+@pytest.mark.parametrize("D,n", [(2048, 1), (4096, 1), (2052, 3), (8192, 2), (257, 2), (4096, 300)])
+def test_residual_step_takes_weights_from_the_product_before(D, n):
+    """Norm weights that the kernel in front makes, in memory that held those of the step before."""
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(D + n)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    x, y, N = draw(n, D), draw(n, D), 8192
+    w, inputs = draw(2 * D, N).mul_(N ** -0.5).bfloat16(), [draw(1, N).bfloat16() for _ in range(2)]
+
+    def boundary(both):
+        out = torch.empty_like(x)
+        return ops.residual_step(x, y, both[:D], both[D:], 1e-5, torch.bfloat16, base=1.0, x_out=out), out
+
+    made = [ops.linear_gemv(c, w, torch.float32)[0] for c in inputs]
+    torch.cuda.synchronize()
+    want = [boundary(m) for m in made]
+    torch.cuda.synchronize()
+    for t in range(20):
+        got = boundary(ops.linear_gemv(inputs[t % 2], w, torch.float32)[0])
+        assert all(torch.equal(a, b) for a, b in zip(got, want[t % 2])), t
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("B", [1, 3, 4, 5, 13, 32])
 @pytest.mark.parametrize("N,M", [(64, 40), (1000, 34), (50, 22)])
