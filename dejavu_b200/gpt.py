@@ -194,16 +194,14 @@ class GPTModel(nn.Module):
         next_mlp_sp_logit, next_att_idx = None, None
         partial_in = False
         for layer in self.layers:  # gpt_dejavu.py:574-594
-            # what the last layer's predictors say of a decoded token is for no layer
-            quiet = {"look_ahead": False} if layer is self.layers[-1] and input_ids.size(1) == 1 and layer.predicts_unheard() else {}
             if self.att_sparse:
                 hidden_states, residual, next_mlp_sp_logit, next_att_idx = layer(
                     hidden_states, residual, head_idx=next_att_idx, mlp_sp_logit=next_mlp_sp_logit,
-                    mixer_kwargs=mixer_kwargs, hidden_is_partial=partial_in, **quiet)
+                    mixer_kwargs=mixer_kwargs, hidden_is_partial=partial_in)
             else:
                 hidden_states, residual, next_mlp_sp_logit = layer(
                     hidden_states, residual, mlp_sp_logit=next_mlp_sp_logit if self.mlp_sparse else None,
-                    mixer_kwargs=mixer_kwargs, hidden_is_partial=partial_in, **quiet)
+                    mixer_kwargs=mixer_kwargs, hidden_is_partial=partial_in)
             partial_in = self.comm is not None
         # final residual add + ln_f (gpt_dejavu.py:606-610)
         last = self.layers[-1]

@@ -321,11 +321,11 @@ class ParallelFusedMLPDejavu(nn.Module):
     def fc2_weight_t(self):
         return self.fc2.weight_t
 
-    def forward(self, x, residual, idx=None, look_ahead=True):
+    def forward(self, x, residual, idx=None):
         do_token_generation = x.size(1) == 1
         # the look-ahead predictor for the NEXT layer runs beside this MLP (fused_dense_sparse_dejavu.py:942-949)
         mlp_logit = None
-        if do_token_generation and self.has_predictor and self.run_predictor and look_ahead:
+        if do_token_generation and self.has_predictor and self.run_predictor:
             with _side(x, "mlp", after=residual) as done:
                 mlp_logit = self.sp(residual)
                 done(mlp_logit)
@@ -655,7 +655,7 @@ class ParallelMHASparseAttMlp(nn.Module):
         # the window advance is folded into the next step's first kernel (no djv_attn_step_finish launch)
         return out.view(B, 1, d)
 
-    def forward(self, x, residual, head_idx=None, mlp_sp_logit=None, seqlen=None, inference_params=None, look_ahead=True, **kwargs):
+    def forward(self, x, residual, head_idx=None, mlp_sp_logit=None, seqlen=None, inference_params=None, **kwargs):
         do_token_generation = x.size(1) == 1
         decoding = inference_params is not None and inference_params.sequence_len_offset > 0
         # Look-ahead work runs beside the attention, as in the reference (sp_stream, mha_dejavu.py:1364-1370,
@@ -672,7 +672,7 @@ class ParallelMHASparseAttMlp(nn.Module):
         result = {"att_idx": None}
 
         def predict_heads():
-            if do_token_generation and self.sp is not None and self.run_predictor and look_ahead:
+            if do_token_generation and self.sp is not None and self.run_predictor:
                 nxt = self.next_mixer if (decoding and FUSE_STEP_OPEN) else None
                 with _side(x, "att", after=residual) as done:
                     scores = self.sp(residual)
@@ -788,32 +788,20 @@ class BlockMlpAttSparse(nn.Module):
         residual = (hidden_states + residual) if residual is not None else hidden_states
         return norm(residual.to(dtype=norm.weight.dtype)), residual
 
-    def predicts_unheard(self) -> bool:
-        """Whether, without a layer behind this one, nobody learns what its predictors say: no hooks that could look at it."""
-        parts = [self, self.mixer, self.mlp, *(m.sp for m in (self.mixer, self.mlp) if getattr(m, "sp", None) is not None)]
-        parts += [c for m in parts[3:] for c in m.children()]
-        return (self.comm is None and type(self) in (BlockMlpAttSparse, BlockDejavu)
-                and type(self.mixer) in (ParallelMHASparseAttMlp, ParallelMHADejavu)
-                and type(self.mlp) in (ParallelFusedMLPDejavu, ParallelFusedMLP)
-                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in parts)
-                and not nn.modules.module._has_any_global_hook())
-
     def forward(self, hidden_states, residual=None, mixer_subset=None, mixer_kwargs=None, head_idx=None,
-                mlp_sp_logit=None, hidden_is_partial=False, look_ahead=True):
+                mlp_sp_logit=None, hidden_is_partial=False):
         # the wait for the head list goes before the LayerNorm launch, so that the QKV projection follows the
         # LayerNorm with a single (programmatic) edge and can prefetch its weights while the LayerNorm runs
         _wait_ready(head_idx)
         hidden_states, residual = self._add_norm(hidden_states, residual, self.norm1, hidden_is_partial)
         if mixer_kwargs is None:
             mixer_kwargs = {}
-        # (said only when there is no layer to look ahead for, so that other mixers and MLPs need not know of it)
-        quiet = {} if look_ahead else {"look_ahead": False}
         if self.returns_att_idx:
             hidden_states, mlp_idx, next_att_idx = self.mixer(hidden_states, residual=residual, head_idx=head_idx,
-                                                              mlp_sp_logit=mlp_sp_logit, **mixer_kwargs, **quiet)
+                                                              mlp_sp_logit=mlp_sp_logit, **mixer_kwargs)
         else:
             hidden_states, mlp_idx = self.mixer(hidden_states, residual=residual, mlp_sp_logit=mlp_sp_logit,
-                                                **mixer_kwargs)  # (has no predictor)
+                                                **mixer_kwargs)
             next_att_idx = None
         if self.comm is not None and self.mlp.can_fuse_after_exchange(hidden_states, mlp_idx):
             _wait_ready(mlp_idx)
@@ -821,7 +809,7 @@ class BlockMlpAttSparse(nn.Module):
                                                                                           self.norm2, mlp_idx)
         else:
             hidden_states, residual = self._add_norm(hidden_states, residual, self.norm2, self.comm is not None)
-            hidden_states, next_mlp_sp_logit = self.mlp(hidden_states, residual, mlp_idx, **(quiet if self.mlp.has_predictor else {}))
+            hidden_states, next_mlp_sp_logit = self.mlp(hidden_states, residual, mlp_idx)
         if self.returns_att_idx:
             return hidden_states, residual, next_mlp_sp_logit, next_att_idx
         return hidden_states, residual, next_mlp_sp_logit
