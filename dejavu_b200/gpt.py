@@ -193,6 +193,8 @@ class GPTModel(nn.Module):
         mixer_kwargs = {"inference_params": inference_params} if inference_params is not None else {}
         next_mlp_sp_logit, next_att_idx = None, None
         partial_in = False
+        # The last layer's predictors run as well, though no layer uses what they say: hooks, a predictor of the caller's own and who
+        # records selections to replay them all listen. (Left out, 4 layers of 9216 took 1.3 % less, so 64 of them 0.1 %.)
         for layer in self.layers:  # gpt_dejavu.py:574-594
             if self.att_sparse:
                 hidden_states, residual, next_mlp_sp_logit, next_att_idx = layer(
