@@ -831,8 +831,7 @@ extern "C" int djv_out_proj_sparse(void *y, const void *w, const void *x, const 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   __half *Y = static_cast<__half *>(y);
   const __half *X = static_cast<const __half *>(x), *W = static_cast<const __half *>(w), *bi = static_cast<const __half *>(bias);
-  static const int k_op = env_int("DJV_OPB", OP_MAX_B);
-  if (B > k_op) {
+  if (B > OP_MAX_B) {
 #define DJV_OM(HD_, NT_)                                                                                                   \
   djv::launch_kernel(out_proj_mma_kernel<HD_, NT_>, dim3(ceil_div(d, OM_ROWS)), dim3(OM_THREADS), 0, st, Y, W, X, head_idx, \
                      n_active_dev, bi, B, d, nheads, nnz, early_prefetch() ? 1 : 0)

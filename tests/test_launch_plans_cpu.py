@@ -157,3 +157,19 @@ for B, shares in ((7, 1), (16, 2), (64, 4)):
     n = project(B, 12, 4, 64, 768)
     assert "qkv_batch" in n["kernel"] and n["grid"] == 12 * 3 * n["cluster"] * shares, n
 """)
+
+
+def test_rows_per_kernel_do_not_depend_on_the_environment(fake):
+    """From which number of rows on the tensor-core kernels take fc2 and the output projection, whatever a sweep may have set."""
+    run(fake, """
+import os
+os.environ.update(DJV_RAB="9", DJV_OPB="9")
+lib = load("libdejavu_b200.so")
+lib.djv_gather_transposed_gemv_scratch_bytes.restype = C.c_size_t
+for B in range(1, 17):
+    need = lib.djv_gather_transposed_gemv_scratch_bytes(B, 4096, 2048)
+    done(lib, lib.djv_gather_transposed_gemv(ptr, ptr, ptr, ptr, None, B, 4096, 2048, L(4096), 0, ptr, C.c_size_t(need), None))
+    assert any("rowaxpy_mma" in n["kernel"] for n in notes()) == (B >= 3), B
+    done(lib, lib.djv_out_proj_sparse(ptr, ptr, ptr, ptr, None, None, B, 4096, 32, 128, 12, None))
+    assert any("out_proj_mma" in n["kernel"] for n in notes()) == (B >= 5), B
+""")
