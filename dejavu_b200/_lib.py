@@ -84,6 +84,7 @@ SIGNATURES = {
     "djv_mlp_sparse_fused": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _ll, _ll, _i, _vp, _sz, _vp]),
     "djv_mlp_sparse_fused_exchange": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _f, _vp, _vp, _vp, _vp, _vp,
                                            _i, _i, _i, _i, _ll, _ll, _i, _vp, _sz, _vp]),
+    "djv_set_early_weight_rows": (None, [_i]),
     "djv_set_early_weight_prefetch": (None, [_i]),
     "djv_set_programmatic_launch": (None, [_i]),
     "djv_batch_sum": (_i, [_vp, _vp, _i, _i, _vp]),

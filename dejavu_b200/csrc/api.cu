@@ -28,9 +28,9 @@ int check_launch(const char *what) {
   return DJV_OK;
 }
 
-static thread_local int g_early_prefetch = 0;
+static thread_local int g_early_prefetch = 0, g_early_rows = 0;
 bool early_prefetch() { return g_early_prefetch != 0 && pdl_enabled(); }
-int early_rows() { return pdl_enabled() ? g_early_prefetch : 0; }
+int early_rows(int unknown) { return !early_prefetch() ? 0 : g_early_rows > 0 ? g_early_rows : unknown; }
 
 static thread_local int g_programmatic_launch = 1;
 bool pdl_enabled() {
@@ -55,7 +55,9 @@ int sm_count() {
 
 extern "C" int djv_version(void) { return 100; }
 
-extern "C" void djv_set_early_weight_prefetch(int rows) { djv::g_early_prefetch = rows; }
+extern "C" void djv_set_early_weight_prefetch(int enabled) { djv::g_early_prefetch = enabled; }
+
+extern "C" void djv_set_early_weight_rows(int rows) { djv::g_early_rows = rows; }
 
 extern "C" void djv_set_programmatic_launch(int enabled) { djv::g_programmatic_launch = enabled; }
 

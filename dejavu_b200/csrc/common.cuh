@@ -43,7 +43,9 @@ bool pdl_enabled();
 // Set by djv_set_early_weight_prefetch for the calling thread: kernels may read their index list / attention
 // state and prefetch weight rows into L2 before they wait for the kernel launched just before them.
 bool early_prefetch();
-int early_rows();  // below which the rows that index lists name may be asked for ahead of the wait (0: none)
+// Below which the rows that index lists name may be asked for ahead of the wait (0: none): djv_set_early_weight_rows, `unknown`
+// where nothing was said there.
+int early_rows(int unknown);
 
 template <typename... P, typename... A>
 inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

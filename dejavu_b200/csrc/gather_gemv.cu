@@ -33,7 +33,7 @@ static void launch_rowdot(const RowdotPlan &p, __half *Y, const __half *W, const
                           int idx64, cudaStream_t st) {
 #define DJV_RD(WPR_, R_, U_, BL_, SP_)                                                                                            \
   djv::launch_kernel(rowdot_kernel<__half, __half, B, ACT, WPR_, R_, U_, BL_, SP_>, p.grid, RD_THREADS, 0, st, Y, W, X, idx, bias, \
-                     M, N, ldw, idx64, idx == nullptr ? M : early_rows(), 0.f, p.per_block, p.rest)
+                     M, N, ldw, idx64, idx == nullptr ? M : early_rows(INT_MAX), 0.f, p.per_block, p.rest)
   DJV_ROWDOT(p, B, DJV_RD);
 #undef DJV_RD
 }

@@ -119,7 +119,7 @@ rowdot_mma_short_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__
   const int g = lane / 4, t = lane % 4;
   const int m0 = blockIdx.x * MS_ROWS;
   const int m_lo = m0 + g, m_hi = m0 + g + 8;
-  if (ahead > 0) {  // the block's share of its rows, of those below `ahead`, while the kernel before this one is still running
+  if (ahead > 0) {  // the block's share of its rows, of those below `ahead` (known to exist), while the kernel before this one runs
     const int row_bytes = N * (int)sizeof(T), per = min(MS_AHEAD, ((row_bytes + S - 1) / S + 15) / 16 * 16);
     if (tid < MS_ROWS && m0 + tid < M && sblk * per < row_bytes) {
       const long long r = load_index(idx, m0 + tid, idx64);
@@ -284,7 +284,7 @@ static int launch_rowdot_mma(TO *Y, const T *W, const T *X, const void *idx, con
     if (rowdot_mma_is_short(M, N, NT, per_sm * sm_count())) {
       const int S = rowdot_mma_short_split(M, N, NT, per_sm);
       djv::launch_kernel_cluster(rowdot_mma_short_kernel<T, TO, NT, ACT>, dim3(ceil_div(M, MS_ROWS), S), dim3(MS_THREADS), 0, st,
-                                 dim3(1, S, 1), Y, W, X, idx, bias, M, N, ldw, idx64, B, act_param, idx == nullptr ? M : early_rows());
+                                 dim3(1, S, 1), Y, W, X, idx, bias, M, N, ldw, idx64, B, act_param, idx == nullptr ? M : early_rows(0));
       count_launch();
       return DJV_OK;
     }

@@ -435,20 +435,22 @@ def batch_sum(x: torch.Tensor) -> torch.Tensor:
 
 
 @contextlib.contextmanager
-def indices_ready(ready: bool = True, rows: int = 1):
+def indices_ready(ready: bool = True, rows: Optional[int] = None):
     """Inside this block the caller promises that the index lists / attention state passed to the operators
     are complete before the kernels can start (produced on another stream and joined with an event): the
     kernels then prefetch their weight rows while the kernel launched before them is still running
     (see djv_set_early_weight_prefetch). `rows`: how many rows the matrices have that the lists name rows of; a gathered
-    product asks ahead only for rows below it."""
+    product then asks ahead only for rows below it (djv_set_early_weight_rows)."""
     lib = _lib.load()
     if ready:
-        lib.djv_set_early_weight_prefetch(max(1, rows))
+        lib.djv_set_early_weight_prefetch(1)
+        lib.djv_set_early_weight_rows(rows or 0)
     try:
         yield
     finally:
         if ready:
             lib.djv_set_early_weight_prefetch(0)
+            lib.djv_set_early_weight_rows(0)
 
 
 def topk_indices_open_step(scores: torch.Tensor, k: int, state: torch.Tensor, cache_len: int) -> torch.Tensor:

@@ -57,7 +57,7 @@ const char *djv_last_error(void);
 const char *djv_status_string(int status);
 /* Number of kernels launched by this library on this process since load (all threads). */
 unsigned long long djv_launch_count(void);
-/* Per calling thread, default 0. While not 0, the gather / head-sparse kernels launched by this thread read
+/* Per calling thread, default 0. While set, the gather / head-sparse kernels launched by this thread read
  * their index list (idx, head_idx, the attention state) and start fetching weight rows BEFORE they wait for the
  * kernel launched just before them on the stream (they are launched with programmatic dependent launch and
  * would otherwise idle until it has drained). It is a hint that the index arguments are already complete at
@@ -67,10 +67,16 @@ unsigned long long djv_launch_count(void);
  * takes the hint when it is given the row count to bound the values, see djv_mlp_sparse_fused). Note that an
  * event wait in front of a programmatically launched kernel does not by itself order that kernel's pre-wait
  * reads after the event: inside a captured CUDA graph such an edge can be programmatic as well, and a list that is
- * still being written can hold anything. djv_gather_gemv and djv_mlp_sparse therefore prefetch only rows below
- * `rows`, the row count of the gathered matrix (with 1, no more than row 0). Activations are always read after the
- * wait. Kernels without an index list (idx == NULL) always prefetch. No reference counterpart. */
-void djv_set_early_weight_prefetch(int rows);
+ * still being written can hold anything: say how many rows the matrix has where that can be
+ * (djv_set_early_weight_rows). Activations are always read after the wait. Kernels without an index list (idx == NULL)
+ * always prefetch. No reference counterpart. */
+void djv_set_early_weight_prefetch(int enabled);
+
+/* Per calling thread, default 0: the matrices that the index lists of djv_gather_gemv and djv_mlp_sparse name rows of
+ * have at least this many rows. Goes with the hint above: rows from there on are not prefetched, whatever a list holds
+ * (requests for addresses that no page backs hold up the memory of the whole device). 0: not known; 1 to 4 rows of x then
+ * prefetch what the list names, more rows nothing. */
+void djv_set_early_weight_rows(int rows);
 
 /* Per calling thread, default 1. Every kernel of the library is launched with programmatic dependent launch and
  * lets its successor start (and wait) as soon as all its own blocks have started: the successor's launch latency

@@ -44,7 +44,7 @@ def notes():
     out = [l.split() for l in fake.fake_notes().decode().splitlines()]
     fake.fake_clear()
     return [dict(what=l[0], device=int(l[1]), kernel=l[2], grid=int(l[3]) * int(l[4]) * int(l[5]), block=int(l[6]), smem=int(l[7]),
-                 cluster=int(l[8])) for l in out]
+                 cluster=int(l[8]), watched=int(l[9]) if len(l) > 9 else None) for l in out]
 ptr = C.c_void_p(P)
 """
 
@@ -172,4 +172,27 @@ for B in range(1, 17):
     assert any("rowaxpy_mma" in n["kernel"] for n in notes()) == (B >= 3), B
     done(lib, lib.djv_out_proj_sparse(ptr, ptr, ptr, ptr, None, None, B, 4096, 32, 128, 12, None))
     assert any("out_proj_mma" in n["kernel"] for n in notes()) == (B >= 5), B
+""")
+
+
+def test_rows_that_may_be_asked_for_ahead(fake):
+    """The hint alone allows all that a list names where rows are asked for line by line, and nothing of unknown size in bulk; with the
+    rows of the matrix said, those below that."""
+    run(fake, """
+lib = load("libdejavu_b200.so")
+def ahead(B, listed=True):
+    fake.fake_watch(9 if B <= 4 else 11)  # of rowdot_kernel and rowdot_mma_short_kernel
+    done(lib, lib.djv_gather_gemv(ptr, ptr, ptr, ptr if listed else None, None, B, 1024, 512, L(1024), 0, 1, None))
+    n, = notes()
+    assert ("rowdot_mma_short" in n["kernel"]) == (B > 4), n
+    return n["watched"]
+for enabled, rows, few, many in ((0, 0, 0, 0), (0, 4096, 0, 0), (1, 0, 2 ** 31 - 1, 0), (7, 0, 2 ** 31 - 1, 0), (1, 4096, 4096, 4096), (1, 1, 1, 1)):
+    lib.djv_set_early_weight_prefetch(enabled)
+    lib.djv_set_early_weight_rows(rows)
+    for B in (1, 2, 3, 4):
+        assert ahead(B) == few, (enabled, rows, B)
+        assert ahead(B, False) == 512
+    for B in (9, 16, 32):
+        assert ahead(B) == many, (enabled, rows, B)
+        assert ahead(B, False) == 512
 """)
