@@ -8,7 +8,7 @@
 
 Each .cu file is compiled to an object in parallel, then linked into the shared libraries that sit next to this file. Beside them
 stands _calls, a small extension module with a binding for each signature of the libraries' functions (_lib.py): a call with 17
-arguments takes 0.5 us through it and 3 us through ctypes.
+arguments takes 0.5 us through it and 3 us through ctypes, which serves where it could not be compiled.
 Nothing is cached outside the package directory. A library can be built alone, so that a program that serves one kind
 of model compiles only what it needs.
 """
@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import argparse
 import os
+import shlex
 import shutil
 import subprocess
 import sys
@@ -160,22 +161,31 @@ PyMODINIT_FUNC PyInit__calls(void) {
     return "\n".join(out)
 
 
-def build_calls(force: bool = False) -> Path:
-    """Generates and compiles _calls, the bindings of the libraries' functions."""
+def build_calls(force: bool = False) -> Path | None:
+    """Generates and compiles _calls, the bindings of the libraries' functions. Where that cannot be done (no C compiler, no
+    headers of the interpreter) the calls go through ctypes: said, and no error."""
     from . import _lib
 
-    if force or _stale(CALLS, [Path(__file__), PKG / "_lib.py"]):
+    if not force and not _stale(CALLS, [Path(__file__), PKG / "_lib.py"]):
+        return CALLS
+    src, part = OBJ / f"_calls.{os.getpid()}.c", CALLS.with_suffix(f".{os.getpid()}.tmp")
+    try:
+        cc = shlex.split(os.environ.get("CC", "")) or [shutil.which("gcc") or "cc"]
         OBJ.mkdir(exist_ok=True)
-        src, part = OBJ / "_calls.c", CALLS.with_suffix(f".{os.getpid()}.tmp")
         src.write_text(_binding_source(sorted(_lib.KINDS, key=_lib.KINDS.get)))
-        cmd = [os.environ.get("CC") or shutil.which("gcc") or "cc", "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"],
-               str(src), "-o", str(part)]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            sys.stderr.write(r.stdout + r.stderr)
-            raise RuntimeError("compiling _calls failed")
-        os.replace(part, CALLS)
-    return CALLS
+        r = subprocess.run([*cc, "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(part)],
+                           capture_output=True, text=True)
+        why = r.stdout + r.stderr
+        if r.returncode == 0 and part.exists():
+            os.replace(part, CALLS)
+            return CALLS
+    except (OSError, ValueError) as e:
+        why = str(e)
+    finally:
+        src.unlink(missing_ok=True)
+        part.unlink(missing_ok=True)
+    sys.stderr.write(f"{why.rstrip()}\n_calls was not compiled: calls into the libraries go through ctypes, 2 to 3 us slower each\n")
+    return None
 
 
 def _stale(target: Path, deps: list[Path]) -> bool:

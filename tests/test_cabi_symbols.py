@@ -134,3 +134,31 @@ def test_compiled_bindings_answer_as_ctypes_does(lib):
             _lib.call("djv_topk", *wrong)
     with pytest.raises(AttributeError):
         _lib.call("djv_no_such_function")
+
+
+@pytest.mark.parametrize("cc,made", [("gcc -pipe", True), ("", True), ("false", False), ("no-such-compiler -O1", False), ("gcc -nostdinc", False), ("gcc '", False)])
+def test_bindings_that_cannot_be_compiled_are_done_without(monkeypatch, tmp_path, capfd, cc, made):
+    from dejavu_b200 import build
+
+    monkeypatch.setenv("CC", cc)
+    monkeypatch.setattr(build, "OBJ", tmp_path / "objects")
+    monkeypatch.setattr(build, "CALLS", tmp_path / "_calls.so")
+    assert build.build_calls() == (build.CALLS if made else None) and build.CALLS.exists() == made
+    assert ("through ctypes" in capfd.readouterr().err) != made
+    assert [p.name for p in tmp_path.rglob("*") if p.is_file()] == (["_calls.so"] if made else [])
+
+
+def test_calls_without_the_compiled_bindings(lib, monkeypatch):
+    import sys
+
+    import dejavu_b200
+    from dejavu_b200 import _lib
+
+    monkeypatch.setattr(_lib, "_calls", None)
+    monkeypatch.setattr(_lib, "_bound", {})
+    monkeypatch.setitem(sys.modules, "dejavu_b200._calls", None)  # (an import of it raises)
+    monkeypatch.delattr(dejavu_b200, "_calls", raising=False)
+    assert not isinstance(_lib._bind("djv_topk"), type(len))
+    assert _lib.query("djv_gather_transposed_gemv_scratch_bytes", 3, 4096, 512) == lib.djv_gather_transposed_gemv_scratch_bytes(3, 4096, 512)
+    with pytest.raises(_lib.DejavuKernelError, match="null scores"):
+        _lib.call("djv_topk", None, None, None, 1, 1, 0, None)
