@@ -931,15 +931,28 @@ static size_t attn_scratch_bytes(int slots, int B, int hd, int S) {
   return AT_COUNTER_BYTES + (size_t)slots * B * attn_splits(S) * (hd + 2) * sizeof(float);
 }
 
+// Splits, blocks of a cluster, of every head's cached tokens: one per 128 tokens (a pass of a block), or as many as fill the device if
+// that is fewer, and of those no more than make the same number of passes. Blocks of clusters start slowly, those without a head
+// too. One of `share` heads of the launch is taken to be in use: all of a list, a third of a step's, whose selection only the device
+// knows. us with one split per 128 tokens / with this, heads of 128, a third of them in use (all of them): 16 sequences, 32 heads, 137
+// tokens 9.5 / 7.0 (19.5 / 13.5), 1090 41.2 / 26.4 (116.8 / 56.2); 8 sequences of 600 11.6 / 9.1 (28.0 / 24.9), 4 of 1090 14.6 / 8.9
+// (31.5 / 24.8); 72 heads, 2 sequences of 1090 15.6 / 9.2 (37.0 / 25.4). One sequence up to 96 heads, and two of 32, keep their splits.
+// Over 1 to 100 sequences, 12 to 96 heads of 32, 64 and 128, 137 to 2048 tokens a step's attention takes 0.71 to 0.80 of the time by
+// head size, nowhere more than 1.05, that of a list of known length 0.60 to 0.70, nowhere more than 1.14. (444 blocks for all heads, whatever
+// the selection, is up to 1.8 with a third of them in use: 3 sequences, 32 heads, 2048 tokens 9.7 / 13.9, one of 96 heads 10.6 / 13.6.)
+static int fitting_splits(int S, int hd, int heads, int share, int B) {
+  const int fill = sm_count() * (hd == 128 ? 185 : hd == 64 ? 370 : 540) / 100;  // blocks of clusters with which the time is least
+  const int passes = ceil_div(S, AT_THREADS), most = attn_splits(S);  // passes of a block alone
+  const int n = max(1, (int)min((long long)most, (long long)share * fill / ((long long)B * heads)));
+  return n == most ? n : ceil_div(passes, ceil_div(passes, n));
+}
+
 // `scratch` is not used any more (the splits combine through distributed shared memory); the parameters stay
 // in the C signatures so that existing callers keep working.
-static int launch_attn(AttnArgs a, int slots, int B, void *scratch, size_t scratch_bytes, cudaStream_t st,
+static int launch_attn(AttnArgs a, int slots, int share, int B, void *scratch, size_t scratch_bytes, cudaStream_t st,
                        const char *op) {
   (void)scratch; (void)scratch_bytes; (void)op;
-  // Blocks of clusters start slowly, those without a head too: splits only as far as they fill the device. 32 heads of 128, 12 of them
-  // in use, us with one split per 128 tokens / with this: 16 sequences of 137 tokens 10.7 / 7.7, of 608 24.6 / 17.5 (all heads
-  // 55.4 / 33.8), 4 of 1090 16.9 / 12.4; one or two sequences as before.
-  const int nsplit = max(1, min(attn_splits(a.S), (int)(3ll * sm_count() / ((long long)B * slots))));
+  const int nsplit = fitting_splits(a.S, a.hd, slots, share, B);
   dim3 grid(slots, B, nsplit), cluster(1, 1, nsplit);
   if (a.hd == 128) djv::launch_kernel_cluster(decode_attn_kernel<128>, grid, AT_THREADS, 0, st, cluster, a);
   else if (a.hd == 64) djv::launch_kernel_cluster(decode_attn_kernel<64>, grid, AT_THREADS, 0, st, cluster, a);
@@ -1055,7 +1068,7 @@ static int attn_step_attend(void *ctx, const void *q, const void *k_cache, const
   t.state = state;
   t.nnz = nheads; t.nheads = nheads; t.hd = hd; t.S = S; t.len = 0;
   t.scale = softmax_scale;
-  int rc = launch_attn(t, nheads, B, scratch, scratch_bytes, static_cast<cudaStream_t>(stream), "attn_step");
+  int rc = launch_attn(t, nheads, 3, B, scratch, scratch_bytes, static_cast<cudaStream_t>(stream), "attn_step");
   if (rc) return rc;
   return check_launch("attn_step_attend");
 }
@@ -1117,7 +1130,7 @@ extern "C" int djv_decode_attn(void *ctx, const void *q, const void *k_cache, co
   t.head_idx = head_idx;
   t.nnz = slots; t.nheads = nheads; t.hd = hd; t.S = S; t.len = len;
   t.scale = softmax_scale;
-  int rc = launch_attn(t, slots, B, scratch, scratch_bytes, static_cast<cudaStream_t>(stream), "decode_attn");
+  int rc = launch_attn(t, slots, 1, B, scratch, scratch_bytes, static_cast<cudaStream_t>(stream), "decode_attn");
   if (rc) return rc;
   return check_launch("decode_attn");
 }

@@ -196,3 +196,28 @@ for enabled, rows, few, many in ((0, 0, 0, 0), (0, 4096, 0, 0), (1, 0, 2 ** 31 -
         assert ahead(B) == many, (enabled, rows, B)
         assert ahead(B, False) == 512
 """)
+
+
+def test_splits_of_cached_tokens(fake):
+    """One per 128 tokens while that fits the device with a third of the heads in use; fewer, and none that saves no pass, where not."""
+    run(fake, """
+lib = load("libdejavu_b200.so")
+def splits(B, nheads, hd, S, listed=0):
+    if listed:
+        done(lib, lib.djv_decode_attn(ptr, ptr, ptr, ptr, ptr, listed, B, nheads, hd, S, S, C.c_float(1), ptr, C.c_size_t(1 << 30), None))
+    else:
+        done(lib, lib.djv_attn_step_attend_batch(ptr, ptr, ptr, ptr, ptr, B, nheads, hd, S, C.c_float(1), ptr, C.c_size_t(1 << 30), None))
+    n, = notes()
+    assert n["grid"] == (listed or nheads) * B * n["cluster"], n
+    return n["cluster"]
+for S, most in ((1, 1), (128, 1), (129, 2), (600, 5), (1024, 8), (2064, 8), (100000, 8)):
+    for B, nheads in ((1, 12), (1, 72), (1, 96), (2, 32), (2, 12)):
+        assert splits(B, nheads, 128, S) == most, (B, nheads, S)
+    for hd in (32, 64, 128):
+        assert splits(300, 40, hd, S) == 1 and splits(65535, 1, hd, S) == 1
+assert [splits(B, 32, 128, 2064) for B in (3, 4, 8, 16, 32)] == [8, 6, 3, 1, 1]
+assert [splits(B, 32, 128, 145) for B in (4, 8, 16)] == [2, 2, 1]
+assert splits(4, 40, 128, 700) == 3  # (5 of 6 fit: two passes, for which 3 do)
+assert [splits(1, 72, 128, 1104, k) for k in (12, 24, 36, 72)] == [8, 8, 5, 3]
+assert [splits(16, 12, hd, 2064) for hd in (32, 64, 128)] == [8, 8, 4]
+""")
