@@ -37,6 +37,16 @@ def test_mlp_sparse_equals_its_two_products(cuda, form, B):
     assert got.shape == want.shape and torch.equal(got, want)
 
 
+@pytest.mark.parametrize("B", [1, 3])
+def test_mlp_sparse_takes_weights_with_a_dimension_of_one_behind(cuda, B):
+    from dejavu_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(B)
+    x, w1, w2 = (torch.randn(n, 136, device=cuda, generator=g).mul_(0.1).half() for n in (B, 520, 520))
+    idx = torch.randperm(520, device=cuda, generator=g)[:77]
+    assert torch.equal(ops.mlp_sparse(x, w1[..., None], w2[..., None], idx), ops.mlp_sparse(x, w1, w2, idx))
+
+
 def test_mlp_sparse_refuses_what_its_products_refuse(cuda):
     from dejavu_b200 import ops
 
