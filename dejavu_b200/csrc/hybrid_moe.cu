@@ -576,7 +576,7 @@ static int launch_mma(const MoeDecodeArgs &a, int slots, bool up, bool down, cud
 constexpr int M1_SPAN = 64;  // outputs whose sums a block keeps before it finishes them
 
 template <typename T, int WPR>
-__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_up_kernel(MoeDecodeArgs a, int slots) {
+__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_up_kernel(MoeDecodeArgs a) {
   constexpr int GROUPS = MO_WARPS / WPR, GLANES = WARP * WPR, U = 2, AT_ONCE = GROUPS * 2;
   static_assert(M1_SPAN % AT_ONCE == 0, "");
   __shared__ float red[M1_SPAN][2][WPR], weight_s[M1_SPAN];
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(MO_THREADS, 4) moe_one_up_kernel(MoeDecodeArgs
 }
 
 template <typename T, int WPR>
-__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_down_kernel(MoeDecodeArgs a, int slots) {
+__global__ void __launch_bounds__(MO_THREADS, 4) moe_one_down_kernel(MoeDecodeArgs a) {
   constexpr int GROUPS = MO_WARPS / WPR, GLANES = WARP * WPR, U = 2, AT_ONCE = GROUPS * 4, N = Chunk<T>::N;
   static_assert(M1_SPAN % AT_ONCE == 0, "");
   __shared__ float red[M1_SPAN][WPR];
@@ -753,16 +753,16 @@ __global__ void __launch_bounds__(MO_THREADS, 4) moe_one_down_kernel(MoeDecodeAr
 
 // As plan_rowdot: the lanes that share a row by passes x trips.
 template <typename T>
-static int launch_one(const MoeDecodeArgs &a, int slots, bool up, bool down, cudaStream_t st) {
+static int launch_one(const MoeDecodeArgs &a, bool up, bool down, cudaStream_t st) {
   constexpr int N = Chunk<T>::N;
   const int resident = 4 * sm_count();
   int wpr = 1;
 #define DJV_GO(KERNEL_, GRID_)                                                                                       \
   switch (wpr) {                                                                                                     \
-    case 1: djv::launch_kernel(KERNEL_<T, 1>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
-    case 2: djv::launch_kernel(KERNEL_<T, 2>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
-    case 4: djv::launch_kernel(KERNEL_<T, 4>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;                \
-    default: djv::launch_kernel(KERNEL_<T, 8>, dim3(GRID_), dim3(MO_THREADS), 0, st, a, slots); break;               \
+    case 1: djv::launch_kernel(KERNEL_<T, 1>, dim3(GRID_), dim3(MO_THREADS), 0, st, a); break;                       \
+    case 2: djv::launch_kernel(KERNEL_<T, 2>, dim3(GRID_), dim3(MO_THREADS), 0, st, a); break;                       \
+    case 4: djv::launch_kernel(KERNEL_<T, 4>, dim3(GRID_), dim3(MO_THREADS), 0, st, a); break;                       \
+    default: djv::launch_kernel(KERNEL_<T, 8>, dim3(GRID_), dim3(MO_THREADS), 0, st, a); break;               \
   }                                                                                                                  \
   count_launch();
   if (up) {
@@ -786,7 +786,7 @@ static int launch_decode(const MoeDecodeArgs &a, bool up, bool down, cudaStream_
   const bool vec_up = a.D % N == 0 && aligned16(a.x) && aligned16(a.w_gu) && aligned16(a.shared_gu);
   const bool vec_down = a.F % N == 0 && (!a.shared_gu || a.F_shared % N == 0) && a.ld_act % N == 0 && aligned16(a.act) &&
                         aligned16(a.w_down) && aligned16(a.shared_down);
-  if (a.B == 1 && vec_up && vec_down && (long long)a.top * a.F + a.F_shared <= (1 << 28)) return launch_one<T>(a, slots, up, down, st);
+  if (a.B == 1 && vec_up && vec_down && (long long)a.top * a.F + a.F_shared <= (1 << 28)) return launch_one<T>(a, up, down, st);
   if constexpr (sizeof(T) == 2) {
     // several rows share weights (both stages take this form or neither: they agree on where a choice's activations are)
     if (a.B >= 2 && a.B <= MM_B && vec_up && vec_down && a.E <= MM_E) {
