@@ -265,7 +265,7 @@ out_proj_mma_kernel(__half *__restrict__ Y, const __half *__restrict__ W, const 
     const int n_pf = n_active_dev ? min(nnz, *n_active_dev) : nnz;
     for (int o = threadIdx.x; o < n_pf * OM_ROWS; o += OM_THREADS) {
       const int n = blockIdx.x * OM_ROWS + o % OM_ROWS, h = head_idx[o / OM_ROWS];
-      if (n < d && h >= 0 && h < nheads) bulk_prefetch_l2(W + ((size_t)n * nheads + h) * HD, HD * 2);
+      if (n < d && ahead_takes(h, nheads)) bulk_prefetch_l2(W + ((size_t)n * nheads + h) * HD, HD * 2);
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "../../include/dejavu_b200.h"
+#include "ahead.cuh"
 
 namespace djv {
 

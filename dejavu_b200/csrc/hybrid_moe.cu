@@ -594,9 +594,9 @@ __global__ void __launch_bounds__(MO_THREADS, 4) moe_one_up_kernel(MoeDecodeArgs
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int row_bytes = nch * 16, rows_ahead = min(2 * ns, max(1, RD_AHEAD / row_bytes));
   for (int r = tid; r < rows_ahead; r += MO_THREADS)
-    for (int off = 0; off < row_bytes; off += RD_PIECE)
+    for (int off = 0; off < row_bytes; off += AHEAD_PIECE)
       bulk_prefetch_l2(reinterpret_cast<const char *>(static_cast<const T *>(a.shared_gu) + ((size_t)2 * fs + r) * a.D) + off,
-                       min(RD_PIECE, row_bytes - off));
+                       min(AHEAD_PIECE, row_bytes - off));
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int e_l = 0;  // of place `lane`: the expert, and its score
   float v_l = 0.f;
@@ -692,9 +692,9 @@ __global__ void __launch_bounds__(MO_THREADS, 4) moe_one_down_kernel(MoeDecodeAr
   if (nfs > 0) {
     const int row_bytes = nfs * 16, rows_ahead = min(last - first, max(1, RD_AHEAD / row_bytes));
     for (int r = tid; r < rows_ahead; r += MO_THREADS)
-      for (int off = 0; off < row_bytes; off += RD_PIECE)
+      for (int off = 0; off < row_bytes; off += AHEAD_PIECE)
         bulk_prefetch_l2(reinterpret_cast<const char *>(static_cast<const T *>(a.shared_down) + (size_t)(first + r) * a.F_shared) + off,
-                         min(RD_PIECE, row_bytes - off));
+                         min(AHEAD_PIECE, row_bytes - off));
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid < a.top) base_s[tid] = static_cast<const T *>(a.w_down) + (size_t)a.chosen[tid] * a.D * a.F;

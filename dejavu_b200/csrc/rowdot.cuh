@@ -53,7 +53,6 @@ constexpr int RD_FEW = 8;     // as many as a block with 4 chunks per row can ha
 // 636.2; this rule 543.6 / 597.2, 455.4, 566.1, 626.2. Lines are an instruction each, and with more bytes the loads of the kernel
 // before queue up behind them. In the sparse steps, whose side streams fill the gaps, neither form gains (8034 / 8019 us for 16
 // steps of 8 layers, 4096 wide, 13488 / 13365 of 4 layers, 9216 wide): those, fp16, keep the lines.
-constexpr int RD_PIECE = 8192;
 constexpr int RD_AHEAD = 16384;
 template <typename T>
 constexpr bool is_half = false;
@@ -87,11 +86,11 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if constexpr (!is_half<T>) {
     // Weights are not produced by any kernel of a step, and a prefetch could not return a stale value anyway.
-    const int row_bytes = nchunks * 16, pieces = (row_bytes + RD_PIECE - 1) / RD_PIECE;
+    const int row_bytes = nchunks * 16, pieces = ahead_pieces(row_bytes);
     const int total = (int)min((long long)(last - first) * pieces, max(1ll, (long long)ahead * pieces / row_bytes));
     for (int p = tid; p < total; p += RD_THREADS) {
-      const int off = p % pieces * RD_PIECE;
-      bulk_prefetch_l2(reinterpret_cast<const char *>(W + (first + p / pieces) * ldw) + off, min(RD_PIECE, row_bytes - off));
+      const AheadSpan s = ahead_piece(p, row_bytes);
+      bulk_prefetch_l2(reinterpret_cast<const char *>(W + (first + s.row) * ldw) + s.offset, s.bytes);
     }
   } else if (ahead) {
     // 8 KB of each of 16 rows, line by line: of rows that are below `ahead`. A list that its maker is still writing (an event between
@@ -101,7 +100,7 @@ rowdot_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restrict__
     const int row_lines = (int)min((long long)LINES, ((long long)N * (int)sizeof(T) + 127) / 128);
     for (int m = first + warp; m < min(last, first + MAX_ROWS); m += RD_WARPS) {
       const long long r = load_index(idx, m, idx64);
-      if (r < 0 || r >= ahead) continue;
+      if (!ahead_takes(r, ahead)) continue;
       const char *w0 = reinterpret_cast<const char *>(W + r * ldw);
       for (int l = lane; l < row_lines; l += WARP) prefetch_l2(w0 + (size_t)l * 128);
     }

@@ -101,10 +101,9 @@ rowdot_mma_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__restri
 constexpr int MS_THREADS = 256;
 constexpr int MS_WARPS = MS_THREADS / WARP;
 constexpr int MS_ROWS = 16;
-// Bytes of each row that a block asks for before it waits for the kernel before it, a row a thread: a LayerNorm, under which HBM has
-// little to do. 16 steps of 8 layers, 4096 wide, 16 sequences 11829 -> 11477 us, 12 sequences, 4 layers 6732 -> 6608. (The ring
+// A block asks for up to 8 KB of each of its rows before it waits for the kernel before it, a row a thread: a LayerNorm, under which
+// HBM has little to do. 16 steps of 8 layers, 4096 wide, 16 sequences 11829 -> 11477 us, 12 sequences, 4 layers 6732 -> 6608. (The ring
 // form, line by line of a list: up to 1 % slower with 5 and 8 sequences.)
-constexpr int MS_AHEAD = 8192;
 
 template <typename T, typename TO, int NT, int ACT>  // NT groups of 8 activation rows
 __global__ void __launch_bounds__(MS_THREADS, NT == 1 ? 5 : 1)
@@ -120,11 +119,10 @@ rowdot_mma_short_kernel(TO *__restrict__ Y, const T *__restrict__ W, const T *__
   const int m0 = blockIdx.x * MS_ROWS;
   const int m_lo = m0 + g, m_hi = m0 + g + 8;
   if (ahead > 0) {  // the block's share of its rows, of those below `ahead` (known to exist), while the kernel before this one runs
-    const int row_bytes = N * (int)sizeof(T), per = min(MS_AHEAD, ((row_bytes + S - 1) / S + 15) / 16 * 16);
-    if (tid < MS_ROWS && m0 + tid < M && sblk * per < row_bytes) {
+    const AheadSpan s = ahead_share(sblk, S, N * (int)sizeof(T));
+    if (tid < MS_ROWS && m0 + tid < M && s.bytes > 0) {
       const long long r = load_index(idx, m0 + tid, idx64);
-      if (r >= 0 && r < ahead)
-        bulk_prefetch_l2(reinterpret_cast<const char *>(W + r * ldw) + sblk * per, min(per, row_bytes - sblk * per));
+      if (ahead_takes(r, ahead)) bulk_prefetch_l2(reinterpret_cast<const char *>(W + r * ldw) + s.offset, s.bytes);
     }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");

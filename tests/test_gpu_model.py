@@ -229,7 +229,7 @@ def test_cuda_graph_decode_equals_eager(cuda, local_exchange):
 
 @pytest.mark.parametrize("B", [2, 4, 18])
 def test_cuda_graph_batched_decode_equals_eager(cuda, B):
-    """A batch decodes through the batch entry points (one state, plain launches): the captured graph replays the
+    """A batch decodes through the batch entry points (one state): the captured graph replays the
     eager step bit for bit, and a second generation on the same model starts from a clean state."""
     cfg = tiny_config(256, 2)
     model = build(cfg, cuda)

@@ -221,3 +221,47 @@ assert splits(4, 40, 128, 700) == 3  # (5 of 6 fit: two passes, for which 3 do)
 assert [splits(1, 72, 128, 1104, k) for k in (12, 24, 36, 72)] == [8, 8, 5, 3]
 assert [splits(16, 12, hd, 2064) for hd in (32, 64, 128)] == [8, 8, 4]
 """)
+
+
+def test_bounds_of_what_is_asked_for_ahead(tmp_path):
+    """Spans start and end on 16 bytes inside their row, do not overlap, and are all of it where nothing caps them; rows that a list
+    may hold while it is being written are refused."""
+    (tmp_path / "ahead.cpp").write_text(f'#include "{ROOT}/dejavu_b200/csrc/ahead.cuh"\n' + """
+#include <limits.h>
+#include <stdio.h>
+#include <string>
+#define CHECK(c) if (!(c)) { printf("%s: %d %d %d\\n", #c, bytes, n, k); return 1; }
+using namespace djv;
+int main() {
+  int n = 0, k = 0;
+  for (int bytes = 16; bytes <= 12 * AHEAD_PIECE; bytes += 16) {
+    n = ahead_pieces(bytes);
+    for (int row = 0; row < 3; ++row) {
+      int at = 0;
+      for (k = 0; k < n; ++k) {
+        const AheadSpan s = ahead_piece(row * n + k, bytes);
+        CHECK(s.row == row && s.offset == at && s.bytes > 0 && s.bytes % 16 == 0 && s.bytes <= AHEAD_PIECE);
+        at += s.bytes;
+      }
+      CHECK(at == bytes);
+    }
+    for (n = 1; n <= 8; ++n) {
+      int at = 0;
+      for (k = 0; k < n; ++k) {
+        const AheadSpan s = ahead_share(k, n, bytes);
+        if (s.bytes <= 0) continue;
+        CHECK(s.row == 0 && s.offset == at && s.bytes % 16 == 0 && s.bytes <= AHEAD_PIECE && s.offset + s.bytes <= bytes);
+        at += s.bytes;
+      }
+      CHECK(at == (bytes < n * AHEAD_PIECE ? bytes : n * AHEAD_PIECE) || (at <= bytes && bytes > n * (AHEAD_PIECE - 16)));
+    }
+  }
+  const int bytes = 0;
+  for (long long r : {-1ll, 4096ll, 0x7f7f7f7fll, 0x7f7f7f7f7f7f7f7fll, LLONG_MIN, -4096ll, 1ll << 32}) CHECK(!ahead_takes(r, 4096));
+  CHECK(ahead_takes(0, 4096) && ahead_takes(4095, 4096) && !ahead_takes(0, 0) && !ahead_takes(1, 1));
+  return 0;
+}
+""")
+    subprocess.run([shutil.which("g++"), "-std=c++17", "-O1", str(tmp_path / "ahead.cpp"), "-o", str(tmp_path / "ahead")], check=True)
+    r = subprocess.run([str(tmp_path / "ahead")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
