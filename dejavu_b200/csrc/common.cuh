@@ -38,8 +38,10 @@ inline int env_int(const char *name, int dflt) {
 // Kernel launch with programmatic dependent launch (PDL): the next kernel of a stream may be scheduled
 // while this one is still running; every kernel of this library starts with pdl_prologue(), which (1) lets
 // its own successor be scheduled early and (2) waits until all its predecessors have completed and their
-// writes are visible, before it touches any memory. Only launch latency is overlapped; ordering of data is
-// the same as without PDL. DJV_PDL=0 in the environment launches the classic way.
+// writes are visible, before it touches any memory, or does the two apart, with work between them that needs no
+// operand: prefetches into L2, which return nothing, and the loads of those weights that the headers name as read early
+// (djv_set_programmatic_launch). Only that is overlapped; ordering of all other data is the same as without PDL.
+// DJV_PDL=0 in the environment launches the classic way.
 bool pdl_enabled();
 // Set by djv_set_early_weight_prefetch for the calling thread: kernels may read their index list / attention
 // state and prefetch weight rows into L2 before they wait for the kernel launched just before them.

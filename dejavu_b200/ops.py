@@ -471,7 +471,8 @@ def topk_indices_open_step(scores: torch.Tensor, k: int, state: torch.Tensor, ca
 def add_layernorm(x, residual, weight, bias, eps: float, xbias=None):
     """r = x + residual (+ xbias); y = LayerNorm(r). Returns (y, r). x, residual (batch, d) fp16.
     Stands in for `residual = dropped + residual; hidden = norm(residual)`
-    (Dejavu/src/models/modules/block_dejavu.py:575-584, 625-636)."""
+    (Dejavu/src/models/modules/block_dejavu.py:575-584, 625-636). weight and bias are read early
+    (djv_set_programmatic_launch): no operator that may still be running writes them."""
     batch, d = x.shape
     _require_cuda(x, residual, weight, bias, xbias)
     assert x.dtype == torch.float16 and weight.dtype == torch.float16 and bias.dtype == torch.float16
@@ -644,7 +645,7 @@ def window_attention_decode(qkv, k_ring, v_ring, sink, freqs, amp: float, pos, h
 
 def gated_linear_attention(proj, a2, a2_bias, tau: float, norm, eps: float, scale: float, state, pos, n: int):
     """proj (B*n, q | k | v | gate | low-rank decay input) -> (B*n, H*dv), normed and gated; state (B, H, dk, dv) fp32
-    is advanced in place (a sequence at position 0 starts from zero)."""
+    is advanced in place (a sequence at position 0 starts from zero). With n = 1 a2 is read early (djv_set_programmatic_launch)."""
     _, H, dk, dv = state.shape
     b, rank = pos.numel(), a2.shape[1]
     assert proj.shape[0] == b * n and proj.shape[1] >= 2 * H * (dk + dv) + rank and proj.stride(1) == 1
@@ -703,7 +704,7 @@ def mlstm(proj, gates, bias_i, bias_f, cap: float, norm, eps: float, scale: floa
           dtype):
     """proj (B*n, q | k | v | output gate), gates (B*n, input | forget) fp32 -> (B*n, H*dv) of `dtype`, normed and gated;
     state (B, H, ...) is advanced in place (a sequence at position 0 starts from zero). n == 1: a decode step, proj is
-    fp32; else proj is of `dtype`."""
+    fp32 and bias_i, bias_f are read early (djv_set_programmatic_launch); else proj is of `dtype`."""
     H, b = state.shape[1], pos.numel()
     assert proj.shape[0] == gates.shape[0] == b * n and proj.stride(1) == 1 and gates.stride(1) == 1
     assert proj.shape[1] >= 2 * H * (dk + dv) and gates.shape[1] >= 2 * H and gates.dtype == torch.float32
@@ -769,7 +770,8 @@ def latent_attention_decode(proj, uk, uv, norm, eps: float, freqs, ring, gate, p
                             stages: int = 7, scratch=None):
     """One token per sequence on the ring itself: proj (B, q | latent | key part, ...) neither normed nor rotated, uk
     (H*dim, rank), uv (H*dv, rank), gate (B, H*dv) or None. Returns (B, H*dv). stages (1 queries and cache row, 2
-    attention, 4 values) and scratch (qc, sums) are for timing the kernels one by one."""
+    attention, 4 values) and scratch (qc, sums) are for timing the kernels one by one. uk and uv are read early
+    (djv_set_programmatic_launch)."""
     B, cap, width = ring.shape
     b, rank = pos.numel(), uk.shape[1]
     dim, dv, rot = uk.shape[0] // heads, uv.shape[0] // heads, width - rank

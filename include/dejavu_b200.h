@@ -85,7 +85,12 @@ void djv_set_early_weight_rows(int rows);
  * per step without / with it: 2 sequences 410 / 394, 16 sequences 509 / 473). Successors launched early sit on the
  * multiprocessors waiting: where kernels of another stream that they depend on find no free slot, or kernels run in
  * several waves of blocks, it can cost more than it hides. 0 launches the kernels of this thread as plain
- * stream-ordered kernels. Never changes a result. */
+ * stream-ordered kernels. Never changes a result.
+ * Read early: some weights are loaded before the kernels in front have finished, and must not be written by kernels of
+ * this library that are still on their way: gamma and beta of djv_add_layernorm, djv_allreduce_add_layernorm and
+ * djv_mlp_sparse_fused_exchange, a2 of djv_gla_decode, bias_i and bias_f of djv_mlstm_decode, uk and uv of
+ * djv_latent_decode. After such a write let an ordinary kernel or copy follow on the stream, or synchronise. Every other
+ * operand may come from the call just before. */
 void djv_set_programmatic_launch(int enabled);
 
 /* ---------------------------------------------------------------------------------------------
