@@ -25,7 +25,8 @@ struct HyperArgs {
 // V columns at a time: 4 (16-byte accesses) or 1. NI: D <= NI * V * blockDim.x, everything a thread reads is on its way before anything
 // is stored (stores could alias the loads behind them, which otherwise wait: a row of 4096 alone took two trips to L2 for its two groups
 // of columns); 0: any D, group by group. A decode step, us before / now: 8 layers 4096 wide (17 boundaries) 701 / 688, 12 layers 2048
-// wide 454 / 448.
+// wide 454 / 448. (With the norm's weights not in L2 by the time of the wait 701; one row of 2048 alone, all of it in L2 already, 2.3
+// with weights and coefficients loaded ahead of the wait, 2.4 so; 200 rows of 4096 8.8 and 9.9.)
 template <typename T, int S, int V, int NI>
 __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   extern __shared__ float u_s[];  // NI == 0: D
@@ -35,29 +36,34 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   const int tid = threadIdx.x, D = a.D;
   constexpr int W = NI > 0 ? NI : 1;
   // Every operand may come from the product just before, the coefficients and the norm's weights too: they are read behind the wait.
-  // Ahead of it they are only brought into L2, from where the other weights of a step have driven them.
-  if (NI > 0 && a.gamma != nullptr && tid % 8 == 0) {
+  // Ahead of it the first block of few rows only brings them into L2, from where the other weights of a step have driven them.
+  if constexpr (NI > 0) {
+    if (blockIdx.x == 0) {
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const int c = (i * (int)blockDim.x + tid) * V;
-      if (c < D) prefetch_l2(a.gamma + c);
+      for (int i = 0; i < NI; ++i) {
+        const int c = (i * (int)blockDim.x + tid) * V;
+        if (a.gamma != nullptr && tid % 8 == 0 && c < D) prefetch_l2(a.gamma + c);
+      }
+      if (a.y != nullptr && tid == 1) prefetch_l2(a.mix);
+      if (a.y != nullptr && tid == 2) prefetch_l2(a.w_out);
+      if (a.w_in != nullptr && tid == 3) prefetch_l2(a.w_in);
     }
   }
-  if (a.y != nullptr && tid == 1) prefetch_l2(a.mix);
-  if (a.y != nullptr && tid == 2) prefetch_l2(a.w_out);
-  if (a.w_in != nullptr && tid == 3) prefetch_l2(a.w_in);
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  float k = 0.f;  // a coefficient per thread, on its way together with the columns
+  // of few rows a thread keeps its coefficient until the loads of the columns are on their way too (of many it would cost registers,
+  // so one block per multiprocessor of three: 4096 rows of 4096 105 / 120 us)
+  auto coefficients = [&](auto &&put) {
+    if (tid < S * S) put(tid, a.y ? a.mix[tid] : (tid / S == tid % S ? 1.f : 0.f));
+    if (tid >= 64 && tid < 64 + S) put(S * S + tid - 64, a.y ? a.w_out[tid - 64] : 0.f);
+    if (tid >= 96 && tid < 96 + S) put(S * S + S + tid - 96, a.w_in ? a.w_in[tid - 96] : 1.f);
+  };
+  float k = 0.f;
   int ki = -1;
-  if (tid < S * S) {
-    ki = tid;
-    k = a.y ? a.mix[tid] : (tid / S == tid % S ? 1.f : 0.f);
-  } else if (tid >= 64 && tid < 64 + S) {
-    ki = S * S + tid - 64;
-    k = a.y ? a.w_out[tid - 64] : 0.f;
-  } else if (tid >= 96 && tid < 96 + S) {
-    ki = S * S + S + tid - 96;
-    k = a.w_in ? a.w_in[tid - 96] : 1.f;
+  if constexpr (NI > 0) {
+    coefficients([&](int i, float v) { ki = i; k = v; });
+  } else {
+    coefficients([&](int i, float v) { coef[i] = v; });
+    __syncthreads();
   }
   float gamma[W][V];
   const int row = a.row_list ? a.row_list[blockIdx.x] : blockIdx.x;
@@ -134,13 +140,21 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
   };
   float u[W][V];
   if constexpr (NI > 0) {
+    const bool wide_gamma = (reinterpret_cast<uintptr_t>(a.gamma) & 15) == 0;
     float xs[NI][S][V], yv[NI][V];
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int c = (i * (int)blockDim.x + tid) * V;
       if (c < D) load(c, xs[i], yv[i]);
+      if (a.gamma != nullptr && c < D) {
+        if (V == 4 && wide_gamma) {
+          const float4 t = *reinterpret_cast<const float4 *>(a.gamma + c);
+          gamma[i][0] = t.x; gamma[i][1 % V] = t.y; gamma[i][2 % V] = t.z; gamma[i][3 % V] = t.w;
+        } else {
 #pragma unroll
-      for (int v = 0; v < V; ++v) gamma[i][v] = a.gamma && c < D ? a.gamma[c + v] : 0.f;
+          for (int v = 0; v < V; ++v) gamma[i][v] = a.gamma[c + v];
+        }
+      }
     }
     if (ki >= 0) coef[ki] = k;
     __syncthreads();
@@ -150,8 +164,6 @@ __global__ void __launch_bounds__(HS_THREADS) hyper_step_kernel(HyperArgs a) {
       if (c < D) update(c, xs[i], yv[i], u[i]);
     }
   } else {
-    if (ki >= 0) coef[ki] = k;
-    __syncthreads();
 #pragma unroll 2
     for (int c = tid * V; c < D; c += blockDim.x * V) {
       float xs[S][V], yv[V];
@@ -276,7 +288,7 @@ __global__ void __launch_bounds__(512) residual_step_kernel(ResidualArgs a) {
   constexpr int W = NI > 0 ? NI : 1;
   float gy[W][4], gh[W][4];
   // the norms' weights: as in hyper_step_kernel, brought into L2 ahead of the wait and read behind it
-  if (NI > 0 && NI <= 2 && tid % 8 == 0) {
+  if (NI > 0 && NI <= 2 && blockIdx.x == 0 && tid % 8 == 0) {
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int c = (i * blockDim.x + tid) * 4;

@@ -322,7 +322,7 @@ def test_hyper_step_takes_operands_from_the_product_before(S, D, n):
     draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
     x, y, N, K = draw(n, S, D), draw(n, D), 8192, S * S + 2 * S
     w_gamma, w_coef = (draw(m, N).mul_(N ** -0.5).bfloat16() for m in (D, K))
-    fixed = draw(D), draw(K)
+    fixed = draw(D + 1)[1:], draw(K)  # (weights that start on 4 bytes only)
     inputs = [draw(1, N).bfloat16() for _ in range(2)]
 
     def boundary(gamma, k):
