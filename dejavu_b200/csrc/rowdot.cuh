@@ -51,8 +51,9 @@ constexpr int RD_FEW = 8;     // as many as a block with 4 chunks per row can ha
 // of 8 KB line by line 568.4 / 624.3, 8 KB in bulk 554.1 / 615.6, 16 KB 547.3 / 607.3, 32 KB 542.1 / 596.3; 12 layers, 2048 wide 472.3,
 // 464.9, 458.7, 451.7, 460.6; with routed experts, 2048 wide 568.1, 576.5, 564.5, 563.6, 569.9, 4096 wide 640.0, 646.0, 630.8, 629.9,
 // 636.2; this rule 543.6 / 597.2, 455.4, 566.1, 626.2. Lines are an instruction each, and with more bytes the loads of the kernel
-// before queue up behind them. In the sparse steps, whose side streams fill the gaps, neither form gains (8034 / 8019 us for 16
-// steps of 8 layers, 4096 wide, 13488 / 13365 of 4 layers, 9216 wide): those, fp16, keep the lines.
+// before queue up behind them. In the sparse steps, fp16, whose side streams fill the gaps, neither form gains: 16 steps of 8 layers,
+// 4096 wide, nothing 8058, line by line 8073, a bulk prefetch per row 8045; 4 layers 9216 wide 13528, 13565, 13550, in runs that differ
+// by 0.1 to 0.4 %. Those keep the lines.
 constexpr int RD_AHEAD = 16384;
 template <typename T>
 constexpr bool is_half = false;

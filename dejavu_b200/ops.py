@@ -208,7 +208,8 @@ def mlp_sparse(x, W1, W2t, idx, bias1=None, bias2=None, push_comm=None, fused=Fa
         assert W1.shape[1] == N and W2t.shape[1] == N
     if not fused:
         f16 = torch.float16
-        Z, N1, N2 = W1.shape[0], W1.shape[1], W2t.shape[1]
+        s1, s2 = W1.shape, W2t.shape  # (a dimension of one behind is no other form)
+        Z, N1, N2 = s1[0], s1[1], s2[1]
         if (push_comm is None and 1 <= batch <= _lib.MAX_BATCH and N1 == N == N2 and W1.stride(1) == 1 and W2t.stride(1) == 1
                 and x.dtype is f16 and W1.dtype is f16 and W2t.dtype is f16 and idx.dtype in (torch.int32, torch.int64)
                 and x.is_cuda and W1.is_cuda and W2t.is_cuda and idx.is_cuda and idx.is_contiguous() and x.is_contiguous()
